@@ -42,7 +42,9 @@ extern "C" {
 
 /* Arithmetic modes for the contraction kernels.  FP32 = CUDA-core fma.rn.f32.
  * 3XTF32 = tensor-core split precision (hi*hi + lo*hi + hi*lo into an f32
- * accumulator), FP32-grade accuracy.  TF32 = single tensor-core pass. Kernels
+ * accumulator, 22 significand bits an operand), FP32-grade accuracy.  TF32 =
+ * single tensor-core pass (11 bits).  The parts are fp16 with a power-of-two
+ * scale per operand, or bf16 where an operand's range asks for it. Kernels
  * that run on CUDA cores (low-channel stencils, streaming ops) ignore it. */
 #define KATSU_MODE_3XTF32 0
 #define KATSU_MODE_TF32 1

@@ -23,13 +23,12 @@ struct katsu_cuda_ctx {
     // it are serialised by stream order.
     float *scratch;
     size_t scratch_floats;
-    // set by conv2d_bwd while one call computes both dX and dW on the implicit-GEMM path: the dX
-    // launch stages g (channels-innermost copy) where the dW launch expects it, once for both
-    int share_g_staging, g_staged;
     // set by the *_staged entry points for the duration of one call: the caller's channels-innermost copy
-    // of x (hi, then lo in 3xTF32 mode), written by katsu_cuda_conv2d_stage; the forward and dW launches use
-    // it instead of staging x themselves
+    // of x (f16_conv.cu), written by katsu_cuda_conv2d_stage; the forward and dW launches use it instead of
+    // staging x themselves
     const float *x_prestaged;
+    // Device memory of the fp16 path (f16_split.cuh): the accumulators of its magnitude pass, the operands' scales.
+    void *f16_state;
     // Buffer written by katsu_cuda_flush_l2.
     float *flush;
     size_t flush_floats;
@@ -127,46 +126,6 @@ int32_t katsu_conv_direct_dx(katsu_cuda_ctx *ctx, const float *w, const float *g
 int32_t katsu_conv_direct_dw(katsu_cuda_ctx *ctx, const float *x, const float *g, float *dw,
                              size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r, size_t s,
                              size_t stride, size_t pad, size_t oh, size_t ow, int accumulate);
-
-// Tensor-core GEMM C[M,N] (+)= A * B (umma_gemm.cu).  a_mn / b_mn: the operand is stored
-// with its M (resp. N) index contiguous rather than K.  *handled = 0 when the shape is not
-// one it takes (alignment, size, FP32 mode); the caller then uses the CUDA-core kernels.
-int32_t katsu_umma_gemm(katsu_cuda_ctx *ctx, const float *a, const float *b, float *c, size_t M, size_t N, size_t K,
-                        bool a_mn, bool b_mn, int accumulate, int *handled);
-
-// The same on pairs of thread blocks (umma_gemm_pair.cu): 256 x 128 tiles, half the B traffic per block.
-// *handled = 0 when M is too small for that; operands already passed katsu_umma_gemm's alignment checks.
-int32_t katsu_umma_gemm_pair(katsu_cuda_ctx *ctx, const float *a, const float *b, float *c, size_t M, size_t N, size_t K,
-                             bool a_mn, bool b_mn, int accumulate, int *handled);
-// Single-pass TF32 with 128 x 256 tiles (umma_gemm_wide.cu); *handled = 0 outside KATSU_MODE_TF32 or for small shapes.
-int32_t katsu_umma_gemm_wide(katsu_cuda_ctx *ctx, const float *a, const float *b, float *c, size_t M, size_t N, size_t K,
-                             bool a_mn, bool b_mn, int accumulate, int *handled);
-
-// dW of a wide convolution through the GEMM kernel (umma_gemm.cu); maps and staging by the caller.
-struct CUtensorMap_st;
-int32_t katsu_umma_conv_dw(katsu_cuda_ctx *ctx, const CUtensorMap_st *map_g, const CUtensorMap_st *map_x,
-                           const CUtensorMap_st *map_x_lo, float *partial, size_t k, size_t c, size_t taps,
-                           size_t total_groups, size_t groups_x, size_t groups_per_img, size_t stride,
-                           const short *off_y, const short *off_x, size_t splits, size_t groups_per_split,
-                           int grouped_maps);
-
-// Wide-channel implicit-GEMM convolution on the tensor cores (conv_igemm.cu); *handled = 0
-// when the shape is outside what it takes.
-// Floats of the staging copy of x that the implicit-GEMM kernels use for this shape in the context's precision
-// mode (0 when the shape takes other kernels), and the pass that writes it.
-size_t katsu_conv_igemm_staged_floats(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t wd, size_t k,
-                                      size_t r, size_t s, size_t stride, size_t pad, size_t oh, size_t ow);
-int32_t katsu_conv_igemm_stage(katsu_cuda_ctx *ctx, const float *x, float *staged, size_t n, size_t c, size_t h,
-                               size_t wd);
-int32_t katsu_conv_igemm_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, float *y,
-                             size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r, size_t s,
-                             size_t stride, size_t pad, size_t oh, size_t ow, int *handled);
-int32_t katsu_conv_igemm_dx(katsu_cuda_ctx *ctx, const float *w, const float *g, float *dx,
-                            size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r, size_t s,
-                            size_t stride, size_t pad, size_t oh, size_t ow, int accumulate, int *handled);
-int32_t katsu_conv_igemm_dw(katsu_cuda_ctx *ctx, const float *x, const float *g, float *dw,
-                            size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r, size_t s,
-                            size_t stride, size_t pad, size_t oh, size_t ow, int accumulate, int *handled);
 
 // Low-channel (C <= 3) 3x3 stride-1 pad-1 convolution on the tensor cores (conv_stem_tc.cu).
 // bias (may be null) and relu are applied in the kernel's epilogue.

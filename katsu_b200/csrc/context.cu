@@ -132,9 +132,12 @@ extern "C" int32_t katsu_cuda_init(int32_t device, katsu_cuda_ctx **out_ctx) {
     if (err == cudaSuccess) err = cudaMalloc(&ctx->status, sizeof(int));
     if (err == cudaSuccess) err = cudaHostAlloc((void **)&ctx->status_host, sizeof(int), cudaHostAllocDefault);
     if (err == cudaSuccess) err = cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
+    if (err == cudaSuccess) err = cudaMalloc(&ctx->f16_state, 1024);
+    if (err == cudaSuccess) err = cudaMemsetAsync(ctx->f16_state, 0, 1024, ctx->stream);
     if (err != cudaSuccess) {
         if (ctx->status_host) cudaFreeHost(ctx->status_host);
         if (ctx->status) cudaFree(ctx->status);
+        if (ctx->f16_state) cudaFree(ctx->f16_state);
         if (ctx->stream) cudaStreamDestroy(ctx->stream);
         if (ctx->pool) cudaMemPoolDestroy((cudaMemPool_t)ctx->pool);
         cudaGetLastError();
@@ -156,6 +159,7 @@ extern "C" int32_t katsu_cuda_shutdown(katsu_cuda_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->flush) cudaFree(ctx->flush);
     if (ctx->status) cudaFree(ctx->status);
+    if (ctx->f16_state) cudaFree(ctx->f16_state);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
     cudaStreamDestroy(ctx->stream);
     // blocks still held by the caller stay valid: the driver releases the pool with its last allocation

@@ -1,8 +1,8 @@
 // Conv2D entry points of the C ABI: argument checks, output geometry and the
-// choice of kernel family.  The arithmetic lives in conv_stencil.cu (low
-// channel counts), conv_igemm.cu (wide channels, tensor cores) and
-// conv_direct.cu (everything else, CUDA cores).
+// choice of kernel family.  The arithmetic lives in conv_stem_tc*.cu and conv_stencil*.cu (low channel counts),
+// f16_conv.cu (everything else on the tensor cores) and conv_direct.cu (FP32 mode and tiny layers, CUDA cores).
 #include "common.cuh"
+#include "f16_split.cuh"
 
 namespace {
 
@@ -42,8 +42,10 @@ int32_t forward(katsu_cuda_ctx *ctx, const float *x, const float *w, const float
     KATSU_TRY(katsu_conv_stem_tc_fwd(ctx, x, w, y, n, c, h, wd, k, r, s, stride, pad, bias, relu, &handled));
     if (handled) return KATSU_OK;  // bias and ReLU were applied in that kernel's epilogue
     KATSU_TRY(katsu_conv_stencil_fwd(ctx, x, w, y, n, c, h, wd, k, r, s, stride, pad, &handled));
-    if (!handled) KATSU_TRY(katsu_conv_igemm_fwd(ctx, x, w, y, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, &handled));
-    if (!handled) KATSU_TRY(katsu_conv_direct_fwd(ctx, x, w, y, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow));
+    if (handled) return katsu_bias_relu_inplace(ctx, y, bias, n, k, g.oh * g.ow, relu);
+    KATSU_TRY(katsu_f16_conv_fwd(ctx, x, w, bias, relu, y, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, &handled));
+    if (handled) return KATSU_OK;
+    KATSU_TRY(katsu_conv_direct_fwd(ctx, x, w, y, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow));
     return katsu_bias_relu_inplace(ctx, y, bias, n, k, g.oh * g.ow, relu);
 }
 
@@ -84,33 +86,28 @@ int32_t backward(katsu_cuda_ctx *ctx, const float *x, const float *w, const floa
     int handled = 0;
     KATSU_TRY(katsu_conv_stencil_bwd(ctx, x, w, gr, dx, dw, n, c, h, wd, k, r, s, stride, pad, accumulate, gscale,
                                      gfactor, &handled));
+    if (handled || (dx == nullptr && dw == nullptr)) return KATSU_OK;
+    KATSU_TRY(katsu_f16_conv_bwd(ctx, x, w, gr, gscale, gfactor, dx, dw, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow,
+                                 accumulate, &handled));
     if (handled) return KATSU_OK;
+    void *scaled = nullptr;
     if (gscale != nullptr || gfactor != 1.f) {
-        // no kernel for this shape applies the scale itself: write the scaled gradient out once
+        // the direct kernels do not apply the scale themselves: write the scaled gradient out once
         const size_t count = n * k * g.oh * g.ow;
-        void *scaled = nullptr;
         KATSU_TRY(katsu_pool_alloc(ctx, count * sizeof(float), &scaled));
-        int32_t rc = scale_copy(ctx, (float *)scaled, gr, gscale, gfactor, count);
-        if (rc == KATSU_OK)
-            rc = backward(ctx, x, w, (const float *)scaled, nullptr, 1.f, dx, dw, n, c, h, wd, k, r, s, stride, pad,
-                          accumulate);
-        cudaFreeAsync(scaled, ctx->stream);
-        return rc;
+        const int32_t rc = scale_copy(ctx, (float *)scaled, gr, gscale, gfactor, count);
+        if (rc != KATSU_OK) {
+            cudaFreeAsync(scaled, ctx->stream);
+            return rc;
+        }
+        gr = (const float *)scaled;
     }
-    ctx->share_g_staging = (dx != nullptr && dw != nullptr) ? 1 : 0;
-    ctx->g_staged = 0;
-    if (dx != nullptr) {
-        KATSU_TRY(katsu_conv_igemm_dx(ctx, w, gr, dx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate, &handled));
-        if (!handled)
-            KATSU_TRY(katsu_conv_direct_dx(ctx, w, gr, dx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate));
-    }
-    if (dw != nullptr) {
-        KATSU_TRY(katsu_conv_igemm_dw(ctx, x, gr, dw, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate, &handled));
-        if (!handled)
-            KATSU_TRY(katsu_conv_direct_dw(ctx, x, gr, dw, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate));
-    }
-    ctx->share_g_staging = ctx->g_staged = 0;
-    return KATSU_OK;
+    int32_t rc = KATSU_OK;
+    if (dx != nullptr) rc = katsu_conv_direct_dx(ctx, w, gr, dx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate);
+    if (rc == KATSU_OK && dw != nullptr)
+        rc = katsu_conv_direct_dw(ctx, x, gr, dw, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow, accumulate);
+    if (scaled) cudaFreeAsync(scaled, ctx->stream);
+    return rc;
 }
 
 }  // namespace
@@ -138,7 +135,14 @@ extern "C" int32_t katsu_cuda_conv2d_staged_floats(katsu_cuda_ctx *ctx, size_t n
     KATSU_TRY(geometry(c, h, wd, k, r, s, stride, pad, &g));
     *floats = 0;
     if (n == 0) return KATSU_OK;
-    *floats = katsu_conv_igemm_staged_floats(ctx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow);
+    // layers of at least 16 channels on both sides, in multiples of 4; others are staged inside the calls
+    if (c < 16 || k < 16 || (c & 3) != 0 || (k & 3) != 0 || n * g.oh * g.ow < 64 ||
+        !katsu_f16_conv_geometry(ctx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow))
+        return KATSU_OK;
+    // (never less than one or two f32 copies of x, what callers that size buffers by hand have been told)
+    const size_t copy = n * c * h * wd * (ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1);
+    *floats = katsu_div_up(katsu_f16_conv_staged_bytes(ctx, n, c, h, wd), sizeof(float));
+    if (*floats < copy) *floats = copy;
     return KATSU_OK;
 }
 
@@ -149,7 +153,8 @@ extern "C" int32_t katsu_cuda_conv2d_stage(katsu_cuda_ctx *ctx, const float *x, 
     KATSU_REQUIRE(n > 0 && c > 0 && h > 0 && wd > 0, "empty input");
     // inputs for which katsu_cuda_conv2d_staged_floats reports 0 whatever the filter: nothing to write
     if (ctx->precision == KATSU_MODE_FP32 || c < 16 || (c & 3) != 0) return KATSU_OK;
-    return katsu_conv_igemm_stage(ctx, x, staged, n, c, h, wd);
+    KATSU_REQUIRE((reinterpret_cast<uintptr_t>(staged) & 15u) == 0, "the staged copy must be 16-byte aligned");
+    return katsu_f16_conv_stage(ctx, x, staged, n, c, h, wd);
 }
 
 extern "C" int32_t katsu_cuda_conv2d_fwd_staged(katsu_cuda_ctx *ctx, const float *x, const float *x_staged, const float *w,

@@ -1,0 +1,638 @@
+// The fp16 tensor-core kernel behind matmul and the convolutions in 3xTF32 and TF32 mode (operands: f16_split.cuh).
+//
+// Reference loops: Tensor::matmul and its VJP (crates/katsu-core/src/tensor.rs:265-273, 418-445), Conv2D forward and
+// backward_buffers (crates/katsu-core/src/conv2d.rs:95-103, 232-262, 269-292).
+//
+// One kernel for three contractions; a result tile is 256 lanes x bn columns (bn = 32 .. 256) on a pair of thread blocks:
+//
+//   GEMM     C[j][i]        = sum_k  A[i][k] B[j][k]                 lanes i (contiguous in C), columns j
+//   CONV     Y[n, o, pixel] = sum_ky sum_(kx, c) X[n, pixel + (ky, kx), c] W[ky][o][(kx, c)]    lanes pixels, columns o
+//   CONV_DW  dW[ky, kx, c][o] = sum_pixel X[pixel + (ky, kx), c] G[pixel, o]                    lanes (ky, kx, c), columns o
+//
+// The lane index is the one that is contiguous in the result, so every store instruction of the epilogue writes whole
+// 128-byte lines whatever the alignment, and NCHW comes out of a channels-innermost contraction without a pass.
+//
+// Convolution operands.  The staged tensor is [n][h][w + gap][cp]; the kx taps of a pixel are then ONE contiguous run of
+// S * cp elements (the gap supplies the zeros left and right of a row).  The tensor map gives that run as its innermost
+// dimension, overlapping from pixel to pixel, so k-blocks of 64 lose nothing to channel counts that are no multiple of 64:
+// a filter row of 35 channels x 3 taps is 2 k-blocks, not 3.  Rows above and below the image are outside the tensor: zeros.
+// Lanes are boxes of bw x bh pixels of nb images, chosen to waste few of them (56 x 56: 8 x 8 x 2, none).  TMA's im2col
+// mode, which would waste none at any size, fetches a pixel in 8 clocks (16 bytes a clock; tiled boxes: 58): the wide
+// layer's forward ran at 2 180 clocks a k-block with it.
+//
+// Passes.  Narrow operands (fp16): hi*hi in TF32 mode (NARROW = 1), lo*hi + hi*lo + hi*hi in 3xTF32 mode (NARROW = 2).
+// Wide operands (bf16): the three largest products of two planes, or the six largest of three.  The tensor core's f32
+// accumulation loses about 3e-8 per accumulation step, so in 3xTF32 mode an accumulator receives at most 192 steps before
+// eight epilogue warps fold it into f32 registers while the other one fills.
+//
+// What bounds it: at 256 x 256 a k-block is 12 (4) MMAs of 128 clocks against 64 (32) KiB of operand fill per block,
+// the ratio of the TF32 kernels at twice their rate.
+//
+// Roles: warps 0-7 drain and store (lane quarter = warp % 4, alternate 32-column chunks by warp / 4), warp 8 issues the
+// TMA loads, warp 9 of the leader block the MMAs.  Persistent over tiles x splits.  Every wait is bounded; both blocks of
+// a pair always reach the cluster barrier at the end.
+#include <cstring>
+
+#include "f16_gemm.cuh"
+#include "sm100.cuh"
+#include "sm100_pair.cuh"
+
+using namespace sm100;
+
+namespace {
+
+constexpr int BM = 128, BK = 64;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int MAX_STAGES = 8;
+constexpr int THREADS = 320;
+constexpr uint32_t kLayoutSw64 = 4;
+constexpr int RASTER_M = 16;
+constexpr int SMEM_RING = 208 * 1024;
+constexpr size_t SMEM = SMEM_RING + 1024;
+
+struct Tile {
+    int split, mt, nt;
+};
+
+// Bands of RASTER_M tile rows, column-major inside a band: blocks running together share operand tiles in L2.
+__device__ __forceinline__ Tile tile_of(int item, const KatsuF16Problem &p) {
+    Tile t;
+    const int per_split = p.m_tiles * p.n_tiles;
+    t.split = item / per_split;
+    const int i = item - t.split * per_split;
+    const int band_tiles = RASTER_M * p.n_tiles;
+    const int band = i / band_tiles, r = i - band * band_tiles;
+    const int rows = min(p.m_tiles - band * RASTER_M, RASTER_M);
+    t.nt = r / rows;
+    t.mt = band * RASTER_M + (r - t.nt * rows);
+    return t;
+}
+
+// k-blocks [begin, end) of one class in one split.
+__device__ __forceinline__ void k_range(const KatsuF16Problem &p, long long total, int split, int *begin, int *end) {
+    const long long b = (long long)split * p.kb_per_split;
+    const long long e = b + p.kb_per_split;
+    *begin = int(b < total ? b : total);
+    *end = int(e < total ? e : total);
+}
+
+template <KatsuF16Kind KIND>
+__device__ __forceinline__ long long class_kblocks(const KatsuF16Problem &p, int py, int px) {
+    if (KIND == KATSU_F16_CONV_DW) return p.blocks;
+    if (KIND == KATSU_F16_GEMM) return p.gemm_chunks;
+    return (long long)(p.row_begin[py + 1] - p.row_begin[py]) * p.chunks[px];
+}
+
+// First pixel of a box; past the last box an image that does not exist, which loads as zeros.
+__device__ __forceinline__ void box_origin(const KatsuF16Problem &p, long long b, int *img, int *y, int *x) {
+    if (b >= p.blocks) {
+        *img = p.n_img;
+        *y = *x = 0;
+        return;
+    }
+    const unsigned q = unsigned(b) / unsigned(p.blocks_x);
+    *x = int(unsigned(b) - q * p.blocks_x) * p.bw;
+    const unsigned n = q / unsigned(p.blocks_y);
+    *y = int(q - n * p.blocks_y) * p.bh;
+    *img = int(n) * p.nb;
+}
+
+// One lane's values of columns col .. col + 31.  Few instructions a column: this runs on eight warps per block and sets the
+// pace of layers with short contractions (with its branches inside the loop the small CNN's second dX took 0.58 ms).
+__device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d, int col, const float (&v)[32], float factor) {
+    const long long stride = p.col_stride;
+    const int live = p.n_total - col;
+    if (live >= 32 && !p.bias && !p.relu && !p.accumulate) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            *d = v[i] * factor;
+            d += stride;
+        }
+        return;
+    }
+    const float floor = p.relu ? 0.f : -INFINITY;
+#pragma unroll
+    for (int i0 = 0; i0 < 32; i0 += 8) {
+        float o[8];
+        const bool all = live >= i0 + 8;
+        if (p.accumulate) {  // the loads of eight columns before the first store
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = (all || i0 + i < live) ? d[i * stride] : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] += v[i0 + i] * factor;
+        } else if (p.bias) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = v[i0 + i] * factor + ((all || i0 + i < live) ? __ldg(p.bias + col + i0 + i) : 0.f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = v[i0 + i] * factor;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (o[i] < floor) o[i] = floor;  // (a NaN stays one)
+            if (all || i0 + i < live) *d = o[i];
+            d += stride;
+        }
+    }
+}
+
+template <int NARROW, KatsuF16Kind KIND>
+__global__ void __launch_bounds__(THREADS, 1)
+f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant__ KatsuF16Problem p) {
+    constexpr bool MN = KIND == KATSU_F16_CONV_DW;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    const bool wide = katsu_f16_wide(p.call);
+    const int planes = NARROW + (wide ? 1 : 0);
+    // k-blocks between two drains: 192 accumulation steps in 3xTF32 mode, up to 12 288 in TF32 mode (4e-4 of 2e-3)
+    const int drain = NARROW == 2 ? (wide ? 8 : 16) : 1024;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int items = p.m_tiles * p.n_tiles * p.splits;
+    const int half = p.bn >> 1;                 // B columns that this block loads
+    const int b_bytes = half * BK * 2;
+    const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
+    const int stages = min(MAX_STAGES, SMEM_RING / stage_bytes);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
+            mbar_init(&full[s], 1);    // the leader's: its own expect_tx arrival, both blocks' bytes
+            mbar_init(&empty[s], 1);   // each block's own copy, released by the leader's commit
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);    // each block's own copy
+            mbar_init(&acc_empty[b], 16);  // the leader's: eight epilogue warps of each block
+        }
+        mbar_init_fence();
+    }
+    if (warp == 9) {
+        tmem_alloc_pair(&tmem_slot, 512);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();  // both blocks' barriers exist before anything is signalled across the pair
+    tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_slot;
+
+    if (warp == 8 && lane == 0) {
+        // ---- TMA producer: this block's lanes of A and half of B's columns; bytes counted on the leader's barrier ----
+        const CUtensorMap *map_a = p.a_second && wide && p.info_a->narrow ? maps.a_second : maps.a, *map_b = maps.b;
+        bool ok = true;
+        int s = 0;
+        uint32_t phase = 1;  // a fresh barrier counts as released
+        for (int item = pair; item < items && ok; item += pairs) {
+            const Tile t = tile_of(item, p);
+            const long long m0 = (2ll * t.mt + rank) * BM;
+            const int n0 = t.nt * p.bn + int(rank) * half;
+            int img = 0, jy = 0, jx = 0;  // CONV: first pixel of this block's lanes
+            if (KIND == KATSU_F16_CONV) box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
+            for (int py = 0; py < p.classes_y && ok; ++py)
+                for (int px = 0; px < p.classes_x && ok; ++px) {
+                    int kb0, kb1;
+                    k_range(p, class_kblocks<KIND>(p, py, px), t.split, &kb0, &kb1);
+                    const int chunks = MN ? 1 : KIND == KATSU_F16_GEMM ? p.gemm_chunks : p.chunks[px];
+                    int row = 0, chunk = 0;
+                    if (!MN && kb1 > kb0) {
+                        row = kb0 / chunks;
+                        chunk = kb0 - row * chunks;
+                        row += p.row_begin[py];
+                    }
+                    for (int i = kb0; i < kb1; ++i) {
+                        if (!mbar_wait(&empty[s], phase, p.status, 171)) { ok = false; break; }
+                        if (leader) mbar_arrive_expect_tx(&full[s], 2 * planes * (p.a_bytes + b_bytes));
+                        const uint32_t bar = map_to_rank(&full[s], 0);
+                        unsigned char *st = smem + s * stage_bytes;
+                        if (KIND == KATSU_F16_GEMM) {
+                            for (int part = 0; part < planes; ++part) {
+                                tma_load_3d_pair(st + part * A_BYTES, map_a + part, bar, i * BK, int(m0), 0);
+                                tma_load_3d_pair(st + b_off + part * b_bytes, map_b + part, bar, i * BK, n0, 0);
+                            }
+                        } else if (KIND == KATSU_F16_CONV) {
+                            for (int part = 0; part < planes; ++part) {
+                                tma_load_4d_pair(st + part * A_BYTES, map_a + part, bar, chunk * BK, jx + p.off_w[px],
+                                                 jy * p.in_step + p.lower_h + p.off_h[row], img);
+                                tma_load_3d_pair(st + b_off + part * b_bytes, map_b + part, bar,
+                                                 p.b_col[px] + chunk * BK, n0, p.b_row[row]);
+                            }
+                            if (++chunk == chunks) {
+                                chunk = 0;
+                                ++row;
+                            }
+                        } else {
+                            int n, oy, ox;
+                            box_origin(p, i, &n, &oy, &ox);
+                            const int per_load = half >= 64 ? 64 : 32;
+                            for (int part = 0; part < planes; ++part) {
+#pragma unroll
+                                for (int g = 0; g < 2; ++g) {
+                                    const int group = (2 * t.mt + int(rank)) * 2 + g;
+                                    const int ky = group / p.groups_per_row, j = group - ky * p.groups_per_row;
+                                    const bool live = group < p.groups;  // past the last one: an image that does not exist
+                                    tma_load_4d_pair(st + part * A_BYTES + g * (A_BYTES / 2), map_a + part, bar,
+                                                     live ? j * 64 : 0, ox, oy * p.in_step + p.lower_h + (live ? ky : 0),
+                                                     live ? n : p.n_img);
+                                }
+                                for (int c = 0; c < half; c += per_load)
+                                    tma_load_4d_pair(st + b_off + part * b_bytes + c * BK * 2,
+                                                     map_b + part, bar, n0 + c, ox, oy, n);
+                            }
+                        }
+                        if (++s == stages) {
+                            s = 0;
+                            phase ^= 1;
+                        }
+                    }
+                }
+        }
+    } else if (warp == 9 && leader) {
+        // ---- MMA issue for the pair: whole warp in the loop, the elect.sync thread issues ----
+        const bool issue = elect_one();
+        const uint32_t idesc = idesc_f16(2 * BM, p.bn, MN, MN, wide);
+        // K-major: 128-byte rows, a 16-element step is 32 bytes.  MN-major: 64 (or 32) columns to a row, a step is 16
+        // rows; groups of 64 columns are A_BYTES / 2 apart.
+        const uint32_t b_layout = MN && half < 64 ? kLayoutSw64 : kLayoutSw128;
+        const uint32_t b_sbo = MN && half < 64 ? 512 : 1024;
+        const uint32_t a_step = MN ? 2048 : 32, b_step = MN ? (half < 64 ? 1024 : 2048) : 32;
+        const uint32_t lbo = MN ? A_BYTES / 2 : 16;
+        bool ok = true;
+        int s = 0, q = 0;  // q: accumulator hand-overs so far
+        uint32_t phase = 0;
+        for (int item = pair; item < items && ok; item += pairs) {
+            const int split = item / (p.m_tiles * p.n_tiles);
+            for (int py = 0; py < p.classes_y && ok; ++py)
+                for (int px = 0; px < p.classes_x && ok; ++px) {
+                    int kb0, kb1;
+                    k_range(p, class_kblocks<KIND>(p, py, px), split, &kb0, &kb1);
+                    const int chunks = MN ? 1 : KIND == KATSU_F16_GEMM ? p.gemm_chunks : p.chunks[px];
+                    int chunk = (!MN && kb1 > kb0) ? kb0 % chunks : 0;
+                    const int last = MN ? BK / 16 : p.steps_last[px];
+                    for (int kb = kb0; kb < kb1 && ok; ++q) {
+                        const int b = q & 1;
+                        if (!mbar_wait_warp(&acc_empty[b], ((q >> 1) & 1) ^ 1, p.status, 172)) { ok = false; break; }
+                        tc_fence_after_sync();
+                        const uint32_t acc = tmem_base + uint32_t(b) * 256;
+                        const int kb_end = min(kb + drain, kb1);
+                        bool first = true;
+                        for (; kb < kb_end; ++kb) {
+                            if (!mbar_wait_warp_ready(&full[s], phase, p.status, 173)) { ok = false; break; }
+                            tc_fence_after_sync();
+                            // descriptors differ in their address field only (16-byte units in the low word)
+                            const uint32_t st = smem_u32(smem + s * stage_bytes);
+                            const uint64_t a0 = smem_desc(st, lbo, 1024, kLayoutSw128);
+                            const uint64_t b0 = smem_desc(st + b_off, lbo, b_sbo, b_layout);
+                            const int steps = (!MN && chunk == chunks - 1) ? last : BK / 16;
+                            if (issue) {
+#pragma unroll
+                                for (int j = 0; j < BK / 16; ++j) {
+                                    if (j < steps) {
+                                        const uint64_t ad = a0 + j * (a_step >> 4), bd = b0 + j * (b_step >> 4);
+                                        const uint32_t na = A_BYTES >> 4, nb = b_bytes >> 4;  // to the next plane
+                                        const bool add = !(first && j == 0);
+                                        if (NARROW == 2) {
+                                            if (wide) {
+                                                mma_f16_pair(acc, ad + 2 * na, bd, idesc, add);
+                                                mma_f16_pair(acc, ad + na, bd + nb, idesc, true);
+                                                mma_f16_pair(acc, ad, bd + 2 * nb, idesc, true);
+                                            }
+                                            mma_f16_pair(acc, ad + na, bd, idesc, add || wide);
+                                            mma_f16_pair(acc, ad, bd + nb, idesc, true);
+                                            mma_f16_pair(acc, ad, bd, idesc, true);
+                                        } else {
+                                            if (wide) {
+                                                mma_f16_pair(acc, ad + na, bd, idesc, add);
+                                                mma_f16_pair(acc, ad, bd + nb, idesc, true);
+                                            }
+                                            mma_f16_pair(acc, ad, bd, idesc, add || wide);
+                                        }
+                                    }
+                                }
+                                // every release goes to this block's barrier and to the peer's copy of it
+                                mma_commit_pair(smem_u32(&empty[s]));
+                                mma_commit_pair(map_to_rank(&empty[s], 1));
+                                if (kb == kb_end - 1) {
+                                    mma_commit_pair(smem_u32(&acc_full[b]));
+                                    mma_commit_pair(map_to_rank(&acc_full[b], 1));
+                                }
+                            }
+                            __syncwarp();
+                            first = false;
+                            if (!MN && ++chunk == chunks) chunk = 0;
+                            if (++s == stages) {
+                                s = 0;
+                                phase ^= 1;
+                            }
+                        }
+                    }
+                }
+        }
+    } else if (warp < 8) {
+        // ---- drains and epilogue: thread = lane of this block's half of the tile, alternate 32-column chunks ----
+        const int quarter = warp & 3, group = warp >> 2;
+        const int col_chunks = p.bn >> 5;
+        float factor = p.gfactor;
+        if (!wide) factor *= __uint_as_float(unsigned(127 - p.info_a->exp - p.info_b->exp) << 23);
+        if (p.gscale) factor *= __ldg(p.gscale);
+        int q = 0;
+        bool alive = true;
+        for (int item = pair; item < items && alive; item += pairs) {
+            const Tile t = tile_of(item, p);
+            const long long m = (2ll * t.mt + rank) * BM + quarter * 32 + lane;
+            const int n0 = t.nt * p.bn;
+            int img = 0, jy = 0, jx = 0;
+            bool in_box = true;
+            if (KIND == KATSU_F16_CONV) {
+                const int r = quarter * 32 + lane;
+                box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
+                const int q1 = r / p.bw, q2 = q1 / p.bh;
+                jx += r - q1 * p.bw;
+                jy += q1 - q2 * p.bh;
+                img += q2;
+                in_box = q2 < p.nb && img < p.n_img;
+            }
+            for (int py = 0; py < p.classes_y && alive; ++py)
+                for (int px = 0; px < p.classes_x && alive; ++px) {
+                    int kb0, kb1;
+                    k_range(p, class_kblocks<KIND>(p, py, px), t.split, &kb0, &kb1);
+                    bool valid = in_box && m < p.m_total;
+                    long long at = m;
+                    if (KIND == KATSU_F16_CONV) {
+                        const int y = p.step * jy + py, x = p.step * jx + px;
+                        valid = valid && y < p.out_h && x < p.out_w;
+                        at = img * p.img_stride + (long long)y * p.out_w + x;
+                    }
+                    float *dst = p.out + t.split * p.split_stride + at + n0 * p.col_stride;
+                    auto wait_acc = [&](int b) -> uint32_t {
+                        alive = mbar_wait_warp(&acc_full[b], (q >> 1) & 1, p.status, 174);
+                        tc_fence_after_sync();
+                        return tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b) * 256;
+                    };
+                    auto release_acc = [&](int b) {
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (leader) mbar_arrive(&acc_empty[b]);
+                            else mbar_arrive_cluster(map_to_rank(&acc_empty[b], 0));
+                        }
+                    };
+                    if (kb1 - kb0 <= drain) {
+                        // one accumulator holds it all: 32 columns at a time, no sums in registers
+                        const uint32_t acc = kb1 > kb0 ? wait_acc(q & 1) : 0;
+                        if (!alive) break;
+#pragma unroll 1
+                        for (int c0 = group * 32; c0 < p.bn; c0 += 64) {
+                            float v[32];
+                            if (kb1 > kb0) {
+                                tmem_ld_32x32(acc + c0, v);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) v[i] = 0.f;
+                            }
+                            if (valid) store_columns(p, dst + c0 * p.col_stride, n0 + c0, v, factor);
+                        }
+                        if (kb1 > kb0) {
+                            release_acc(q & 1);
+                            ++q;
+                        }
+                        continue;
+                    }
+                    float run[4][32];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) run[c][i] = 0.f;
+                    for (int kb = kb0; kb < kb1; kb += drain, ++q) {
+                        const uint32_t acc = wait_acc(q & 1);
+                        if (!alive) break;
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            if (2 * c + group < col_chunks) {
+                                float v[32];
+                                tmem_ld_32x32(acc + (2 * c + group) * 32, v);
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) run[c][i] += v[i];
+                            }
+                        }
+                        release_acc(q & 1);
+                    }
+                    if (!alive) break;
+                    if (!valid) continue;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const int c0 = (2 * c + group) * 32;
+                        if (c0 < p.bn) store_columns(p, dst + c0 * p.col_stride, n0 + c0, run[c], factor);
+                    }
+                }
+        }
+    }
+    // Neither block leaves (or gives its tensor memory back) while the other may still signal its barriers,
+    // read its half of B or hold accumulators: every path above ends here.
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 9) tmem_dealloc_pair(tmem_base, 512);
+}
+
+__global__ void __launch_bounds__(256)
+f16_fold_kernel(const float *__restrict__ partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels, size_t plane, int relu) {
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < splits; ++q) s += __ldg(partial + size_t(q) * count + i);
+        if (bias) s += __ldg(bias + (i / plane) % channels);
+        if (relu) s = fmaxf(s, 0.f);
+        out[i] = accumulate ? out[i] + s : s;
+    }
+}
+
+template <int NARROW, KatsuF16Kind KIND>
+int32_t launch(katsu_cuda_ctx *ctx, const KatsuF16Maps &maps, const KatsuF16Problem &p, unsigned pairs) {
+    auto kernel = f16_pair_kernel<NARROW, KIND>;
+    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
+    cudaLaunchConfig_t config;
+    memset(&config, 0, sizeof(config));
+    config.gridDim = dim3(2 * pairs, 1, 1);
+    config.blockDim = dim3(THREADS, 1, 1);
+    config.dynamicSmemBytes = SMEM;
+    config.stream = ctx->stream;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = 2;
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    cudaError_t err = cudaLaunchKernelEx(&config, kernel, maps, p);
+    ctx->launches += 1;
+    if (err != cudaSuccess) return katsu_set_error(KATSU_ERR_CUDA, "fp16 kernel launch failed: %s", cudaGetErrorString(err));
+    return KATSU_OK;
+}
+
+}  // namespace
+
+// Estimated clocks of every way to cut the problem; the cheapest wins.  A k-block costs the tensor pipe
+// passes * 4 * bn / 2 clocks and the fill of (128 + bn / 2) * 128 bytes per part at about 60 bytes a clock; an item costs
+// its pipeline start and its stores besides; splits pay for writing and folding their slabs.
+KatsuF16Plan katsu_f16_plan(const katsu_cuda_ctx *ctx, KatsuF16Kind kind, long long m_total, int n_total,
+                            long long kblocks, double out_floats) {
+    const int parts = ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1, passes = parts == 2 ? 3 : 1;
+    const double pairs = ctx->num_sms / 2;
+    const long long m_tiles = (m_total + 2 * BM - 1) / (2 * BM);
+    KatsuF16Plan best = {0, 1};
+    double best_cost = 0;
+    for (int bn = 32; bn <= 256; bn += 32) {
+        if (kind == KATSU_F16_CONV_DW && bn != 64 && bn != 128 && bn != 256) continue;
+        const long long tiles = m_tiles * ((n_total + bn - 1) / bn);
+        const double pipe = passes * 4 * bn / 2.0, fill = (BM + bn / 2) * 128.0 * parts / 60.0;
+        const double per_kb = (pipe > fill ? pipe : fill) + 30;
+        // unsplit, or as many splits as fill one to four waves
+        for (int w = 0; w <= 4; ++w) {
+            long long splits = w == 0 ? 1 : (long long)(w * pairs) / tiles;
+            if (w > 0 && splits <= 1) continue;
+            if (splits > kblocks / 2) splits = kblocks / 2;
+            if (splits < 1) splits = 1;
+            if (splits > 512) splits = 512;
+            const long long kb = (kblocks + splits - 1) / splits;
+            splits = (kblocks + kb - 1) / kb;
+            const long long waves = (long long)((tiles * splits + pairs - 1) / pairs);
+            double cost = waves * (kb * per_kb + 1200 + bn * 6);
+            if (kind == KATSU_F16_CONV_DW) cost += splits * out_floats * 8 / 3000;
+            else if (splits > 1) cost += (splits + 1) * out_floats * 4 / 2500 + 5000;
+            if (best.bn == 0 || cost < best_cost) {
+                best.bn = bn;
+                best.splits = (int)splits;
+                best_cost = cost;
+            }
+        }
+    }
+    return best;
+}
+
+int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16Maps &maps, KatsuF16Problem p,
+                         const KatsuF16Plan &plan, float *partial, long long split_stride) {
+    const int parts = katsu_f16_narrow_planes(ctx);
+    p.bn = plan.bn;
+    p.splits = plan.splits;
+    p.m_tiles = (int)((p.m_total + 2 * BM - 1) / (2 * BM));
+    p.n_tiles = (p.n_total + plan.bn - 1) / plan.bn;
+    long long most = 0;  // k-blocks of the longest class
+    if (kind == KATSU_F16_CONV_DW) {
+        most = p.blocks;
+    } else if (kind == KATSU_F16_GEMM) {
+        most = p.gemm_chunks;
+    } else {
+        for (int y = 0; y < p.classes_y; ++y)
+            for (int x = 0; x < p.classes_x; ++x) {
+                const long long kb = (long long)(p.row_begin[y + 1] - p.row_begin[y]) * p.chunks[x];
+                if (kb > most) most = kb;
+            }
+    }
+    p.kb_per_split = (int)((most + plan.splits - 1) / plan.splits);
+    if (p.kb_per_split < 1) p.kb_per_split = 1;
+    p.split_stride = 0;
+    if (plan.splits > 1 || kind == KATSU_F16_CONV_DW) {
+        p.out = partial;
+        p.split_stride = split_stride;
+        p.accumulate = 0;
+        p.bias = nullptr;
+        p.relu = 0;
+    }
+    p.status = ctx->status;
+    const long long items = (long long)p.m_tiles * p.n_tiles * p.splits;
+    if (items > 0x3fffffff) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "too many tiles");
+    const unsigned pairs = (unsigned)(items < ctx->num_sms / 2 ? items : ctx->num_sms / 2);
+    if (parts == 2) {
+        if (kind == KATSU_F16_GEMM) return launch<2, KATSU_F16_GEMM>(ctx, maps, p, pairs);
+        if (kind == KATSU_F16_CONV) return launch<2, KATSU_F16_CONV>(ctx, maps, p, pairs);
+        return launch<2, KATSU_F16_CONV_DW>(ctx, maps, p, pairs);
+    }
+    if (kind == KATSU_F16_GEMM) return launch<1, KATSU_F16_GEMM>(ctx, maps, p, pairs);
+    if (kind == KATSU_F16_CONV) return launch<1, KATSU_F16_CONV>(ctx, maps, p, pairs);
+    return launch<1, KATSU_F16_CONV_DW>(ctx, maps, p, pairs);
+}
+
+int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const float *partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels,
+                       size_t plane, int relu) {
+    size_t blocks = katsu_div_up(count, (size_t)256);
+    if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
+    KATSU_LAUNCH(ctx, f16_fold_kernel, (unsigned)blocks, 256, 0, partial, out, count, splits, accumulate,
+                 bias, channels, plane, relu);
+    return KATSU_OK;
+}
+
+bool katsu_f16_rows_maps(CUtensorMap *maps, const KatsuF16Planes &planes, int count, size_t cols, size_t rows, size_t d2,
+                         size_t row_pitch, size_t d2_pitch, int box_rows) {
+    katsu_tensor_map_encode_fn encode = katsu_tensor_map_encoder();
+    if (encode == nullptr) return false;
+    cuuint64_t dims[3] = {cols, rows, d2};
+    cuuint64_t strides[2] = {row_pitch * 2, d2_pitch * 2};
+    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1}, estr[3] = {1, 1, 1};
+    for (int i = 0; i < count; ++i)
+        if (encode(maps + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, planes.base + i * planes.stride, dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    return true;
+}
+
+bool katsu_f16_window_maps(CUtensorMap *maps, const KatsuF16Planes &planes, long long offset, int count, size_t channels,
+                           size_t width, size_t height, size_t images, size_t w_pitch, size_t h_pitch, size_t n_pitch,
+                           int step_h, int box_channels, const KatsuF16Box &box) {
+    katsu_tensor_map_encode_fn encode = katsu_tensor_map_encoder();
+    if (encode == nullptr) return false;
+    cuuint64_t dims[4] = {channels, width, height, images};
+    cuuint64_t strides[3] = {w_pitch * 2, h_pitch * 2, n_pitch * 2};
+    cuuint32_t gbox[4] = {(cuuint32_t)box_channels, (cuuint32_t)box.bw, (cuuint32_t)((box.bh - 1) * step_h + 1), (cuuint32_t)box.nb};
+    cuuint32_t estr[4] = {1, 1, (cuuint32_t)step_h, 1};
+    for (int i = 0; i < count; ++i)
+        if (encode(maps + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, planes.base + offset + i * (long long)planes.stride, dims, strides,
+                   gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box_channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    return true;
+}
+
+// Boxes narrower than 8 pixels (and than the grid) scatter the result over half-used 32-byte sectors and are taken only
+// when they save a tenth of the lanes or more; among equals wide boxes of few images go first.
+KatsuF16Box katsu_f16_box(int lanes, bool exact, int step_h, size_t width, size_t height, size_t images) {
+    KatsuF16Box best = {0, 0, 0, 0, 0, 0};
+    const unsigned w = (unsigned)width, h = (unsigned)height, n = (unsigned)images;
+    const unsigned most_h = 255 / step_h + 1;  // a tensor map's box spans at most 256 rows of the tensor
+    double best_cost = 0;
+    auto consider = [&](unsigned bw, unsigned bh, unsigned nb) {
+        if (bh > most_h) return;
+        const unsigned bx = (w + bw - 1) / bw, by = (h + bh - 1) / bh, bn = (n + nb - 1) / nb;
+        double cost = double(bx) * double(by) * double(bn);
+        if (!exact && bw < 8 && bw < w) cost *= 1.1 * 8 / (bw + 7);
+        if (best.bw == 0 || cost < best_cost) {
+            best = {(int)bw, (int)bh, (int)nb, (int)bx, (int)by, (long long)bx * by * bn};
+            best_cost = cost;
+        }
+    };
+    if (exact) {
+        for (int bw = lanes; bw >= 1; bw >>= 1)
+            for (int bh = lanes / bw; bh >= 1; bh >>= 1) consider(bw, bh, lanes / (bw * bh));
+        return best;
+    }
+    auto of_width = [&](unsigned bw) {
+        if (bw > (unsigned)lanes) return;
+        const unsigned rest = lanes / bw;
+        auto of_height = [&](unsigned bh) {
+            if (bh > rest || bh > h) return;
+            const unsigned nb = rest / bh;
+            consider(bw, bh, nb < n ? nb : n);
+        };
+        of_height(rest < h ? rest : h);
+        for (unsigned parts = 1; parts <= 6 && parts <= h; ++parts) of_height((h + parts - 1) / parts);
+        for (unsigned bh = 16; bh >= 1; bh >>= 1) of_height(bh);
+    };
+    for (unsigned parts = 1; parts <= 8 && parts <= w; ++parts) of_width((w + parts - 1) / parts);
+    for (unsigned bw = 64; bw >= 4; bw >>= 1)
+        if (bw <= w) of_width(bw);
+    return best;
+}

@@ -1,0 +1,129 @@
+// Operands of the fp16 tensor-core path: f32 tensors as one or two fp16 planes with a common power-of-two scale.
+//
+// A tensor v is held as v * 2^exp ~ hi + lo with hi = fp16(v * 2^exp) and lo = fp16(v * 2^exp - hi), both rounded to
+// nearest; exp places the largest magnitude in [2^14, 2^15).  hi alone carries the 11 significand bits of TF32, hi + lo
+// carry 22, what the two TF32 parts of 3xTF32 carry (there both parts are truncated), and the tensor core multiplies
+// fp16 at twice the rate of TF32 from half the bytes.  Products of fp16 values are exact in the f32 accumulator, and
+// 2^-(exp_a + exp_b) is applied to the f32 sums, so the scale itself costs no rounding.
+//
+// What fp16 lacks is range.  Below 2^-14 it goes subnormal: an element's error never exceeds 2^-25 of the scaled
+// range = 2^-39 of the tensor's largest magnitude.  The pass that finds that magnitude therefore also finds the
+// SMALLEST maximum over all groups of 128 consecutive elements that are not all zero, and a tensor counts as narrow
+// only if every group's maximum is within 2^17 of the tensor's (two planes) or 2^28 (one plane): then no element's
+// error exceeds 2^-22 (2^-11) of the largest magnitude in its own neighbourhood, which is the bar of the TF32 forms.
+//
+// If one operand of a call has a wider range, or holds infinities or NaNs, all of the call's operands are written as
+// bf16 planes instead: each the leading 8 significand bits of what the planes before it left, three of them (two in
+// TF32 mode), no scale.  bf16 has the exponents of f32, and three planes hold all 24 bits.  The products kept are
+// those down to 2^-16 (six; three in TF32 mode), at the cost of 3xTF32.  The choice is made on the device, by every
+// kernel of the call from the same KatsuF16Info values; no value crosses to the host.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+
+struct KatsuF16Info {
+    int narrow;  // 1: fp16 planes can stand for the tensor
+    int exp;     // scale exponent of those
+};
+
+// The operands of one call (unused entries null).
+struct KatsuF16Call {
+    const KatsuF16Info *info[3];
+};
+
+__device__ __forceinline__ bool katsu_f16_wide(const KatsuF16Call &call) {
+    bool narrow = true;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (call.info[i]) narrow = narrow && call.info[i]->narrow;
+    return !narrow;
+}
+
+// One operand whose magnitude is to be found.
+struct KatsuAmaxJob {
+    const float *src;
+    size_t count;
+    KatsuF16Info *info;
+};
+
+enum KatsuStageKind { KATSU_STAGE_NHWC, KATSU_STAGE_ROWS, KATSU_STAGE_WEIGHTS };
+
+// Fp16 planes of a tensor: plane i starts i * stride elements behind the first.  Room for one more than the mode's
+// narrow form needs.
+struct KatsuF16Planes {
+    __half *base;
+    size_t stride;
+};
+
+// One operand to be written as planes.
+//   NHWC     src [n][c][h * w] -> [n][h][w + gap][cp], channels padded with zeros to cp (a multiple of 8), `gap` zero
+//            pixels behind every row and in front of the first; `tail` more zero elements behind the last row.
+//            (n = 1, h = 1, gap = 0 is a transposed matrix.)
+//   ROWS     src [n][c] -> [n][cp]
+//   WEIGHTS  src [k][c][r][s] -> [r][rows][width]; backward = 0: rows are k and column kx * cp + c is tap kx;
+//            backward = 1: rows are c and the columns of x-parity class j start at col_begin[j], tap t of the class
+//            (kx = kx_last[j] - t * stride) holding cp columns, channel k innermost.
+struct KatsuStageJob {
+    int kind;
+    const float *src;
+    KatsuF16Planes to;
+    const KatsuF16Info *info;
+    int only_if_mixed;  // 1: written only when this operand is narrow and the call is not (a narrow copy exists already)
+    int n, c, h, w, gap, cp, tail;
+    int k, r, s, width, backward, classes, stride;
+    int col_begin[8], kx_last[8], class_taps[8];
+};
+
+// Largest magnitude and usability of up to three operands, one launch.
+int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count);
+// Writes up to KATSU_STAGE_JOBS operands' planes, one launch.
+constexpr int KATSU_STAGE_JOBS = 4;
+int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const KatsuStageJob *jobs, int count);
+
+// Planes of the narrow form in the context's mode, and of room for either form.
+static inline int katsu_f16_narrow_planes(const katsu_cuda_ctx *ctx) { return ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1; }
+
+// Device slots for the operands of one call.
+enum { KATSU_INFO_A, KATSU_INFO_B, KATSU_INFO_G, KATSU_INFO_SLOTS };
+KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot);
+
+// Bump allocator over a scratch block; every piece is 256-byte aligned.
+struct KatsuArena {
+    char *base;
+    size_t bytes;
+    void *take(size_t n) {
+        void *p = base + bytes;
+        bytes += (n + 255) / 256 * 256;
+        return p;
+    }
+    KatsuF16Planes planes(size_t n, int count) {
+        KatsuF16Planes p;
+        p.stride = (n + 127) / 128 * 128;
+        p.base = static_cast<__half *>(take(p.stride * count * sizeof(__half)));
+        return p;
+    }
+    float *floats(size_t n) { return static_cast<float *>(take(n * sizeof(float))); }
+};
+
+static inline size_t katsu_round_up(size_t n, size_t to) { return (n + to - 1) / to * to; }
+
+// The fp16 path of matmul (f16_matmul.cu); *handled = 0 when the shape or mode is not one it takes.
+int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b, float *c, size_t m, size_t k, size_t n,
+                             int *handled);
+int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b, const float *g, float *da, float *db,
+                             size_t m, size_t k, size_t n, int accumulate, int *handled);
+
+// The fp16 path of the convolutions (f16_conv.cu), *handled as above.
+bool katsu_f16_conv_geometry(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
+                             size_t s, size_t stride, size_t pad, size_t oh, size_t ow);
+size_t katsu_f16_conv_staged_bytes(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w);
+int32_t katsu_f16_conv_stage(katsu_cuda_ctx *ctx, const float *x, void *staged, size_t n, size_t c, size_t h, size_t w);
+int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, const float *bias, int relu, float *y,
+                           size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r, size_t s, size_t stride, size_t pad,
+                           size_t oh, size_t ow, int *handled);
+int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, const float *gr, const float *gscale,
+                           float gfactor, float *dx, float *dw, size_t n, size_t c, size_t h, size_t wd, size_t k, size_t r,
+                           size_t s, size_t stride, size_t pad, size_t oh, size_t ow, int accumulate,
+                           int *handled);

@@ -1,0 +1,418 @@
+// The passes in front of the fp16 tensor-core kernels: the largest magnitude of an operand with the range check, and
+// the operand's fp16 planes in the layout its kernel loads (f16_split.cuh).
+//
+// Both are bound by HBM: the first reads the operand once (4 bytes an element), the second reads it again (from L2
+// when the operand fits there) and writes 2 or 4 bytes an element.  Up to three operands share a launch, because in
+// small calls a launch costs more than the pass.
+#include "f16_split.cuh"
+
+namespace {
+
+constexpr int THREADS = 256;
+
+// ---- largest magnitude ------------------------------------------------------------------------------------------
+struct AmaxAcc {
+    unsigned amax, inverted_min, ticket, pad;
+};
+
+struct AmaxSegment {
+    const float *src;
+    unsigned long long count;
+    KatsuF16Info *info;
+    AmaxAcc *acc;
+    unsigned first_block, blocks;
+};
+
+struct AmaxParams {
+    AmaxSegment seg[3];
+    int segments;
+    int span;  // groups must reach 2^-span of the tensor's maximum
+};
+
+__device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned max4(float4 v) {
+    return max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w)));
+}
+
+// A group is the 128 consecutive floats that a warp reads at once; the last group of a tensor reaches back so that
+// it is a full one.  Magnitudes compare as their bit patterns, which puts infinities and NaNs above every number.
+__global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ AmaxParams p) {
+    int si = 0;
+    while (si + 1 < p.segments && blockIdx.x >= p.seg[si + 1].first_block) ++si;
+    const AmaxSegment &sg = p.seg[si];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned long long groups = (sg.count + 127) / 128;
+    const unsigned long long stride = (unsigned long long)sg.blocks * (THREADS / 32);
+    const bool vec = (reinterpret_cast<uintptr_t>(sg.src) & 15u) == 0;
+    unsigned most = 0, least = 0x7fffffffu;
+    auto load = [&](unsigned long long g) -> unsigned {
+        unsigned long long at = g * 128;
+        unsigned m = 0;
+        if (at + 128 <= sg.count && vec) {
+            m = max4(__ldg(reinterpret_cast<const float4 *>(sg.src + at) + lane));
+        } else {
+            if (at + 128 > sg.count) at = sg.count > 128 ? sg.count - 128 : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned long long e = at + lane + 32 * i;
+                if (e < sg.count) m = max(m, magnitude(__ldg(sg.src + e)));
+            }
+        }
+        return m;
+    };
+    auto take = [&](unsigned m) {
+        m = __reduce_max_sync(0xffffffffu, m);
+        most = max(most, m);
+        if (m != 0) least = min(least, m);
+    };
+    unsigned long long g = (unsigned long long)(blockIdx.x - sg.first_block) * (THREADS / 32) + warp;
+    for (; g + 7 * stride < groups; g += 8 * stride) {  // eight 16-byte loads in flight per thread
+        unsigned m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = load(g + i * stride);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) take(m[i]);
+    }
+    for (; g < groups; g += stride) take(load(g));
+
+    __shared__ unsigned sh_most[THREADS / 32], sh_least[THREADS / 32];
+    if (lane == 0) {
+        sh_most[warp] = most;
+        sh_least[warp] = least;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int i = 1; i < THREADS / 32; ++i) {
+        most = max(most, sh_most[i]);
+        least = min(least, sh_least[i]);
+    }
+    atomicMax(&sg.acc->amax, most);
+    atomicMax(&sg.acc->inverted_min, 0x7fffffffu - least);
+    __threadfence();
+    if (atomicAdd(&sg.acc->ticket, 1u) != sg.blocks - 1) return;
+    // last block of the segment: publish, and leave the accumulator as the next launch wants to find it
+    __threadfence();
+    most = atomicExch(&sg.acc->amax, 0u);
+    least = 0x7fffffffu - atomicExch(&sg.acc->inverted_min, 0u);
+    atomicExch(&sg.acc->ticket, 0u);
+    KatsuF16Info info;
+    const int exponent = int(most >> 23) - 127;  // floor(log2(amax)) of a normal number
+    info.exp = 14 - exponent;
+    // 2^-48 .. 2^48 keeps the product of two operands' scales inside f32
+    info.narrow = exponent >= -48 && exponent <= 48 && (int(most >> 23) - int(least >> 23)) < p.span;
+    if (most == 0) {  // all zeros
+        info.exp = 0;
+        info.narrow = 1;
+    }
+    *sg.info = info;
+}
+
+// ---- fp16 planes ------------------------------------------------------------------------------------------------
+struct StageParams {
+    KatsuF16Call call;
+    int narrow_planes;
+    KatsuStageJob job[KATSU_STAGE_JOBS];
+    unsigned first_block[KATSU_STAGE_JOBS], blocks[KATSU_STAGE_JOBS];
+    int jobs;
+};
+
+// How the values of one job are written.
+struct Writer {
+    KatsuF16Planes to;
+    float scale;
+    int planes;  // planes of the form in use
+    bool wide;
+};
+
+// Two scaled values as packed hi and lo halves.  Two values to a conversion: with one each, the conversion pipe and not
+// memory set the pace of these passes.
+__device__ __forceinline__ void split_narrow(float a, float b, unsigned *hi, unsigned *lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    *hi = *reinterpret_cast<const unsigned *>(&h);
+    *lo = *reinterpret_cast<const unsigned *>(&l);
+}
+
+// The leading 8 significand bits of v as a bf16 pattern in the upper half of a word, and what is left of v.  An infinity
+// or NaN is its first plane alone.
+__device__ __forceinline__ unsigned peel(float *v) {
+    unsigned bits = __float_as_uint(*v);
+    if ((bits & 0x7f800000u) == 0x7f800000u) {
+        if (bits & 0x007fffffu) bits |= 0x00400000u;  // a NaN stays one without its lower bits
+        *v = 0.f;
+        return bits & 0xffff0000u;
+    }
+    bits &= 0xffff0000u;
+    *v -= __uint_as_float(bits);
+    return bits;
+}
+
+__device__ __forceinline__ unsigned peel2(float *a, float *b) { return (peel(a) >> 16) | peel(b); }
+
+// Eight consecutive elements at `at` (16-byte aligned).
+__device__ __forceinline__ void write8(const Writer &w, size_t at, float (&v)[8]) {
+    if (!w.wide) {
+        uint4 hi, lo;
+        split_narrow(v[0] * w.scale, v[1] * w.scale, &hi.x, &lo.x);
+        split_narrow(v[2] * w.scale, v[3] * w.scale, &hi.y, &lo.y);
+        split_narrow(v[4] * w.scale, v[5] * w.scale, &hi.z, &lo.z);
+        split_narrow(v[6] * w.scale, v[7] * w.scale, &hi.w, &lo.w);
+        *reinterpret_cast<uint4 *>(w.to.base + at) = hi;
+        if (w.planes == 2) *reinterpret_cast<uint4 *>(w.to.base + w.to.stride + at) = lo;
+    } else {
+        for (int i = 0; i < w.planes; ++i) {
+            uint4 o;
+            o.x = peel2(&v[0], &v[1]);
+            o.y = peel2(&v[2], &v[3]);
+            o.z = peel2(&v[4], &v[5]);
+            o.w = peel2(&v[6], &v[7]);
+            *reinterpret_cast<uint4 *>(w.to.base + i * w.to.stride + at) = o;
+        }
+    }
+}
+
+__device__ __forceinline__ void zero8(const Writer &w, size_t at) {
+    for (int i = 0; i < w.planes; ++i) *reinterpret_cast<uint4 *>(w.to.base + i * w.to.stride + at) = make_uint4(0, 0, 0, 0);
+}
+
+// CT channels x 4096 / CT pixels through shared memory: 16-byte reads along pixels, 16-byte writes along channels (8 fp16
+// channels of a pixel to a thread).  The tile's columns are XORed with the channel group so that both sides are free of
+// bank conflicts: a warp writes one or two channel rows, and reads 8 channel groups of 4 pixels (CT = 64) or 4 groups of
+// 8 pixels (CT = 32).  Few instructions a value matter here: with a thread per channel pair, and a division per pixel and
+// channel, this pass was bound by instruction issue (0.20 ms for 103 M values, 4.1 TB/s).
+template <int CT>
+__device__ void stage_nhwc_tiles(const KatsuStageJob &j, const Writer &out, unsigned block, float *tile) {
+    constexpr int PT = 4096 / CT, GROUPS = CT / 8, XOR = 32 / GROUPS;
+    const int hw = j.h * j.w, ptiles = (hw + PT - 1) / PT, ctiles = (j.c + CT - 1) / CT;
+    const unsigned n = block / unsigned(ptiles * ctiles), rest = block - n * unsigned(ptiles * ctiles);
+    const int pt = rest / unsigned(ctiles);
+    const int p0 = pt * PT, c0 = (rest - pt * ctiles) * CT;
+    const float *src = j.src + (size_t(n) * j.c + c0) * hw + p0;
+    const int channels = min(j.c - c0, CT), pixels = min(hw - p0, PT);
+    if ((hw & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15u) == 0) {
+        // a float4 a thread: PT / 4 threads to a channel
+        const int quad = threadIdx.x % (PT / 4), row0 = threadIdx.x / (PT / 4);
+        constexpr int STEP = THREADS / (PT / 4);
+        float4 v[CT / STEP];
+#pragma unroll
+        for (int i = 0; i < CT / STEP; ++i) {
+            const int row = row0 + STEP * i;
+            v[i] = (row < channels && quad * 4 < pixels) ? __ldg(reinterpret_cast<const float4 *>(src + size_t(row) * hw) + quad)
+                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < CT / STEP; ++i) {
+            const int row = row0 + STEP * i;
+            const int col = (quad * 4) ^ ((row >> 3) * XOR);
+            *reinterpret_cast<float4 *>(tile + row * PT + col) = v[i];
+        }
+    } else {
+        const int col0 = threadIdx.x % PT, row0 = threadIdx.x / PT;
+        constexpr int STEP = THREADS / PT;
+        float v[CT / STEP];
+#pragma unroll
+        for (int i = 0; i < CT / STEP; ++i) {
+            const int row = row0 + STEP * i;
+            v[i] = (row < channels && col0 < pixels) ? __ldg(src + size_t(row) * hw + col0) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < CT / STEP; ++i) {
+            const int row = row0 + STEP * i;
+            tile[row * PT + (col0 ^ ((row >> 3) * XOR))] = v[i];
+        }
+    }
+    __syncthreads();
+    const int g = threadIdx.x % GROUPS, first = threadIdx.x / GROUPS;
+    if (c0 + g * 8 >= j.cp) return;
+    constexpr int STEP = THREADS / GROUPS;
+    int y = (p0 + first) / j.w, x = (p0 + first) - y * j.w;
+    const float *column = tile + g * 8 * PT;
+#pragma unroll
+    for (int i = 0; i < PT / STEP; ++i) {
+        const int p = first + STEP * i;
+        if (p >= pixels) break;
+        const float *from = column + (p ^ (g * XOR));
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = from[u * PT];
+        const size_t at = ((size_t(n) * j.h + y) * (j.w + j.gap) + x) * j.cp + c0 + g * 8;
+        write8(out, at, v);
+        if (x == j.w - 1)
+            for (int q = 1; q <= j.gap; ++q) zero8(out, at + size_t(q) * j.cp);
+        x += STEP;
+        while (x >= j.w) {
+            x -= j.w;
+            ++y;
+        }
+    }
+}
+
+// Channels to a tile: 32 where that many are all there are, or where 64 would leave half a tile or more empty.
+__host__ __device__ inline int tile_channels(int c) { return ((c + 31) / 32) & 1 && c < 160 ? 32 : 64; }
+
+// Up to 16 channels: a thread per pixel and 8 channels, no transposition needed for whole-sector writes.
+__device__ void stage_nhwc_narrow(const KatsuStageJob &j, const Writer &out, unsigned block, unsigned blocks) {
+    const int hw = j.h * j.w, eights = j.cp / 8;
+    const size_t pixels = size_t(j.n) * hw, total = pixels * eights;
+    for (size_t i = size_t(block) * THREADS + threadIdx.x; i < total; i += size_t(blocks) * THREADS) {
+        const int e = int(i / pixels);
+        const size_t q = i - size_t(e) * pixels;
+        const int n = int(q / hw), p = int(q - size_t(n) * hw);
+        const int y = p / j.w, x = p - y * j.w;
+        const float *src = j.src + (size_t(n) * j.c + e * 8) * hw + p;
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = (e * 8 + u < j.c) ? __ldg(src + size_t(u) * hw) : 0.f;
+        const size_t at = ((size_t(n) * j.h + y) * (j.w + j.gap) + x) * j.cp + e * 8;
+        write8(out, at, v);
+        if (x == j.w - 1)
+            for (int q2 = 1; q2 <= j.gap; ++q2) zero8(out, at + size_t(q2) * j.cp);
+    }
+}
+
+__device__ void stage_rows(const KatsuStageJob &j, const Writer &out, unsigned block, unsigned blocks) {
+    const unsigned eights = j.cp / 8;
+    const size_t total = size_t(j.n) * eights;
+    const bool vec = (j.c & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15u) == 0;
+    for (size_t i = size_t(block) * THREADS + threadIdx.x; i < total; i += size_t(blocks) * THREADS) {
+        const size_t row = i / eights;
+        const int c0 = int(i - row * eights) * 8;
+        const float *src = j.src + row * j.c + c0;
+        float v[8];
+        if (vec && c0 + 8 <= j.c) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = c0 + u < j.c ? __ldg(src + u) : 0.f;
+        }
+        write8(out, i * 8, v);
+    }
+}
+
+// Eight columns of one weight row to a thread; cp and every class's first column are multiples of 8.
+__device__ void stage_weights(const KatsuStageJob &j, const Writer &out, unsigned block, unsigned blocks) {
+    const int rows = j.backward ? j.c : j.k, inner = j.backward ? j.k : j.c;
+    const unsigned eights = j.width / 8, taps = j.r * j.s;
+    const size_t total = size_t(j.r) * rows * eights;
+    const size_t step = j.backward ? size_t(j.c) * taps : taps;  // between channels of the contraction
+    for (size_t i = size_t(block) * THREADS + threadIdx.x; i < total; i += size_t(blocks) * THREADS) {
+        const int col = int(i % eights) * 8;
+        const size_t rest = i / eights;
+        const int row = int(rest % rows), ky = int(rest / rows);
+        int kx, ch;
+        bool live;
+        if (j.backward) {
+            int q = 0;
+            while (q + 1 < j.classes && col >= j.col_begin[q + 1]) ++q;
+            const int t = (col - j.col_begin[q]) / j.cp;
+            ch = (col - j.col_begin[q]) - t * j.cp;
+            kx = j.kx_last[q] - t * j.stride;
+            live = t < j.class_taps[q];
+        } else {
+            kx = col / j.cp;
+            ch = col - kx * j.cp;
+            live = true;
+        }
+        const float *src = j.src + (j.backward ? size_t(ch) * step + size_t(row) * taps : size_t(row) * j.c * taps + size_t(ch) * taps) +
+                           ky * j.s + kx;
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = (live && ch + u < inner) ? __ldg(src + u * step) : 0.f;
+        write8(out, i * 8, v);
+    }
+}
+
+__global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ StageParams p) {
+    __shared__ __align__(16) float tile[4096];
+    int ji = 0;
+    while (ji + 1 < p.jobs && blockIdx.x >= p.first_block[ji + 1]) ++ji;
+    const KatsuStageJob &j = p.job[ji];
+    const unsigned block = blockIdx.x - p.first_block[ji];
+    Writer out;
+    out.to = j.to;
+    out.wide = katsu_f16_wide(p.call);
+    out.planes = p.narrow_planes + (out.wide ? 1 : 0);
+    out.scale = out.wide ? 1.f : __uint_as_float(unsigned(127 + j.info->exp) << 23);
+    if (j.only_if_mixed && !(out.wide && j.info->narrow)) return;
+    if (j.kind == KATSU_STAGE_NHWC) {
+        if (block == 0) {
+            // zero pixels in front of the first row, zeros behind the last
+            for (int i = threadIdx.x * 8; i < j.gap * j.cp; i += THREADS * 8) {
+                Writer front = out;
+                front.to.base -= size_t(j.gap) * j.cp;
+                zero8(front, i);
+            }
+            const size_t end = size_t(j.n) * j.h * (j.w + j.gap) * j.cp;
+            for (int i = threadIdx.x * 8; i < j.tail; i += THREADS * 8) zero8(out, end + i);
+        }
+        if (j.c <= 16) stage_nhwc_narrow(j, out, block, p.blocks[ji]);
+        else if (tile_channels(j.c) == 32) stage_nhwc_tiles<32>(j, out, block, tile);
+        else stage_nhwc_tiles<64>(j, out, block, tile);
+    } else if (j.kind == KATSU_STAGE_ROWS) {
+        stage_rows(j, out, block, p.blocks[ji]);
+    } else {
+        stage_weights(j, out, block, p.blocks[ji]);
+    }
+}
+
+}  // namespace
+
+KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) {
+    return reinterpret_cast<KatsuF16Info *>(static_cast<char *>(ctx->f16_state) + 256) + slot;
+}
+
+int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count) {
+    AmaxParams p;
+    p.segments = count;
+    p.span = ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28;
+    unsigned at = 0;
+    for (int i = 0; i < count; ++i) {
+        AmaxSegment &s = p.seg[i];
+        s.src = jobs[i].src;
+        s.count = jobs[i].count;
+        s.info = jobs[i].info;
+        s.acc = static_cast<AmaxAcc *>(ctx->f16_state) + i;
+        // a warp takes eight groups of 128 at once; at most eight resident blocks per SM
+        size_t blocks = katsu_div_up(jobs[i].count, size_t(128) * 8 * (THREADS / 32));
+        if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
+        if (blocks < 1) blocks = 1;
+        s.first_block = at;
+        s.blocks = (unsigned)blocks;
+        at += s.blocks;
+    }
+    KATSU_LAUNCH(ctx, amax_kernel, at, THREADS, 0, p);
+    return KATSU_OK;
+}
+
+int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const KatsuStageJob *jobs, int count) {
+    StageParams p;
+    p.call = call;
+    p.narrow_planes = katsu_f16_narrow_planes(ctx);
+    p.jobs = count;
+    size_t at = 0;
+    for (int i = 0; i < count; ++i) {
+        const KatsuStageJob &j = jobs[i];
+        p.job[i] = j;
+        size_t blocks;
+        const size_t hw = size_t(j.h) * j.w;
+        if (j.kind == KATSU_STAGE_NHWC && j.c > 16) {
+            const size_t ct = tile_channels(j.c);
+            blocks = size_t(j.n) * katsu_div_up(hw, 4096 / ct) * katsu_div_up((size_t)j.c, ct);
+        } else {
+            const size_t units = j.kind == KATSU_STAGE_NHWC ? size_t(j.n) * hw * (j.cp / 8)
+                                 : j.kind == KATSU_STAGE_ROWS ? size_t(j.n) * (j.cp / 8)
+                                                              : size_t(j.r) * (j.backward ? j.c : j.k) * (j.width / 8);
+            blocks = katsu_div_up(units, (size_t)THREADS);
+            if (blocks > size_t(ctx->num_sms) * 64) blocks = size_t(ctx->num_sms) * 64;
+        }
+        p.first_block[i] = (unsigned)at;
+        p.blocks[i] = (unsigned)blocks;
+        at += blocks;
+    }
+    if (at > 0x7fffffffu) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "operand too large to stage");
+    KATSU_LAUNCH(ctx, stage_kernel, (unsigned)at, THREADS, 0, p);
+    return KATSU_OK;
+}

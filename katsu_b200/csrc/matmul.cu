@@ -11,6 +11,7 @@
 //  * a general 64x64-tile kernel with arbitrary element strides, so the same
 //    code serves a@b, g@b^T and a^T@g without materialising a transpose.
 #include "common.cuh"
+#include "f16_split.cuh"
 
 namespace {
 
@@ -413,7 +414,7 @@ extern "C" int32_t katsu_cuda_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, co
 #undef CALL
     }
     int handled = 0;
-    KATSU_TRY(katsu_umma_gemm(ctx, a, b, c, m, n, k, false, true, 0, &handled));
+    KATSU_TRY(katsu_f16_matmul_fwd(ctx, a, b, c, m, k, n, &handled));
     if (handled) return KATSU_OK;
     return gemm_strided(ctx, a, b, c, m, n, k, k, 1, n, 1, 0);
 }
@@ -435,6 +436,10 @@ extern "C" int32_t katsu_cuda_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, co
     // da == db (the reference's "same parent on both edges", tensor.rs:425-444, possible when
     // m == k == n): the second product is added to the first whatever `accumulate` says.
     const int accumulate_db = (da != nullptr && da == db) ? 1 : accumulate;
+    int f16 = 0;
+    if (!skinny && (da != nullptr || db != nullptr))
+        KATSU_TRY(katsu_f16_matmul_bwd(ctx, a, b, g, da, db, m, k, n, accumulate, &f16));
+    if (f16) return KATSU_OK;
     if (da != nullptr) {
         if (skinny) {
 #define CALL(NP) skinny_da<NP>(ctx, g, b, da, m, k, n, accumulate)
@@ -442,10 +447,8 @@ extern "C" int32_t katsu_cuda_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, co
 #undef CALL
             KATSU_TRY(rc);
         } else {
-            // da[m,k] = g[m,n] @ b^T : A(i,p)=g[i*n+p], B(p,j)=b[j*n+p]  (both K-major for the tensor cores)
-            int handled = 0;
-            KATSU_TRY(katsu_umma_gemm(ctx, g, b, da, m, k, n, false, false, accumulate, &handled));
-            if (!handled) KATSU_TRY(gemm_strided(ctx, g, b, da, m, k, n, n, 1, 1, n, accumulate));
+            // da[m,k] = g[m,n] @ b^T : A(i,p)=g[i*n+p], B(p,j)=b[j*n+p]
+            KATSU_TRY(gemm_strided(ctx, g, b, da, m, k, n, n, 1, 1, n, accumulate));
         }
     }
     if (db != nullptr) {
@@ -455,10 +458,8 @@ extern "C" int32_t katsu_cuda_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, co
 #undef CALL
             KATSU_TRY(rc);
         } else {
-            // db[k,n] = a^T @ g : A(i,p)=a[p*k+i], B(p,j)=g[p*n+j]  (both MN-major for the tensor cores)
-            int handled = 0;
-            KATSU_TRY(katsu_umma_gemm(ctx, a, g, db, k, n, m, true, true, accumulate_db, &handled));
-            if (!handled) KATSU_TRY(gemm_strided(ctx, a, g, db, k, n, m, 1, k, n, 1, accumulate_db));
+            // db[k,n] = a^T @ g : A(i,p)=a[p*k+i], B(p,j)=g[p*n+j]
+            KATSU_TRY(gemm_strided(ctx, a, g, db, k, n, m, 1, k, n, 1, accumulate_db));
         }
     }
     return KATSU_OK;
