@@ -74,8 +74,12 @@ int32_t katsu_cuda_stream(katsu_cuda_ctx *ctx, void **out_stream);
  * synchronise the device.  A buffer must be freed through a context whose
  * stream has seen (or been synchronised with) its last use. */
 int32_t katsu_cuda_alloc(katsu_cuda_ctx *ctx, size_t count, float **out_ptr);
+/* The same without the zeros, for buffers that the next call overwrites. */
+int32_t katsu_cuda_alloc_uninit(katsu_cuda_ctx *ctx, size_t count, float **out_ptr);
 int32_t katsu_cuda_free(katsu_cuda_ctx *ctx, float *ptr);
 int32_t katsu_cuda_zero(katsu_cuda_ctx *ctx, float *dst, size_t count);
+/* dst[i] = value: the seed of a backward pass (tensor.rs:309-314) without a host buffer to copy from. */
+int32_t katsu_cuda_fill(katsu_cuda_ctx *ctx, float *dst, float value, size_t count);
 /* Explicit host<->device transfer for the device storage variant of
  * TensorNode.data (crates/katsu-core/src/tensor.rs:101-107).  d2h waits for the
  * stream (and, like katsu_cuda_sync, returns KATSU_ERR_TIMEOUT when a bounded

@@ -37,8 +37,10 @@ SIGNATURES = {
     "katsu_cuda_launch_count": [_ctx, ctypes.POINTER(ctypes.c_uint64)],
     "katsu_cuda_stream": [_ctx, ctypes.POINTER(ctypes.c_void_p)],
     "katsu_cuda_alloc": [_ctx, _sz, ctypes.POINTER(_ptr)],
+    "katsu_cuda_alloc_uninit": [_ctx, _sz, ctypes.POINTER(_ptr)],
     "katsu_cuda_free": [_ctx, _ptr],
     "katsu_cuda_zero": [_ctx, _ptr, _sz],
+    "katsu_cuda_fill": [_ctx, _ptr, ctypes.c_float, _sz],
     "katsu_cuda_h2d": [_ctx, _ptr, ctypes.c_void_p, _sz],
     "katsu_cuda_d2h": [_ctx, ctypes.c_void_p, _ptr, _sz],
     "katsu_cuda_d2h_async": [_ctx, ctypes.c_void_p, _ptr, _sz],

@@ -37,6 +37,8 @@ struct katsu_cuda_ctx {
     int *status_host;
     // cudaMemPool_t private to the context: katsu_cuda_alloc and the scratch come from it.
     void *pool;
+    // Freed blocks kept for the next katsu_cuda_alloc of their size (context.cu).
+    struct KatsuBlockCache *blocks;
     // NCCL communicator (void* so this header does not need nccl.h).
     void *comm;
     int comm_ranks;

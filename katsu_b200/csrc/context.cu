@@ -2,10 +2,13 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <stdlib.h>
+
+#include <map>
 #include <new>
+#include <unordered_map>
 
 #include "common.cuh"
-#include <stdlib.h>
 
 static thread_local char g_error[512] = "";
 
@@ -23,6 +26,69 @@ int32_t katsu_bind(katsu_cuda_ctx *ctx) {
     if (ctx == nullptr) return katsu_set_error(KATSU_ERR_INVALID_ARG, "null context");
     KATSU_CUDA_TRY(cudaSetDevice(ctx->device));
     return KATSU_OK;
+}
+
+// ---- freed blocks ----------------------------------------------------------------------------------------------
+// A training step frees and allocates the same few buffers of up to hundreds of megabytes.  The pool serves that from
+// cached memory only while it finds a fitting piece; when steps of different sizes alternate it maps and unmaps physical
+// memory inside a step (the small CNN's step took 3 to 40 ms that way, 2 ms of it kernels).  So a freed block stays
+// whole and goes to the next request of nearly its size.  All use of a context's blocks is on its one stream, so reuse
+// needs no event, and one host thread drives a context.  At most an eighth of the device's memory is held; an allocation
+// that fails gives everything held back and tries again; shutdown gives everything back.
+struct KatsuBlockCache {
+    std::unordered_map<void *, size_t> sizes;  // of every block this context has handed out or holds
+    std::multimap<size_t, void *> held;
+    size_t held_bytes = 0, most_bytes = 0;
+};
+
+static size_t block_bytes(size_t bytes) {
+    const size_t grain = bytes < (size_t(1) << 20) ? 512 : size_t(2) << 20;
+    return (bytes + grain - 1) / grain * grain;
+}
+
+static void give_back_blocks(katsu_cuda_ctx *ctx) {
+    KatsuBlockCache &cache = *ctx->blocks;
+    for (auto &entry : cache.held) {
+        cache.sizes.erase(entry.second);
+        cudaFreeAsync(entry.second, ctx->stream);
+    }
+    cache.held.clear();
+    cache.held_bytes = 0;
+}
+
+static int32_t take_block(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
+    KatsuBlockCache &cache = *ctx->blocks;
+    const size_t want = block_bytes(bytes);
+    auto it = cache.held.lower_bound(want);
+    if (it != cache.held.end() && it->first <= want + want / 8) {
+        *out = it->second;
+        cache.held_bytes -= it->first;
+        cache.held.erase(it);
+        return KATSU_OK;
+    }
+    int32_t rc = katsu_pool_alloc(ctx, want, out);
+    if (rc != KATSU_OK && !cache.held.empty()) {
+        give_back_blocks(ctx);
+        cudaStreamSynchronize(ctx->stream);
+        rc = katsu_pool_alloc(ctx, want, out);
+    }
+    if (rc == KATSU_OK) cache.sizes[*out] = want;
+    return rc;
+}
+
+// False when the block is not one of this context's (another context of the device handed it out).
+static bool keep_block(katsu_cuda_ctx *ctx, void *ptr) {
+    KatsuBlockCache &cache = *ctx->blocks;
+    auto it = cache.sizes.find(ptr);
+    if (it == cache.sizes.end()) return false;
+    const size_t bytes = it->second;
+    if (cache.held_bytes + bytes > cache.most_bytes) {
+        cache.sizes.erase(it);
+        return false;
+    }
+    cache.held.emplace(bytes, ptr);
+    cache.held_bytes += bytes;
+    return true;
 }
 
 int32_t katsu_pool_alloc(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
@@ -107,6 +173,12 @@ extern "C" int32_t katsu_cuda_init(int32_t device, katsu_cuda_ctx **out_ctx) {
     ctx->device = device;
     ctx->num_sms = prop.multiProcessorCount;
     ctx->precision = KATSU_MODE_3XTF32;
+    ctx->blocks = new (std::nothrow) KatsuBlockCache();
+    if (ctx->blocks == nullptr) {
+        delete ctx;
+        return katsu_set_error(KATSU_ERR_ALLOC, "out of host memory");
+    }
+    ctx->blocks->most_bytes = prop.totalGlobalMem / 8;
     // katsu_cuda_alloc / katsu_cuda_free and the kernels' scratch are stream-ordered allocations
     // from a pool private to this context that keeps freed blocks cached: an autograd step
     // allocates and frees the same few hundred MB of adjoint buffers every time, and cudaMalloc /
@@ -141,6 +213,7 @@ extern "C" int32_t katsu_cuda_init(int32_t device, katsu_cuda_ctx **out_ctx) {
         if (ctx->stream) cudaStreamDestroy(ctx->stream);
         if (ctx->pool) cudaMemPoolDestroy((cudaMemPool_t)ctx->pool);
         cudaGetLastError();
+        delete ctx->blocks;
         delete ctx;
         return katsu_set_error(KATSU_ERR_CUDA, "context setup: %s", cudaGetErrorString(err));
     }
@@ -156,6 +229,7 @@ extern "C" int32_t katsu_cuda_shutdown(katsu_cuda_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->comm) katsu_comm_destroy_impl(ctx);
     if (ctx->scratch) cudaFreeAsync(ctx->scratch, ctx->stream);
+    give_back_blocks(ctx);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->flush) cudaFree(ctx->flush);
     if (ctx->status) cudaFree(ctx->status);
@@ -165,6 +239,7 @@ extern "C" int32_t katsu_cuda_shutdown(katsu_cuda_ctx *ctx) {
     // blocks still held by the caller stay valid: the driver releases the pool with its last allocation
     if (ctx->pool) cudaMemPoolDestroy((cudaMemPool_t)ctx->pool);
     cudaGetLastError();
+    delete ctx->blocks;
     delete ctx;
     return KATSU_OK;
 }
@@ -196,21 +271,28 @@ extern "C" int32_t katsu_cuda_stream(katsu_cuda_ctx *ctx, void **out_stream) {
 }
 
 // ---- memory ----------------------------------------------------------------
-extern "C" int32_t katsu_cuda_alloc(katsu_cuda_ctx *ctx, size_t count, float **out_ptr) {
+extern "C" int32_t katsu_cuda_alloc_uninit(katsu_cuda_ctx *ctx, size_t count, float **out_ptr) {
     KATSU_REQUIRE(out_ptr != nullptr, "out_ptr is null");
     *out_ptr = nullptr;
     KATSU_TRY(katsu_bind(ctx));
     if (count == 0) return KATSU_OK;
-    if (count > SIZE_MAX / sizeof(float))
+    if (count > SIZE_MAX / sizeof(float) / 2)
         return katsu_set_error(KATSU_ERR_ALLOC, "allocation of %zu floats overflows", count);
-    float *p = nullptr;
-    KATSU_TRY(katsu_pool_alloc(ctx, count * sizeof(float), (void **)&p));
-    cudaError_t err = cudaMemsetAsync(p, 0, count * sizeof(float), ctx->stream);
+    void *p = nullptr;
+    KATSU_TRY(take_block(ctx, count * sizeof(float), &p));
+    *out_ptr = (float *)p;
+    return KATSU_OK;
+}
+
+extern "C" int32_t katsu_cuda_alloc(katsu_cuda_ctx *ctx, size_t count, float **out_ptr) {
+    KATSU_TRY(katsu_cuda_alloc_uninit(ctx, count, out_ptr));
+    if (count == 0) return KATSU_OK;
+    cudaError_t err = cudaMemsetAsync(*out_ptr, 0, count * sizeof(float), ctx->stream);
     if (err != cudaSuccess) {
-        cudaFreeAsync(p, ctx->stream);
+        katsu_cuda_free(ctx, *out_ptr);
+        *out_ptr = nullptr;
         return katsu_set_error(KATSU_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(err));
     }
-    *out_ptr = p;
     return KATSU_OK;
 }
 
@@ -219,7 +301,7 @@ extern "C" int32_t katsu_cuda_free(katsu_cuda_ctx *ctx, float *ptr) {
     if (ptr == nullptr) return KATSU_OK;
     // Stream-ordered: work already queued on this context's stream may still use the block;
     // work queued on another context must have been synchronised by the caller.
-    KATSU_CUDA_TRY(cudaFreeAsync(ptr, ctx->stream));
+    if (!keep_block(ctx, ptr)) KATSU_CUDA_TRY(cudaFreeAsync(ptr, ctx->stream));
     return KATSU_OK;
 }
 

@@ -89,8 +89,12 @@ size_t element_count(const std::vector<size_t> &shape) {
 // ---------------------------------------------------------------------------
 // storage
 // ---------------------------------------------------------------------------
-DeviceBuffer::DeviceBuffer(size_t n) : count(n) {
-    if (n != 0) check(katsu_cuda_alloc(device_context(), n, &ptr));
+DeviceBuffer::DeviceBuffer(size_t n, Fill fill) : count(n) {
+    if (n != 0) check((fill == Zeros ? katsu_cuda_alloc : katsu_cuda_alloc_uninit)(device_context(), n, &ptr));
+}
+
+static std::shared_ptr<DeviceBuffer> uninit_buffer(size_t n) {
+    return std::make_shared<DeviceBuffer>(n, DeviceBuffer::Uninit);
 }
 
 DeviceBuffer::~DeviceBuffer() {
@@ -120,7 +124,7 @@ struct Adjoint {
             if (!dense) dense = std::make_shared<DeviceBuffer>(numel);
             return dense->ptr;
         }
-        auto buffer = std::make_shared<DeviceBuffer>(numel);
+        auto buffer = std::make_shared<DeviceBuffer>(numel, kind == Bcast ? DeviceBuffer::Zeros : DeviceBuffer::Uninit);
         if (numel) {
             if (kind == Bcast)
                 check(katsu_cuda_bcast_acc(device_context(), buffer->ptr, scalar->ptr, numel));  // 0 + s
@@ -132,6 +136,38 @@ struct Adjoint {
         scalar.reset();
         source.reset();
         return dense->ptr;
+    }
+
+    // The dense buffer as the target of an addition: its own copy if another adjoint shares it (see share).
+    float *to_add() {
+        to_dense();
+        if (dense.use_count() > 1) {
+            auto own = uninit_buffer(numel);
+            if (numel) check(katsu_cuda_d2d(device_context(), own->ptr, dense->ptr, numel));
+            dense = std::move(own);
+        }
+        return dense->ptr;
+    }
+
+    // The buffer for a first contribution that overwrites every element (0 + v == v).
+    float *to_overwrite() {
+        if (kind != Dense || !dense || dense.use_count() > 1) {
+            dense = uninit_buffer(numel);
+            kind = Dense;
+            scalar.reset();
+            source.reset();
+        }
+        return dense->ptr;
+    }
+
+    // A first contribution that is another adjoint's values unchanged (Add, Reshape): both hold the one buffer, and
+    // whoever is added to later takes its own copy first.
+    void share(Adjoint &other) {
+        other.to_dense();
+        dense = other.dense;
+        kind = Dense;
+        scalar.reset();
+        source.reset();
     }
 };
 
@@ -158,14 +194,14 @@ struct TensorNode {
 
     const float *device() const {
         if (!dev) {
-            auto buffer = std::make_shared<DeviceBuffer>(numel);
+            auto buffer = uninit_buffer(numel);
             if (lazy_square) {
                 const float *p = parents[0].device_data();
                 if (numel) check(katsu_cuda_mul(device_context(), p, p, buffer->ptr, numel));
                 lazy_square = false;
             } else if (numel) {
+                // (from pageable memory: the call returns once the values have been staged)
                 check(katsu_cuda_h2d(device_context(), buffer->ptr, host.data(), numel));
-                check(katsu_cuda_sync(device_context()));
             }
             dev = std::move(buffer);
         }
@@ -261,7 +297,7 @@ static const float *staged_input(const Tensor &x, size_t n, size_t c, size_t h, 
     check(katsu_cuda_get_precision(ctx, &mode));
     const TensorNode &node = *x.node();
     if (!node.staged || node.staged->count != floats || node.staged_mode != mode) {
-        auto buffer = std::make_shared<DeviceBuffer>(floats);
+        auto buffer = uninit_buffer(floats);
         check(katsu_cuda_conv2d_stage(ctx, x.device_data(), buffer->ptr, n, c, h, w));
         node.staged = std::move(buffer);
         node.staged_mode = mode;
@@ -334,7 +370,7 @@ Tensor Tensor::elementwise(const Tensor &rhs, Op::Kind kind) const {
     if (shape() != rhs.shape()) fail(ErrorKind::ShapeMismatch);
     // y * y: the values wait until somebody reads them; sum() and backward never need them stored
     if (kind == Op::Mul && g_loss_fusion && id() == rhs.id()) return make_lazy_square(*this);
-    auto out = std::make_shared<DeviceBuffer>(numel());
+    auto out = uninit_buffer(numel());
     const float *a = node_->device();
     const float *b = rhs.node_->device();
     if (kind == Op::Add)
@@ -351,7 +387,7 @@ Tensor Tensor::mul(const Tensor &rhs) const { return elementwise(rhs, Op::Mul); 
 
 // tensor.rs:243-247 (tree order on the device instead of a left fold)
 Tensor Tensor::sum() const {
-    auto out = std::make_shared<DeviceBuffer>(1);
+    auto out = uninit_buffer(1);
     if (node_->lazy_square && !node_->dev)  // sum(p * p) in one pass over p, bit-identical to mul then sum
         check(katsu_cuda_sumsq(device_context(), node_->parents[0].device_data(), out->ptr, numel()));
     else
@@ -367,7 +403,7 @@ Tensor Tensor::matmul(const Tensor &rhs) const {
     const size_t m = shape()[0], k = shape()[1], n = rhs.shape()[1];
     if (k != rhs.shape()[0]) fail(ErrorKind::MatmulMismatch, "", k, rhs.shape()[0]);
     const size_t count = element_count({m, n});
-    auto out = std::make_shared<DeviceBuffer>(count);
+    auto out = std::make_shared<DeviceBuffer>(count, k != 0 ? DeviceBuffer::Uninit : DeviceBuffer::Zeros);
     if (count != 0 && k != 0)
         check(katsu_cuda_matmul_fwd(device_context(), node_->device(), rhs.node_->device(), out->ptr, m, k, n));
     Op op;
@@ -431,7 +467,7 @@ bool is_square(const Tensor &node) {
 // A private one-element copy of a device scalar (the original is an adjoint that may later be
 // published as a gradient and accumulated into).
 std::shared_ptr<DeviceBuffer> copy_scalar(const float *src) {
-    auto out = std::make_shared<DeviceBuffer>(1);
+    auto out = uninit_buffer(1);
     check(katsu_cuda_d2d(device_context(), out->ptr, src, 1));
     return out;
 }
@@ -463,26 +499,28 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
             }
             if (op.bias) {
                 const Tensor &b = parents[2];
-                float *pb = pending.at(b.id()).to_dense();
+                const bool first_b = !touched.count(b.id());
+                float *pb = first_b ? pending.at(b.id()).to_overwrite() : pending.at(b.id()).to_add();
                 float *dg = nullptr;
                 if (op.relu && node.numel()) {
-                    masked = std::make_shared<DeviceBuffer>(node.numel());
+                    masked = uninit_buffer(node.numel());
                     dg = masked->ptr;
                 }
                 check(katsu_cuda_bias_relu_bwd(ctx, node.device_data(), g, dg, pb, node.shape()[0], node.shape()[1], plane,
-                                               op.relu ? 1 : 0, touched.count(b.id()) ? 1 : 0));
+                                               op.relu ? 1 : 0, first_b ? 0 : 1));
                 touched.insert(b.id());
                 if (dg != nullptr) g = dg;
             } else if (op.relu && node.numel()) {
-                masked = std::make_shared<DeviceBuffer>(node.numel());
+                masked = uninit_buffer(node.numel());
                 check(katsu_cuda_bias_relu_bwd(ctx, node.device_data(), g, masked->ptr, nullptr, node.shape()[0],
                                                node.shape()[1], plane, 1, 0));
                 g = masked->ptr;
             }
-            float *px = pending.at(x.id()).to_dense(), *pw = pending.at(w.id()).to_dense();
             if (x.id() != w.id()) {
                 // backward_buffers + `pending[parent] += grad` (tensor.rs:374-390)
                 const int acc_x = touched.count(x.id()) ? 1 : 0, acc_w = touched.count(w.id()) ? 1 : 0;
+                float *px = acc_x ? pending.at(x.id()).to_add() : pending.at(x.id()).to_overwrite();
+                float *pw = acc_w ? pending.at(w.id()).to_add() : pending.at(w.id()).to_overwrite();
                 const float *xs_staged = staged_input(x, xs[0], xs[1], xs[2], xs[3], ws[0], ws[2], ws[3], op.stride, op.padding);
                 if (acc_x == acc_w) {
                     check(katsu_cuda_conv2d_bwd_staged(ctx, x.device_data(), xs_staged, w.device_data(), g, gscale, gfactor,
@@ -503,9 +541,9 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
                 DeviceBuffer dx(x.numel()), dw(w.numel());
                 check(katsu_cuda_conv2d_bwd(ctx, x.device_data(), w.device_data(), g, dx.ptr, dw.ptr, xs[0], xs[1],
                                             xs[2], xs[3], ws[0], ws[2], ws[3], op.stride, op.padding, 0));
+                float *px = pending.at(x.id()).to_add();
                 check(katsu_cuda_axpy_acc(ctx, px, dx.ptr, x.numel()));
-                check(katsu_cuda_axpy_acc(ctx, pw, dw.ptr, w.numel()));
-                check(katsu_cuda_sync(ctx));
+                check(katsu_cuda_axpy_acc(ctx, px, dw.ptr, w.numel()));
                 touched.insert(x.id());
             }
             return;
@@ -523,20 +561,24 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
                     target.source = y.node()->dev;
                     target.dense.reset();
                 } else if (node.numel()) {
-                    check(katsu_cuda_square_vjp(ctx, target.to_dense(), y.device_data(), own.scalar->ptr, node.numel(), 1));
+                    check(katsu_cuda_square_vjp(ctx, target.to_add(), y.device_data(), own.scalar->ptr, node.numel(), 1));
                 }
                 touched.insert(y.id());
                 return;
             }
-            const float *g = own.to_dense();
             // Both edges are visited even when they are the same node (tensor.rs:392-409).
             for (int side = 0; side < 2; ++side) {
                 const Tensor &parent = parents[side], &other = parents[1 - side];
-                float *target = pending.at(parent.id()).to_dense();
-                if (op.kind == Op::Add)
-                    check(katsu_cuda_axpy_acc(ctx, target, g, node.numel()));
+                Adjoint &target = pending.at(parent.id());
+                const bool first = !touched.count(parent.id());
+                if (op.kind == Op::Add && first)
+                    target.share(own);
+                else if (op.kind == Op::Add)
+                    check(katsu_cuda_axpy_acc(ctx, target.to_add(), own.to_dense(), node.numel()));
+                else if (first)  // fl(g * other) is what adding it to zero leaves
+                    check(katsu_cuda_mul(ctx, own.to_dense(), other.device_data(), target.to_overwrite(), node.numel()));
                 else
-                    check(katsu_cuda_mul_acc(ctx, target, g, other.device_data(), node.numel()));
+                    check(katsu_cuda_mul_acc(ctx, target.to_add(), own.to_dense(), other.device_data(), node.numel()));
                 touched.insert(parent.id());
             }
             return;
@@ -551,13 +593,16 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
                 target.scalar = copy_scalar(g);
                 target.dense.reset();
             } else {
-                check(katsu_cuda_bcast_acc(ctx, target.to_dense(), g, parent.numel()));
+                check(katsu_cuda_bcast_acc(ctx, target.to_add(), g, parent.numel()));
             }
             touched.insert(parent.id());
             return;
         }
         case Op::Reshape:
-            check(katsu_cuda_axpy_acc(ctx, pending.at(parents[0].id()).to_dense(), own.to_dense(), node.numel()));
+            if (touched.count(parents[0].id()))
+                check(katsu_cuda_axpy_acc(ctx, pending.at(parents[0].id()).to_add(), own.to_dense(), node.numel()));
+            else
+                pending.at(parents[0].id()).share(own);
             touched.insert(parents[0].id());
             return;
         case Op::Matmul: {
@@ -565,9 +610,10 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
             const size_t m = a.shape()[0], k = a.shape()[1], n = b.shape()[1];
             if (node.numel() == 0 || k == 0) return;  // tensor.rs:421-423
             const float *g = own.to_dense();
-            float *pa = pending.at(a.id()).to_dense(), *pb = pending.at(b.id()).to_dense();
             if (a.id() != b.id()) {
                 const int acc_a = touched.count(a.id()) ? 1 : 0, acc_b = touched.count(b.id()) ? 1 : 0;
+                float *pa = acc_a ? pending.at(a.id()).to_add() : pending.at(a.id()).to_overwrite();
+                float *pb = acc_b ? pending.at(b.id()).to_add() : pending.at(b.id()).to_overwrite();
                 if (acc_a == acc_b) {
                     check(katsu_cuda_matmul_bwd(ctx, a.device_data(), b.device_data(), g, pa, pb, m, k, n, acc_a));
                 } else {
@@ -575,8 +621,9 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
                     check(katsu_cuda_matmul_bwd(ctx, a.device_data(), b.device_data(), g, nullptr, pb, m, k, n, acc_b));
                 }
             } else {
+                float *pa = pending.at(a.id()).to_add();
                 check(katsu_cuda_matmul_bwd(ctx, a.device_data(), b.device_data(), g, pa, nullptr, m, k, n, 1));
-                check(katsu_cuda_matmul_bwd(ctx, a.device_data(), b.device_data(), g, nullptr, pb, m, k, n, 1));
+                check(katsu_cuda_matmul_bwd(ctx, a.device_data(), b.device_data(), g, nullptr, pa, m, k, n, 1));
             }
             touched.insert(a.id());
             touched.insert(b.id());
@@ -594,10 +641,10 @@ void Tensor::backward_with(const std::vector<float> &seed) const {
     const std::vector<Tensor> order = topological_order();
     Pending pending;
     for (const Tensor &node : order) pending[node.id()].numel = node.numel();
-    if (numel() != 0) {
-        check(katsu_cuda_h2d(ctx, pending.at(id()).to_dense(), seed.data(), numel()));
-        check(katsu_cuda_sync(ctx));  // `seed` may be a temporary
-    }
+    if (numel() == 1)
+        check(katsu_cuda_fill(ctx, pending.at(id()).to_overwrite(), seed[0], 1));
+    else if (numel() != 0)  // (from pageable memory: `seed` may go away once the call has returned)
+        check(katsu_cuda_h2d(ctx, pending.at(id()).to_overwrite(), seed.data(), numel()));
     Touched touched;
     touched.insert(id());  // the seed
     for (auto it = order.rbegin(); it != order.rend(); ++it) op_backward(*it, pending.at(it->id()), pending, touched);
@@ -610,7 +657,13 @@ void Tensor::backward_with(const std::vector<float> &seed) const {
         if (n.has_grad()) {
             // tensor.rs:353-356: old += new, element by element
             const float *add = adjoint.to_dense();
-            check(katsu_cuda_axpy_acc(ctx, n.dense_grad()->ptr, add, n.numel));
+            n.dense_grad();
+            if (n.grad_dev.use_count() > 1) {  // another node's gradient is the same buffer (Adjoint::share)
+                auto own = uninit_buffer(n.numel);
+                if (n.numel) check(katsu_cuda_d2d(ctx, own->ptr, n.grad_dev->ptr, n.numel));
+                n.grad_dev = std::move(own);
+            }
+            check(katsu_cuda_axpy_acc(ctx, n.grad_dev->ptr, add, n.numel));
         } else if (adjoint.kind == Adjoint::Dense) {
             adjoint.to_dense();  // a node nothing contributed to still gets Some(zeros)
             n.grad_dev = std::move(adjoint.dense);  // tensor.rs:357-359: the adjoint buffer becomes the gradient
@@ -715,7 +768,7 @@ Conv2D Conv2D::from_weights_bias(Tensor weights, Tensor bias, size_t stride, siz
 Tensor Conv2D::forward(const Tensor &input) {
     const Geometry geometry(input, weights_, stride_, padding_);
     const std::vector<size_t> shape = geometry.output_shape();
-    auto out = std::make_shared<DeviceBuffer>(element_count(shape));
+    auto out = uninit_buffer(element_count(shape));
     if (out->count != 0) {
         // the input is read through its staged copy, which the backward pass of this layer finds again
         const float *staged = staged_input(input, geometry.batch, geometry.cin, geometry.h, geometry.w, geometry.cout,
@@ -748,12 +801,12 @@ std::pair<Tensor, Tensor> Conv2D::backward(const Tensor &grad_output) const {
     const Geometry geometry(input, weights_, stride_, padding_);
     const size_t expected = element_count(geometry.output_shape());
     if (grad_output.numel() != expected) fail(ErrorKind::DataLength, "", expected, grad_output.numel());
-    auto dx = std::make_shared<DeviceBuffer>(input.numel());
-    auto dw = std::make_shared<DeviceBuffer>(weights_.numel());
+    auto dx = uninit_buffer(input.numel());
+    auto dw = uninit_buffer(weights_.numel());
     const float *g = grad_output.device_data();
     std::shared_ptr<DeviceBuffer> masked;
     if (relu_ && expected != 0) {  // addition: the upstream gradient passes where the activation did
-        masked = std::make_shared<DeviceBuffer>(expected);
+        masked = uninit_buffer(expected);
         check(katsu_cuda_bias_relu_bwd(device_context(), output.device_data(), g, masked->ptr, nullptr, geometry.batch,
                                        geometry.cout, geometry.oh * geometry.ow, 1, 0));
         g = masked->ptr;

@@ -92,7 +92,9 @@ struct TensorNode;
 struct DeviceBuffer {
     float *ptr = nullptr;
     size_t count = 0;
-    explicit DeviceBuffer(size_t count);  // zero-filled (zeros_buffer, tensor.rs:120-125)
+    enum Fill { Zeros, Uninit };
+    // Zeros as in zeros_buffer (tensor.rs:120-125), or nothing where the next call overwrites every element.
+    explicit DeviceBuffer(size_t count, Fill fill = Zeros);
     ~DeviceBuffer();
     DeviceBuffer(const DeviceBuffer &) = delete;
     DeviceBuffer &operator=(const DeviceBuffer &) = delete;

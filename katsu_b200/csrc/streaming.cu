@@ -241,6 +241,10 @@ __global__ void __launch_bounds__(256) bias_relu_bwd_kernel(const float *__restr
     }
 }
 
+__global__ void __launch_bounds__(256) fill_kernel(float *dst, float value, size_t count) {
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) dst[i] = value;
+}
+
 __global__ void __launch_bounds__(256) bias_grad_fold_kernel(const float *__restrict__ partial, float *dbias, int channels,
                                                              int slices, int accumulate) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,6 +362,16 @@ extern "C" int32_t katsu_cuda_bcast_acc(katsu_cuda_ctx *ctx, float *dst, const f
     return ew_launch<Ew::BcastAcc>(ctx, dst, g, nullptr, count);
 }
 
+extern "C" int32_t katsu_cuda_fill(katsu_cuda_ctx *ctx, float *dst, float value, size_t count) {
+    KATSU_TRY(katsu_bind(ctx));
+    if (count == 0) return KATSU_OK;
+    KATSU_REQUIRE(dst != nullptr, "dst is null");
+    size_t blocks = katsu_div_up(count, 256);
+    if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
+    KATSU_LAUNCH(ctx, fill_kernel, (unsigned)blocks, 256, 0, dst, value, count);
+    return KATSU_OK;
+}
+
 int32_t katsu_sum_impl(katsu_cuda_ctx *ctx, const float *a, float *out, size_t count, bool square) {
     KATSU_TRY(katsu_bind(ctx));
     KATSU_REQUIRE(out != nullptr, "out is null");
@@ -370,13 +384,13 @@ int32_t katsu_sum_impl(katsu_cuda_ctx *ctx, const float *a, float *out, size_t c
     size_t chunk = katsu_div_up(count, parts);
     chunk = katsu_div_up(chunk, 1024) * 1024;  // multiple of 4 so 128-bit loads stay aligned
     parts = katsu_div_up(count, chunk);
-    float *partial = nullptr;
-    KATSU_TRY(katsu_scratch(ctx, parts, &partial));
+    float *partial = out;  // a single partial is the sum
+    if (parts > 1) KATSU_TRY(katsu_scratch(ctx, parts, &partial));
     if (square)
         KATSU_LAUNCH(ctx, sum_partial_kernel<true>, (unsigned)parts, 256, 0, a, count, chunk, partial);
     else
         KATSU_LAUNCH(ctx, sum_partial_kernel<false>, (unsigned)parts, 256, 0, a, count, chunk, partial);
-    KATSU_LAUNCH(ctx, sum_final_kernel, 1, 256, 0, partial, (int)parts, out);
+    if (parts > 1) KATSU_LAUNCH(ctx, sum_final_kernel, 1, 256, 0, partial, (int)parts, out);
     return KATSU_OK;
 }
 
