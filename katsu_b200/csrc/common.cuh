@@ -27,7 +27,8 @@ struct katsu_cuda_ctx {
     // of x (f16_conv.cu), written by katsu_cuda_conv2d_stage; the forward and dW launches use it instead of
     // staging x themselves
     const float *x_prestaged;
-    // Device memory of the fp16 path (f16_split.cuh): the accumulators of its magnitude pass, the operands' scales.
+    // 1 KiB of device memory: accumulators of the magnitude pass and scales of its operands (f16_split.cuh, first
+    // half), ticket of the sum (streaming.cu, at 512).
     void *f16_state;
     // Buffer written by katsu_cuda_flush_l2.
     float *flush;

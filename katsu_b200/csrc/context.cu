@@ -5,10 +5,12 @@
 #include <stdlib.h>
 
 #include <map>
+#include <mutex>
 #include <new>
 #include <unordered_map>
 
 #include "common.cuh"
+#include "launch.cuh"
 
 static thread_local char g_error[512] = "";
 
@@ -25,6 +27,20 @@ extern "C" const char *katsu_cuda_last_error_string(void) { return g_error; }
 int32_t katsu_bind(katsu_cuda_ctx *ctx) {
     if (ctx == nullptr) return katsu_set_error(KATSU_ERR_INVALID_ARG, "null context");
     KATSU_CUDA_TRY(cudaSetDevice(ctx->device));
+    return KATSU_OK;
+}
+
+int32_t katsu_prepare_kernel(katsu_cuda_ctx *ctx, const void *kernel, size_t smem) {
+    // contexts of several threads may launch the same kernel for the first time
+    static std::mutex lock;
+    static std::unordered_map<const void *, size_t> *prepared = new std::unordered_map<const void *, size_t>[64];
+    const std::lock_guard<std::mutex> hold(lock);
+    std::unordered_map<const void *, size_t> &of_device = prepared[ctx->device & 63];
+    auto it = of_device.find(kernel);
+    if (it != of_device.end() && it->second >= smem) return KATSU_OK;
+    if (smem) KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    of_device[kernel] = smem;
     return KATSU_OK;
 }
 

@@ -26,6 +26,7 @@
 // in flight (6.5 B/clk per SM), and one TMA tensor store per tile (32 x 4 x K box, 128-byte
 // inner rows) saturated near 16 B/clk per SM; the SM needs ~23 B/clk to fill HBM.
 #include "common.cuh"
+#include "launch.cuh"
 #include <string.h>
 
 #include "sm100.cuh"
@@ -318,7 +319,7 @@ int32_t fwd_launch_groups(katsu_cuda_ctx *ctx, const float *x, const float *w, f
     d.a_stages = (cols - d.acc_buffers * d.np) / 64;
     if (d.a_stages > 3) d.a_stages = 3;
     auto kernel = stem_fwd_tc_kernel<CIN, GROUPS>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, smem));
     const size_t total_tiles = size_t(d.n) * d.tiles_x * d.tiles_y;
     size_t grid = size_t(ctx->num_sms) * (GROUPS == 1 ? 2 : 1);
     if (grid > total_tiles) grid = total_tiles;

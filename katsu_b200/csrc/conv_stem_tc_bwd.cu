@@ -24,6 +24,7 @@
 //   Two warps issue MMAs (two M-tiles each): the elect.sync thread of one converged warp
 //   sustains one N = 32 MMA per ~22 cycles, two such warps reach the pipe's 16 (measured).
 #include "common.cuh"
+#include "launch.cuh"
 #include <string.h>
 
 #include "sm100.cuh"
@@ -321,7 +322,7 @@ int32_t dx_launch(katsu_cuda_ctx *ctx, const float *w, const float *g, float *dx
     }
     const size_t smem = dx_smem_bytes<CIN>(d.kblocks, d.gs);
     auto kernel = stem_dx_tc_kernel<CIN>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, smem));
     const size_t total_tiles = size_t(d.n) * d.tiles_x * d.tiles_y;
     size_t grid = size_t(ctx->num_sms);
     if (grid > total_tiles) grid = total_tiles;
@@ -622,7 +623,7 @@ int32_t dw_launch(katsu_cuda_ctx *ctx, const float *x, const float *g, float *dw
     size_t smem = size_t(DW_GS + DW_BS) * 8192 + 32 * 128 * 4 + size_t(DW_XS) * XT * 4 + 1024;
     if (smem < 100 * 1024) smem = 100 * 1024;
     auto kernel = stem_dw_tc_kernel<CIN>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, smem));
     const size_t total_tiles = size_t(d.n) * d.tiles_x * d.tiles_y;
     size_t grid = size_t(ctx->num_sms) * 2;
     if (grid > total_tiles) grid = total_tiles;

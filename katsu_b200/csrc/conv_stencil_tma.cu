@@ -9,6 +9,7 @@
 // window loads and FMAs.
 //   dx[c, iy, ix] = sum_{oc, ky, kx} g[oc, iy+1-ky, ix+1-kx] * w[oc, c, ky, kx]   (conv2d.rs:288)
 #include "common.cuh"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 using namespace sm100;
@@ -143,7 +144,7 @@ int32_t launch_th(katsu_cuda_ctx *ctx, const float *g, const float *w, float *dx
     d.tiles_y = (d.h + TH - 1) / TH;
     const size_t smem = (2 * size_t(G_STAGE) + size_t(d.kp) * WP) * sizeof(float);
     auto kernel = stencil_dx_tma_kernel<CIN, TH>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, smem));
     const unsigned grid = (unsigned)(size_t(d.n) * d.tiles_x * d.tiles_y);
     KATSU_LAUNCH(ctx, kernel, grid, 4 * TH, smem, map_g, w, dx, d);
     return KATSU_OK;
@@ -305,7 +306,7 @@ int32_t dw_launch(katsu_cuda_ctx *ctx, const CUtensorMap &map_g, const CUtensorM
     constexpr int XT = (CIN * DW_XR * GP + 31) / 32 * 32;
     const size_t smem = (2 * size_t(DW_G_STAGE) + 2 * size_t(XT)) * sizeof(float);
     auto kernel = stencil_dw_tma_kernel<CIN>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, smem));
     const size_t total_tiles = size_t(d.n) * d.tiles_x * d.tiles_y;
     size_t grid = size_t(ctx->num_sms) * 2;
     if (grid > total_tiles) grid = total_tiles;

@@ -9,6 +9,7 @@
 //
 // Any channel count: staging pads channels to 8, and the window view makes k-blocks out of S * channels.
 #include "f16_gemm.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -262,6 +263,8 @@ namespace {
 __global__ void __launch_bounds__(256)
 f16_dw_fold_kernel(const float *__restrict__ partial, float *dw, int k, int c, int r, int s, int cp, int groups_per_row, int splits, int accumulate) {
     __shared__ float sums[8][32];
+    launch_next();
+    launch_wait();
     const size_t lanes = size_t(r) * groups_per_row * 64, elems = lanes * k;
     const size_t j = size_t(blockIdx.x) * 32 + (threadIdx.x & 31);
     const int part = threadIdx.x >> 5;
@@ -421,8 +424,10 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.groups = (int)(r * gpr);
             p.groups_per_row = (int)gpr;
             KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_CONV_DW, mw, p, plan_dw, partial_dw, (long long)dw_count));
-            KATSU_LAUNCH(ctx, f16_dw_fold_kernel, (unsigned)katsu_div_up(dw_count, (size_t)32), 256, 0, partial_dw, dw,
-                         (int)k, (int)c, (int)r, (int)s, (int)cp, (int)gpr, plan_dw.splits, accumulate);
+            KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)f16_dw_fold_kernel, 0));
+            KATSU_TRY(katsu_launch_chained(ctx, f16_dw_fold_kernel, (unsigned)katsu_div_up(dw_count, (size_t)32), 256, 0, 1,
+                                           partial_dw, dw, (int)k, (int)c, (int)r, (int)s, (int)cp, (int)gpr, plan_dw.splits,
+                                           accumulate));
         }
     }
     return KATSU_OK;

@@ -31,9 +31,8 @@
 // Roles: warps 0-7 drain and store (lane quarter = warp % 4, alternate 32-column chunks by warp / 4), warp 8 issues the
 // TMA loads, warp 9 of the leader block the MMAs.  Persistent over tiles x splits.  Every wait is bounded; both blocks of
 // a pair always reach the cluster barrier at the end.
-#include <cstring>
-
 #include "f16_gemm.cuh"
+#include "launch.cuh"
 #include "sm100.cuh"
 #include "sm100_pair.cuh"
 
@@ -144,10 +143,6 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
-    const bool wide = katsu_f16_wide(p.call);
-    const int planes = NARROW + (wide ? 1 : 0);
-    // k-blocks between two drains: 192 accumulation steps in 3xTF32 mode, up to 12 288 in TF32 mode (4e-4 of 2e-3)
-    const int drain = NARROW == 2 ? (wide ? 8 : 16) : 1024;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
@@ -155,8 +150,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     const int items = p.m_tiles * p.n_tiles * p.splits;
     const int half = p.bn >> 1;                 // B columns that this block loads
     const int b_bytes = half * BK * 2;
-    const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
-    const int stages = min(MAX_STAGES, SMEM_RING / stage_bytes);
+    launch_next();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) {
@@ -178,6 +172,13 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     cluster_sync_all();  // both blocks' barriers exist before anything is signalled across the pair
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_slot;
+    launch_wait();
+    const bool wide = katsu_f16_wide(p.call);
+    const int planes = NARROW + (wide ? 1 : 0);
+    // k-blocks between two drains: 192 accumulation steps in 3xTF32 mode, up to 12 288 in TF32 mode (4e-4 of 2e-3)
+    const int drain = NARROW == 2 ? (wide ? 8 : 16) : 1024;
+    const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
+    const int stages = min(MAX_STAGES, SMEM_RING / stage_bytes);
 
     if (warp == 8 && lane == 0) {
         // ---- TMA producer: this block's lanes of A and half of B's columns; bytes counted on the leader's barrier ----
@@ -439,6 +440,8 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 
 __global__ void __launch_bounds__(256)
 f16_fold_kernel(const float *__restrict__ partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels, size_t plane, int relu) {
+    launch_next();
+    launch_wait();
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
         float s = 0.f;
 #pragma unroll 8
@@ -452,24 +455,8 @@ f16_fold_kernel(const float *__restrict__ partial, float *out, size_t count, int
 template <int NARROW, KatsuF16Kind KIND>
 int32_t launch(katsu_cuda_ctx *ctx, const KatsuF16Maps &maps, const KatsuF16Problem &p, unsigned pairs) {
     auto kernel = f16_pair_kernel<NARROW, KIND>;
-    KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
-    cudaLaunchConfig_t config;
-    memset(&config, 0, sizeof(config));
-    config.gridDim = dim3(2 * pairs, 1, 1);
-    config.blockDim = dim3(THREADS, 1, 1);
-    config.dynamicSmemBytes = SMEM;
-    config.stream = ctx->stream;
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeClusterDimension;
-    attribute.val.clusterDim.x = 2;
-    attribute.val.clusterDim.y = 1;
-    attribute.val.clusterDim.z = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    cudaError_t err = cudaLaunchKernelEx(&config, kernel, maps, p);
-    ctx->launches += 1;
-    if (err != cudaSuccess) return katsu_set_error(KATSU_ERR_CUDA, "fp16 kernel launch failed: %s", cudaGetErrorString(err));
-    return KATSU_OK;
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)kernel, SMEM));
+    return katsu_launch_chained(ctx, kernel, 2 * pairs, THREADS, SMEM, 2, maps, p);
 }
 
 }  // namespace
@@ -559,9 +546,9 @@ int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const float *partial, float *out, si
                        size_t plane, int relu) {
     size_t blocks = katsu_div_up(count, (size_t)256);
     if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
-    KATSU_LAUNCH(ctx, f16_fold_kernel, (unsigned)blocks, 256, 0, partial, out, count, splits, accumulate,
-                 bias, channels, plane, relu);
-    return KATSU_OK;
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)f16_fold_kernel, 0));
+    return katsu_launch_chained(ctx, f16_fold_kernel, (unsigned)blocks, 256, 0, 1, partial, out, count, splits, accumulate, bias,
+                                channels, plane, relu);
 }
 
 bool katsu_f16_rows_maps(CUtensorMap *maps, const KatsuF16Planes &planes, int count, size_t cols, size_t rows, size_t d2,

@@ -10,14 +10,14 @@
 
 namespace {
 
-// Multiply-adds from which the path pays: its fixed part (magnitudes, planes, product, fold) is about
-// 15 us, which the CUDA-core kernels need for about this much work.
-constexpr double MIN_MACS = 6e6;
+// Multiply-adds from which the path pays against the CUDA cores (gemm_small_kernel, about 5 T multiply-adds a second): its
+// fixed part, three or four launches, is 15 us.  In TF32 mode the line lies lower, since that mode is chosen for speed.
+double least_macs(const katsu_cuda_ctx *ctx) { return ctx->precision == KATSU_MODE_3XTF32 ? 4e7 : 1.5e7; }
 
 bool takes(const katsu_cuda_ctx *ctx, size_t m, size_t k, size_t n) {
     if (ctx->precision == KATSU_MODE_FP32 || ctx->f16_state == nullptr) return false;
     if (m > 0x3fffffff || n > 0x3fffffff || k > 0x3fffffff) return false;
-    return double(m) * double(n) * double(k) >= MIN_MACS;
+    return double(m) * double(n) * double(k) >= least_macs(ctx);
 }
 
 KatsuStageJob rows_job(const float *src, size_t rows, size_t cols, const KatsuF16Planes &to, const KatsuF16Info *info) {

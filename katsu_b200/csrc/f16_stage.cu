@@ -5,6 +5,7 @@
 // when the operand fits there) and writes 2 or 4 bytes an element.  Up to three operands share a launch, because in
 // small calls a launch costs more than the pass.
 #include "f16_split.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -37,6 +38,8 @@ __device__ __forceinline__ unsigned max4(float4 v) {
 // A group is the 128 consecutive floats that a warp reads at once; the last group of a tensor reaches back so that
 // it is a full one.  Magnitudes compare as their bit patterns, which puts infinities and NaNs above every number.
 __global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ AmaxParams p) {
+    launch_next();
+    launch_wait();
     int si = 0;
     while (si + 1 < p.segments && blockIdx.x >= p.seg[si + 1].first_block) ++si;
     const AmaxSegment &sg = p.seg[si];
@@ -327,6 +330,8 @@ __device__ void stage_weights(const KatsuStageJob &j, const Writer &out, unsigne
 
 __global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ StageParams p) {
     __shared__ __align__(16) float tile[4096];
+    launch_next();
+    launch_wait();
     int ji = 0;
     while (ji + 1 < p.jobs && blockIdx.x >= p.first_block[ji + 1]) ++ji;
     const KatsuStageJob &j = p.job[ji];
@@ -383,8 +388,8 @@ int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count)
         s.blocks = (unsigned)blocks;
         at += s.blocks;
     }
-    KATSU_LAUNCH(ctx, amax_kernel, at, THREADS, 0, p);
-    return KATSU_OK;
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)amax_kernel, 0));
+    return katsu_launch_chained(ctx, amax_kernel, at, THREADS, 0, 1, p);
 }
 
 int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const KatsuStageJob *jobs, int count) {
@@ -413,6 +418,6 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
         at += blocks;
     }
     if (at > 0x7fffffffu) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "operand too large to stage");
-    KATSU_LAUNCH(ctx, stage_kernel, (unsigned)at, THREADS, 0, p);
-    return KATSU_OK;
+    KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)stage_kernel, 0));
+    return katsu_launch_chained(ctx, stage_kernel, (unsigned)at, THREADS, 0, 1, p);
 }

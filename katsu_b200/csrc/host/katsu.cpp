@@ -109,7 +109,7 @@ DeviceBuffer::~DeviceBuffer() {
 // exactly the values the reference's node-by-node VJPs would have stored (tensor.rs:392-417):
 //   Bcast   every element is scalar[0]                       (Sum VJP into a fresh adjoint)
 //   Scaled  element i is t + t with t = fl(scalar[0] * source[i])   (both Mul edges of y * y into y's fresh adjoint)
-// `scalar` is a private one-element copy, `source` the node's own immutable values.
+// `scalar` is another node's one-element adjoint (shared, see share()), `source` the node's own immutable values.
 struct Adjoint {
     enum Kind { Dense, Bcast, Scaled };
     Kind kind = Dense;
@@ -464,12 +464,15 @@ bool is_square(const Tensor &node) {
     return node.op().kind == Op::Mul && node.parents()[0].id() == node.parents()[1].id();
 }
 
-// A private one-element copy of a device scalar (the original is an adjoint that may later be
-// published as a gradient and accumulated into).
-std::shared_ptr<DeviceBuffer> copy_scalar(const float *src) {
-    auto out = uninit_buffer(1);
-    check(katsu_cuda_d2d(device_context(), out->ptr, src, 1));
-    return out;
+// The seed of loss.backward(): the number 1 on the device, for good.  It is shared like any adjoint, so nothing adds to it.
+std::shared_ptr<DeviceBuffer> device_one() {
+    static auto *one = new std::shared_ptr<DeviceBuffer>();
+    if (!*one) {
+        auto buffer = uninit_buffer(1);
+        check(katsu_cuda_fill(device_context(), buffer->ptr, 1.0f, 1));
+        *one = std::move(buffer);
+    }
+    return *one;
 }
 
 // Op::backward, tensor.rs:365-449: adds this node's contribution to the
@@ -590,7 +593,7 @@ void op_backward(const Tensor &node, Adjoint &own, Pending &pending, Touched &to
             if (g_loss_fusion && is_square(parent) && !touched.count(parent.id())) {
                 // the adjoint of y * y is the broadcast of g[0]: kept as that one number
                 target.kind = Adjoint::Bcast;
-                target.scalar = copy_scalar(g);
+                target.scalar = own.dense;
                 target.dense.reset();
             } else {
                 check(katsu_cuda_bcast_acc(ctx, target.to_add(), g, parent.numel()));
@@ -641,7 +644,9 @@ void Tensor::backward_with(const std::vector<float> &seed) const {
     const std::vector<Tensor> order = topological_order();
     Pending pending;
     for (const Tensor &node : order) pending[node.id()].numel = node.numel();
-    if (numel() == 1)
+    if (numel() == 1 && seed[0] == 1.0f)
+        pending.at(id()).dense = device_one();
+    else if (numel() == 1)
         check(katsu_cuda_fill(ctx, pending.at(id()).to_overwrite(), seed[0], 1));
     else if (numel() != 0)  // (from pageable memory: `seed` may go away once the call has returned)
         check(katsu_cuda_h2d(ctx, pending.at(id()).to_overwrite(), seed.data(), numel()));

@@ -12,6 +12,8 @@
 //    code serves a@b, g@b^T and a^T@g without materialising a transpose.
 #include "common.cuh"
 #include "f16_split.cuh"
+#include "launch.cuh"
+#include "sm100_pair.cuh"
 
 namespace {
 
@@ -318,6 +320,87 @@ skinny_db_kernel(const float *__restrict__ a, const float *__restrict__ g, float
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same product for results too small to give every SM a 64 x 64 tile (a linear layer on a small batch: one tile, a
+// chain of K / 16 slices, 158 us for [32,784] @ [784,10]): 32 x 32 tiles, 2 x 2 outputs a thread, and the contraction
+// split over the S <= 8 blocks of a cluster, which add their tiles through each other's shared memory in rank order.
+// Bound by latency: a chunk of 32 is loaded into registers while the one before it is multiplied.  5 us for that layer.
+// ---------------------------------------------------------------------------
+constexpr int ST = 32;
+
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(256)
+gemm_small_kernel(const float *__restrict__ a, const float *__restrict__ b, float *c, int M, int N, int K, size_t sa_i,
+                  size_t sa_p, size_t sb_p, size_t sb_j, int accumulate, int tiles_n, int splits, int k_per_split) {
+    __shared__ __align__(16) float As[ST][ST + 2], Bs[ST][ST + 2], tile_sum[ST * ST];
+    launch_next();
+    launch_wait();
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int tile = blockIdx.x / splits, rank = blockIdx.x - tile * splits;
+    const int i0 = (tile / tiles_n) * ST, j0 = (tile % tiles_n) * ST;
+    const int k_begin = rank * k_per_split, k_end = min(K, k_begin + k_per_split);
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    float av[4], bv[4];
+    // element e of a chunk: the unit-stride axis walks fastest
+    auto load = [&](int p0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = tid + 256 * q;
+            const int ai = sa_p == 1 ? e >> 5 : e & 31, ap = sa_p == 1 ? e & 31 : e >> 5;
+            const int bj = sb_j == 1 ? e & 31 : e >> 5, bp = sb_j == 1 ? e >> 5 : e & 31;
+            av[q] = (i0 + ai < M && p0 + ap < k_end) ? __ldg(a + size_t(i0 + ai) * sa_i + size_t(p0 + ap) * sa_p) : 0.f;
+            bv[q] = (j0 + bj < N && p0 + bp < k_end) ? __ldg(b + size_t(p0 + bp) * sb_p + size_t(j0 + bj) * sb_j) : 0.f;
+        }
+    };
+    if (k_begin < k_end) load(k_begin);
+    for (int p0 = k_begin; p0 < k_end; p0 += ST) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = tid + 256 * q;
+            if (sa_p == 1) As[e & 31][e >> 5] = av[q]; else As[e >> 5][e & 31] = av[q];
+            if (sb_j == 1) Bs[e >> 5][e & 31] = bv[q]; else Bs[e & 31][e >> 5] = bv[q];
+        }
+        __syncthreads();
+        if (p0 + ST < k_end) load(p0 + ST);
+#pragma unroll
+        for (int pp = 0; pp < ST; ++pp) {
+            const float2 x = *reinterpret_cast<const float2 *>(&As[pp][ty * 2]);
+            const float2 y = *reinterpret_cast<const float2 *>(&Bs[pp][tx * 2]);
+            acc[0][0] = fmaf(x.x, y.x, acc[0][0]);
+            acc[0][1] = fmaf(x.x, y.y, acc[0][1]);
+            acc[1][0] = fmaf(x.y, y.x, acc[1][0]);
+            acc[1][1] = fmaf(x.y, y.y, acc[1][1]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) tile_sum[(ty * 2 + u) * ST + tx * 2 + v] = acc[u][v];
+    if (splits > 1) sm100::cluster_sync_all();
+    else __syncthreads();
+    const int share = ST * ST / splits;
+    for (int e = tid; e < share; e += 256) {
+        const int o = rank * share + e;
+        float sum = tile_sum[o];
+        if (splits > 1) {
+            sum = 0.f;
+            for (int q = 0; q < splits; ++q) sum += ld_cluster_f32(sm100::map_to_rank(&tile_sum[o], q));
+        }
+        const int i = i0 + (o >> 5), j = j0 + (o & 31);
+        if (i < M && j < N) {
+            float *dst = c + size_t(i) * N + j;
+            *dst = accumulate ? *dst + sum : sum;
+        }
+    }
+    if (splits > 1) sm100::cluster_sync_all();  // no block leaves while another reads its tile
+}
+
 bool aligned16(const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 int32_t gemm_strided(katsu_cuda_ctx *ctx, const float *a, const float *b, float *c, size_t M, size_t N, size_t K,
@@ -325,6 +408,17 @@ int32_t gemm_strided(katsu_cuda_ctx *ctx, const float *a, const float *b, float 
     if (M > 0x7fffffff || N > 0x7fffffff || K > 0x7fffffff)
         return katsu_set_error(KATSU_ERR_UNSUPPORTED, "a matmul dimension exceeds 2^31-1");
     const size_t gy = katsu_div_up(M, 64), gx = katsu_div_up(N, 64);
+    if (gx * gy * 2 <= (size_t)ctx->num_sms) {
+        // fewer 64 x 64 tiles than half the SMs: smaller tiles, and the contraction split while SMs are idle
+        const size_t tiles = katsu_div_up(M, (size_t)ST) * katsu_div_up(N, (size_t)ST);
+        unsigned splits = 1;
+        while (splits < 8 && tiles * splits * 2 <= (size_t)ctx->num_sms * 2 && K >= (size_t)ST * splits * 2) splits *= 2;
+        const size_t per = katsu_div_up(katsu_div_up(K, (size_t)splits), (size_t)ST) * ST;
+        KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)gemm_small_kernel, 0));
+        return katsu_launch_chained(ctx, gemm_small_kernel, (unsigned)(tiles * splits), 256, 0, splits, a, b, c, (int)M, (int)N,
+                                    (int)K, sa_i, sa_p, sb_p, sb_j, accumulate, (int)katsu_div_up(N, (size_t)ST), (int)splits,
+                                    (int)per);
+    }
     if (gy > 65535) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "matmul output has too many row tiles");
     dim3 grid((unsigned)gx, (unsigned)gy);
     KATSU_LAUNCH(ctx, gemm_strided_kernel, grid, 256, 0, a, b, c, (int)M, (int)N, (int)K, sa_i, sa_p, sb_p, sb_j,

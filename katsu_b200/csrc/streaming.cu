@@ -92,7 +92,7 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Stage 1: block b folds elements b*chunk .. (b+1)*chunk into partial[b].
+// Block b folds elements b*chunk .. (b+1)*chunk into partial[b].
 // Fixed assignment of elements to threads and a fixed tree make the result
 // independent of scheduling (bit-reproducible run to run).
 // SQUARE: every element is squared (one rounded multiply, as Tensor::mul would store it) on the way
@@ -100,9 +100,11 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <bool SQUARE>
 __device__ __forceinline__ float sum_term(float v) { return SQUARE ? __fmul_rn(v, v) : v; }
 
+// The block that finishes last folds the partials, in f64 and a fixed order, and writes out[0]; it leaves the ticket
+// as it found it.
 template <bool SQUARE>
-__global__ void __launch_bounds__(256) sum_partial_kernel(const float *__restrict__ a, size_t count,
-                                                          size_t chunk, float *__restrict__ partial) {
+__global__ void __launch_bounds__(256) sum_kernel(const float *__restrict__ a, size_t count, size_t chunk,
+                                                  float *partial, unsigned *ticket, float *__restrict__ out) {
     const size_t begin = size_t(blockIdx.x) * chunk;
     size_t end = begin + chunk;
     if (end > count) end = count;
@@ -122,28 +124,39 @@ __global__ void __launch_bounds__(256) sum_partial_kernel(const float *__restric
     }
     float v = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
     __shared__ float warp_part[8];
+    __shared__ bool last;
     if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x < 32) {
         float t = threadIdx.x < 8 ? warp_part[threadIdx.x] : 0.f;
         t = warp_sum(t);
-        if (threadIdx.x == 0) partial[blockIdx.x] = t;
+        if (threadIdx.x == 0) {
+            if (gridDim.x == 1) {
+                out[0] = t;
+                last = false;
+            } else {
+                partial[blockIdx.x] = t;
+                __threadfence();
+                last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+            }
+        }
     }
-}
-
-// Stage 2: one block folds the partials in f64 and writes out[0].
-__global__ void __launch_bounds__(256) sum_final_kernel(const float *__restrict__ partial, int parts,
-                                                        float *__restrict__ out) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < parts; i += blockDim.x) acc += (double)partial[i];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double fold = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) fold += (double)__ldcg(partial + i);
     __shared__ double sh[256];
-    sh[threadIdx.x] = acc;
+    sh[threadIdx.x] = fold;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
         if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[0] = (float)sh[0];
+    if (threadIdx.x == 0) {
+        out[0] = (float)sh[0];
+        *ticket = 0;
+    }
 }
 
 // dst[i] (+)= t + t with t = fl(s[0] * src[i]): the two Mul VJP edges of q = y * y (both lead to y,
@@ -384,13 +397,11 @@ int32_t katsu_sum_impl(katsu_cuda_ctx *ctx, const float *a, float *out, size_t c
     size_t chunk = katsu_div_up(count, parts);
     chunk = katsu_div_up(chunk, 1024) * 1024;  // multiple of 4 so 128-bit loads stay aligned
     parts = katsu_div_up(count, chunk);
-    float *partial = out;  // a single partial is the sum
+    float *partial = nullptr;
     if (parts > 1) KATSU_TRY(katsu_scratch(ctx, parts, &partial));
-    if (square)
-        KATSU_LAUNCH(ctx, sum_partial_kernel<true>, (unsigned)parts, 256, 0, a, count, chunk, partial);
-    else
-        KATSU_LAUNCH(ctx, sum_partial_kernel<false>, (unsigned)parts, 256, 0, a, count, chunk, partial);
-    if (parts > 1) KATSU_LAUNCH(ctx, sum_final_kernel, 1, 256, 0, partial, (int)parts, out);
+    unsigned *ticket = reinterpret_cast<unsigned *>(static_cast<char *>(ctx->f16_state) + 512);
+    auto kernel = square ? sum_kernel<true> : sum_kernel<false>;
+    KATSU_LAUNCH(ctx, kernel, (unsigned)parts, 256, 0, a, count, chunk, partial, ticket, out);
     return KATSU_OK;
 }
 
