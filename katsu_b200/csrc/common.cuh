@@ -27,9 +27,9 @@ struct katsu_cuda_ctx {
     // of x (f16_conv.cu), written by katsu_cuda_conv2d_stage; the forward and dW launches use it instead of
     // staging x themselves
     const float *x_prestaged;
-    // 1 KiB of device memory: accumulators of the magnitude pass and scales of its operands (f16_split.cuh, first
-    // half), ticket of the sum (streaming.cu, at 512).
+    // 1 KiB of device memory: what the magnitude pass found of a call's operands (f16_split.cuh, first half), ticket of the sum (streaming.cu, at 512).
     void *f16_state;
+    int f16_set;  // set of operand slots of the current call
     // Buffer written by katsu_cuda_flush_l2.
     float *flush;
     size_t flush_floats;

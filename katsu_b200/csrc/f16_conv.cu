@@ -175,12 +175,14 @@ size_t katsu_f16_conv_staged_bytes(const katsu_cuda_ctx *ctx, size_t n, size_t c
 }
 
 int32_t katsu_f16_conv_stage(katsu_cuda_ctx *ctx, const float *x, void *staged, size_t n, size_t c, size_t h, size_t w) {
-    KatsuF16Info *info = static_cast<KatsuF16Info *>(staged);
+    katsu_f16_new_call(ctx);
+    KatsuF16Info *info = katsu_f16_slot(ctx, KATSU_INFO_A);
     const Staged p = staged_at(static_cast<char *>(staged) + STAGED_HEADER, n, c, h, w, STAGED_GAP, 0);
     const KatsuAmaxJob amax = {x, n * c * h * w, info};
     KATSU_TRY(katsu_f16_amax(ctx, &amax, 1));
-    const KatsuStageJob job = nhwc_job(x, p, c, 0, info);
-    return katsu_f16_stage(ctx, KatsuF16Call{{info, nullptr, nullptr}}, &job, 1);
+    KatsuStageJob job = nhwc_job(x, p, c, 0, info);
+    job.info_copy = static_cast<KatsuF16Info *>(staged);
+    return katsu_f16_stage(ctx, katsu_f16_call(ctx, info, nullptr, nullptr), &job, 1);
 }
 
 bool katsu_f16_conv_geometry(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
@@ -196,19 +198,20 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     if (!geometry_ok(ctx, g) || !worth_it(g)) return KATSU_OK;
     const int planes = katsu_f16_narrow_planes(ctx) + 1;
     const size_t cp = katsu_round_up(c, 8), width = s * cp, chunks = katsu_div_up(width, 64);
+    katsu_f16_new_call(ctx);
     KatsuF16Info *ix = katsu_f16_slot(ctx, KATSU_INFO_A), *iw = katsu_f16_slot(ctx, KATSU_INFO_B);
     const KatsuF16Info *info = ix;
     Staged held;
     const bool prestaged = held_x(ctx, g, &info, &held);
     const size_t out_count = n * oh * ow * k;
     const KatsuF16Box box = katsu_f16_box(128, false, (int)stride, ow, oh, n);
-    if (box.blocks > 0x7fffffff) return KATSU_OK;
+    if (box.blocks > 0x7fffffff) return katsu_f16_drop_call(ctx);
     const KatsuF16Plan plan = katsu_f16_plan(ctx, KATSU_F16_CONV, box.blocks * 128, (int)k, (long long)(r * chunks), double(out_count));
     KatsuArena arena = {nullptr, 0};
     for (int pass = 0; pass < 2; ++pass) {  // the first only adds up the sizes
         if (pass) {
             float *base = nullptr;
-            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return KATSU_OK;  // no room: the other kernels
+            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return katsu_f16_drop_call(ctx);  // no room: the other kernels
             arena = {reinterpret_cast<char *>(base), 0};
         }
         // (room for x also when the caller holds a copy: a narrow copy is of no use to a wide call)
@@ -221,9 +224,9 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         if (!x_window_maps(ctx, maps.a, prestaged ? held : own, g, box) ||
             (prestaged && !x_window_maps(ctx, maps.a_second, own, g, box)) ||
             !katsu_f16_rows_maps(maps.b, ws, planes, width, k, r, width, k * width, plan.bn / 2))
-            return KATSU_OK;
+            return katsu_f16_drop_call(ctx);
         *handled = 1;
-        const KatsuF16Call call = {{info, iw, nullptr}};
+        const KatsuF16Call call = katsu_f16_call(ctx, info, iw, nullptr);
         KatsuAmaxJob amax[2] = {{w, k * c * r * s, iw}, {x, n * c * h * wd, ix}};
         KATSU_TRY(katsu_f16_amax(ctx, amax, prestaged ? 1 : 2));
         KatsuStageJob jobs[2] = {nhwc_job(x, own, c, 0, info), weights_job(w, ws, g, cp, width, iw)};
@@ -300,6 +303,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     const size_t cp = katsu_round_up(c, 8), kp = katsu_round_up(k, 8);
     const size_t gap = q.left > q.right ? q.left : q.right;
     const size_t tail = katsu_round_up((size_t(q.most_taps) + q.most_rel_x + 2) * kp + 64, 8);
+    katsu_f16_new_call(ctx);
     KatsuF16Info *ix = katsu_f16_slot(ctx, KATSU_INFO_A), *iw = katsu_f16_slot(ctx, KATSU_INFO_B), *ig = katsu_f16_slot(ctx, KATSU_INFO_G);
     const KatsuF16Info *info = ix;
     Staged held;
@@ -327,14 +331,14 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     const size_t gpr = katsu_div_up(s * cp, (size_t)64), dw_lanes = r * gpr * 64, dw_count = dw_lanes * k;
     const KatsuF16Box box_dw = katsu_f16_box(64, true, (int)stride, ow, oh, n);
     const long long kb_dw = box_dw.blocks;
-    if (box_dx.blocks > 0x7fffffff || box_dw.blocks > 0x7fffffff) return KATSU_OK;
+    if (box_dx.blocks > 0x7fffffff || box_dw.blocks > 0x7fffffff) return katsu_f16_drop_call(ctx);
     const KatsuF16Plan plan_dw = katsu_f16_plan(ctx, KATSU_F16_CONV_DW, (long long)dw_lanes, (int)k, kb_dw, double(dw_count));
 
     KatsuArena arena = {nullptr, 0};
     for (int pass = 0; pass < 2; ++pass) {
         if (pass) {
             float *base = nullptr;
-            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return KATSU_OK;
+            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return katsu_f16_drop_call(ctx);
             arena = {reinterpret_cast<char *>(base), 0};
         }
         void *gs = arena.take(staged_bytes(ctx, n, k, oh, ow, gap, tail));
@@ -348,14 +352,14 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         if (dx && (!katsu_f16_window_maps(md.a, sg.planes, q.first_x * (long long)kp, planes, size_t(q.most_taps) * kp,
                                           q.grid_w + q.most_rel_x, oh, n, kp, sg.row(), sg.image(), 1, 64, box_dx) ||
                    !katsu_f16_rows_maps(md.b, ws, planes, width, c, r, width, c * width, plan_dx.bn / 2)))
-            return KATSU_OK;
+            return katsu_f16_drop_call(ctx);
         if (dw && (!x_window_maps(ctx, mw.a, prestaged ? held : own, g, box_dw) ||
                    (prestaged && !x_window_maps(ctx, mw.a_second, own, g, box_dw)) ||
                    !katsu_f16_window_maps(mw.b, sg.planes, 0, planes, kp, ow, oh, n, kp, sg.row(), sg.image(), 1,
                                           plan_dw.bn >= 128 ? 64 : 32, box_dw)))
-            return KATSU_OK;
+            return katsu_f16_drop_call(ctx);
         *handled = 1;
-        const KatsuF16Call call = {{ig, dx ? iw : nullptr, dw ? info : nullptr}};
+        const KatsuF16Call call = katsu_f16_call(ctx, ig, dx ? iw : nullptr, dw ? info : nullptr);
         KatsuAmaxJob amax[3];
         KatsuStageJob jobs[3];
         int na = 0, nj = 0;

@@ -98,10 +98,13 @@ __device__ __forceinline__ void box_origin(const KatsuF16Problem &p, long long b
 
 // One lane's values of columns col .. col + 31.  Few instructions a column: this runs on eight warps per block and sets the
 // pace of layers with short contractions (with its branches inside the loop the small CNN's second dX took 0.58 ms).
-__device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d, int col, const float (&v)[32], float factor) {
+// `bias` is column col + lane's, loaded before the accumulator was waited for; all lanes of the warp call this together.
+__device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d, bool valid, int col, const float (&v)[32],
+                                              float factor, float bias) {
     const long long stride = p.col_stride;
     const int live = p.n_total - col;
     if (live >= 32 && !p.bias && !p.relu && !p.accumulate) {
+        if (!valid) return;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
             *d = v[i] * factor;
@@ -114,22 +117,19 @@ __device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d
     for (int i0 = 0; i0 < 32; i0 += 8) {
         float o[8];
         const bool all = live >= i0 + 8;
-        if (p.accumulate) {  // the loads of eight columns before the first store
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = (all || i0 + i < live) ? d[i * stride] : 0.f;
+        for (int i = 0; i < 8; ++i) o[i] = v[i0 + i] * factor + __shfl_sync(0xffffffffu, bias, i0 + i);
+        if (p.accumulate && valid) {  // the loads of eight columns before the first store
+            float old[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] += v[i0 + i] * factor;
-        } else if (p.bias) {
+            for (int i = 0; i < 8; ++i) old[i] = (all || i0 + i < live) ? d[i * stride] : 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = v[i0 + i] * factor + ((all || i0 + i < live) ? __ldg(p.bias + col + i0 + i) : 0.f);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = v[i0 + i] * factor;
+            for (int i = 0; i < 8; ++i) o[i] += old[i];
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             if (o[i] < floor) o[i] = floor;  // (a NaN stays one)
-            if (all || i0 + i < live) *d = o[i];
+            if (valid && (all || i0 + i < live)) *d = o[i];
             d += stride;
         }
     }
@@ -167,12 +167,14 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
         tmem_alloc_pair(&tmem_slot, 512);
         tmem_relinquish_pair();
     }
+    if (warp == 8 && lane < 2 * NARROW) tma_prefetch_desc(lane < NARROW ? &maps.a[lane] : &maps.b[lane - NARROW]);
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();  // both blocks' barriers exist before anything is signalled across the pair
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_slot;
     launch_wait();
+    const KatsuF16Info info_a = katsu_f16_load(p.info_a), info_b = katsu_f16_load(p.info_b);
     const bool wide = katsu_f16_wide(p.call);
     const int planes = NARROW + (wide ? 1 : 0);
     // k-blocks between two drains: 192 accumulation steps in 3xTF32 mode, up to 12 288 in TF32 mode (4e-4 of 2e-3)
@@ -182,7 +184,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 
     if (warp == 8 && lane == 0) {
         // ---- TMA producer: this block's lanes of A and half of B's columns; bytes counted on the leader's barrier ----
-        const CUtensorMap *map_a = p.a_second && wide && p.info_a->narrow ? maps.a_second : maps.a, *map_b = maps.b;
+        const CUtensorMap *map_a = p.a_second && wide && katsu_f16_narrow(info_a, p.call.span) ? maps.a_second : maps.a, *map_b = maps.b;
         bool ok = true;
         int s = 0;
         uint32_t phase = 1;  // a fresh barrier counts as released
@@ -336,7 +338,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
         const int quarter = warp & 3, group = warp >> 2;
         const int col_chunks = p.bn >> 5;
         float factor = p.gfactor;
-        if (!wide) factor *= __uint_as_float(unsigned(127 - p.info_a->exp - p.info_b->exp) << 23);
+        if (!wide) factor *= __uint_as_float(unsigned(127 - katsu_f16_exp(info_a) - katsu_f16_exp(info_b)) << 23);
         if (p.gscale) factor *= __ldg(p.gscale);
         int q = 0;
         bool alive = true;
@@ -367,6 +369,10 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         at = img * p.img_stride + (long long)y * p.out_w + x;
                     }
                     float *dst = p.out + t.split * p.split_stride + at + n0 * p.col_stride;
+                    auto bias_of = [&](int c0) {
+                        const int col = n0 + c0 + lane;
+                        return p.bias && col < p.n_total ? __ldg(p.bias + col) : 0.f;
+                    };
                     auto wait_acc = [&](int b) -> uint32_t {
                         alive = mbar_wait_warp(&acc_full[b], (q >> 1) & 1, p.status, 174);
                         tc_fence_after_sync();
@@ -382,10 +388,15 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                     };
                     if (kb1 - kb0 <= drain) {
                         // one accumulator holds it all: 32 columns at a time, no sums in registers
+                        float bias[4];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) bias[c] = bias_of((2 * c + group) * 32);
                         const uint32_t acc = kb1 > kb0 ? wait_acc(q & 1) : 0;
                         if (!alive) break;
-#pragma unroll 1
-                        for (int c0 = group * 32; c0 < p.bn; c0 += 64) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const int c0 = (2 * c + group) * 32;
+                            if (c0 >= p.bn) break;
                             float v[32];
                             if (kb1 > kb0) {
                                 tmem_ld_32x32(acc + c0, v);
@@ -393,7 +404,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) v[i] = 0.f;
                             }
-                            if (valid) store_columns(p, dst + c0 * p.col_stride, n0 + c0, v, factor);
+                            store_columns(p, dst + c0 * p.col_stride, valid, n0 + c0, v, factor, bias[c]);
                         }
                         if (kb1 > kb0) {
                             release_acc(q & 1);
@@ -421,11 +432,10 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         release_acc(q & 1);
                     }
                     if (!alive) break;
-                    if (!valid) continue;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int c0 = (2 * c + group) * 32;
-                        if (c0 < p.bn) store_columns(p, dst + c0 * p.col_stride, n0 + c0, run[c], factor);
+                        if (c0 < p.bn) store_columns(p, dst + c0 * p.col_stride, valid, n0 + c0, run[c], factor, bias_of(c0));
                     }
                 }
         }

@@ -101,6 +101,7 @@ int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     q.n_columns = m;
     q.k = k;
     q.out = c;
+    katsu_f16_new_call(ctx);
     KatsuF16Info *ia = katsu_f16_slot(ctx, KATSU_INFO_A), *ib = katsu_f16_slot(ctx, KATSU_INFO_B);
     q.info_lanes = ib;
     q.info_columns = ia;
@@ -108,7 +109,7 @@ int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     for (int pass = 0; pass < 2; ++pass) {  // the first only adds up the sizes
         if (pass) {
             float *base = nullptr;
-            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return KATSU_OK;  // no room: the other kernels
+            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return katsu_f16_drop_call(ctx);  // no room: the other kernels
             arena = {reinterpret_cast<char *>(base), 0};
         }
         q.lanes = arena.planes(n * kp, planes);
@@ -116,7 +117,7 @@ int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b
         float *partial = arena.floats(partial_floats(q));
         if (!pass) continue;
         *handled = 1;
-        const KatsuF16Call call = {{ia, ib, nullptr}};
+        const KatsuF16Call call = katsu_f16_call(ctx, ia, ib, nullptr);
         const KatsuAmaxJob amax[2] = {{a, m * k, ia}, {b, k * n, ib}};
         KATSU_TRY(katsu_f16_amax(ctx, amax, 2));
         const KatsuStageJob jobs[2] = {transposed_job(b, k, n, q.lanes, ib), rows_job(a, m, k, q.columns, ia)};
@@ -131,6 +132,7 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     *handled = 0;
     if (!takes(ctx, m, k, n)) return KATSU_OK;
     const int planes = katsu_f16_narrow_planes(ctx) + 1;
+    katsu_f16_new_call(ctx);
     KatsuF16Info *ia = katsu_f16_slot(ctx, KATSU_INFO_A), *ib = katsu_f16_slot(ctx, KATSU_INFO_B), *ig = katsu_f16_slot(ctx, KATSU_INFO_G);
     Product qa = {}, qb = {};
     qa.plan = plan_for(ctx, k, m, n);
@@ -148,7 +150,7 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     for (int pass = 0; pass < 2; ++pass) {
         if (pass) {
             float *base = nullptr;
-            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return KATSU_OK;
+            if (katsu_scratch(ctx, arena.bytes / 4, &base) != KATSU_OK) return katsu_f16_drop_call(ctx);
             arena = {reinterpret_cast<char *>(base), 0};
         }
         float *partial_a = nullptr, *partial_b = nullptr;
@@ -164,7 +166,7 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
         }
         if (!pass) continue;
         *handled = 1;
-        const KatsuF16Call call = {{ig, da ? ib : nullptr, db ? ia : nullptr}};
+        const KatsuF16Call call = katsu_f16_call(ctx, ig, da ? ib : nullptr, db ? ia : nullptr);
         KatsuAmaxJob amax[3];
         KatsuStageJob jobs[4];
         int na = 0, nj = 0;

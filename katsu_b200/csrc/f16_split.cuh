@@ -23,22 +23,38 @@
 
 #include "common.cuh"
 
+// What the magnitude pass finds of an operand, as f32 bit patterns: the largest magnitude, and 0x7fffffff minus the
+// smallest maximum of a group (so that both grow from zero and both are plain atomic maxima).
 struct KatsuF16Info {
-    int narrow;  // 1: fp16 planes can stand for the tensor
-    int exp;     // scale exponent of those
+    unsigned most, inverted_least;
 };
 
-// The operands of one call (unused entries null).
+// The operands of one call (unused entries null) and the range that counts as narrow in its mode: 2^span.
 struct KatsuF16Call {
     const KatsuF16Info *info[3];
+    int span;
 };
 
+// 2^-48 .. 2^48 keeps the product of two operands' scales inside f32.
+__device__ __forceinline__ bool katsu_f16_narrow(KatsuF16Info info, int span) {
+    const int top = int(info.most >> 23), low = int((0x7fffffffu - info.inverted_least) >> 23);
+    return info.most == 0 || (top >= 127 - 48 && top <= 127 + 48 && top - low < span);
+}
+
+__device__ __forceinline__ int katsu_f16_exp(KatsuF16Info info) {  // of a narrow operand
+    return info.most == 0 ? 0 : 14 - (int(info.most >> 23) - 127);
+}
+
+__device__ __forceinline__ KatsuF16Info katsu_f16_load(const KatsuF16Info *info) {
+    const uint2 v = *reinterpret_cast<const uint2 *>(info);
+    return KatsuF16Info{v.x, v.y};
+}
+
 __device__ __forceinline__ bool katsu_f16_wide(const KatsuF16Call &call) {
-    bool narrow = true;
+    KatsuF16Info v[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-        if (call.info[i]) narrow = narrow && call.info[i]->narrow;
-    return !narrow;
+    for (int i = 0; i < 3; ++i) v[i] = call.info[i] ? katsu_f16_load(call.info[i]) : KatsuF16Info{0, 0};
+    return !(katsu_f16_narrow(v[0], call.span) && katsu_f16_narrow(v[1], call.span) && katsu_f16_narrow(v[2], call.span));
 }
 
 // One operand whose magnitude is to be found.
@@ -70,6 +86,7 @@ struct KatsuStageJob {
     const float *src;
     KatsuF16Planes to;
     const KatsuF16Info *info;
+    KatsuF16Info *info_copy;  // where to leave a copy of it, or null
     int only_if_mixed;  // 1: written only when this operand is narrow and the call is not (a narrow copy exists already)
     int n, c, h, w, gap, cp, tail;
     int k, r, s, width, backward, classes, stride;
@@ -85,9 +102,13 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
 // Planes of the narrow form in the context's mode, and of room for either form.
 static inline int katsu_f16_narrow_planes(const katsu_cuda_ctx *ctx) { return ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1; }
 
-// Device slots for the operands of one call.
+// Device slots for the operands of one call.  There are two sets, used in turn: the staging pass of a call clears the
+// other one for the next call.  katsu_f16_new_call picks the set and must come before the call's slots are taken.
 enum { KATSU_INFO_A, KATSU_INFO_B, KATSU_INFO_G, KATSU_INFO_SLOTS };
+void katsu_f16_new_call(katsu_cuda_ctx *ctx);
+int32_t katsu_f16_drop_call(katsu_cuda_ctx *ctx);  // nothing was launched for it after all; KATSU_OK
 KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot);
+KatsuF16Call katsu_f16_call(const katsu_cuda_ctx *ctx, const KatsuF16Info *a, const KatsuF16Info *b, const KatsuF16Info *c);
 
 // Bump allocator over a scratch block; every piece is 256-byte aligned.
 struct KatsuArena {

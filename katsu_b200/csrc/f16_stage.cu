@@ -12,22 +12,16 @@ namespace {
 constexpr int THREADS = 256;
 
 // ---- largest magnitude ------------------------------------------------------------------------------------------
-struct AmaxAcc {
-    unsigned amax, inverted_min, ticket, pad;
-};
-
 struct AmaxSegment {
     const float *src;
     unsigned long long count;
     KatsuF16Info *info;
-    AmaxAcc *acc;
     unsigned first_block, blocks;
 };
 
 struct AmaxParams {
     AmaxSegment seg[3];
     int segments;
-    int span;  // groups must reach 2^-span of the tensor's maximum
 };
 
 __device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
@@ -89,31 +83,16 @@ __global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ A
         most = max(most, sh_most[i]);
         least = min(least, sh_least[i]);
     }
-    atomicMax(&sg.acc->amax, most);
-    atomicMax(&sg.acc->inverted_min, 0x7fffffffu - least);
-    __threadfence();
-    if (atomicAdd(&sg.acc->ticket, 1u) != sg.blocks - 1) return;
-    // last block of the segment: publish, and leave the accumulator as the next launch wants to find it
-    __threadfence();
-    most = atomicExch(&sg.acc->amax, 0u);
-    least = 0x7fffffffu - atomicExch(&sg.acc->inverted_min, 0u);
-    atomicExch(&sg.acc->ticket, 0u);
-    KatsuF16Info info;
-    const int exponent = int(most >> 23) - 127;  // floor(log2(amax)) of a normal number
-    info.exp = 14 - exponent;
-    // 2^-48 .. 2^48 keeps the product of two operands' scales inside f32
-    info.narrow = exponent >= -48 && exponent <= 48 && (int(most >> 23) - int(least >> 23)) < p.span;
-    if (most == 0) {  // all zeros
-        info.exp = 0;
-        info.narrow = 1;
-    }
-    *sg.info = info;
+    // no result is waited for: the kernels behind this one read the slots when it has ended
+    atomicMax(&sg.info->most, most);
+    if (most) atomicMax(&sg.info->inverted_least, 0x7fffffffu - least);
 }
 
 // ---- fp16 planes ------------------------------------------------------------------------------------------------
 struct StageParams {
     KatsuF16Call call;
     int narrow_planes;
+    KatsuF16Info *clear;  // the other set of slots
     KatsuStageJob job[KATSU_STAGE_JOBS];
     unsigned first_block[KATSU_STAGE_JOBS], blocks[KATSU_STAGE_JOBS];
     int jobs;
@@ -338,10 +317,13 @@ __global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ 
     const unsigned block = blockIdx.x - p.first_block[ji];
     Writer out;
     out.to = j.to;
+    const KatsuF16Info own = katsu_f16_load(j.info);
     out.wide = katsu_f16_wide(p.call);
     out.planes = p.narrow_planes + (out.wide ? 1 : 0);
-    out.scale = out.wide ? 1.f : __uint_as_float(unsigned(127 + j.info->exp) << 23);
-    if (j.only_if_mixed && !(out.wide && j.info->narrow)) return;
+    out.scale = out.wide ? 1.f : __uint_as_float(unsigned(127 + katsu_f16_exp(own)) << 23);
+    if (blockIdx.x == 0 && threadIdx.x < KATSU_INFO_SLOTS) p.clear[threadIdx.x] = KatsuF16Info{0, 0};
+    if (block == 0 && threadIdx.x == 0 && j.info_copy) *j.info_copy = own;
+    if (j.only_if_mixed && !(out.wide && katsu_f16_narrow(own, p.call.span))) return;
     if (j.kind == KATSU_STAGE_NHWC) {
         if (block == 0) {
             // zero pixels in front of the first row, zeros behind the last
@@ -365,21 +347,32 @@ __global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ 
 
 }  // namespace
 
-KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) {
-    return reinterpret_cast<KatsuF16Info *>(static_cast<char *>(ctx->f16_state) + 256) + slot;
+static KatsuF16Info *slots(const katsu_cuda_ctx *ctx, int set) {
+    return reinterpret_cast<KatsuF16Info *>(static_cast<char *>(ctx->f16_state) + set * 64);
+}
+
+void katsu_f16_new_call(katsu_cuda_ctx *ctx) { ctx->f16_set ^= 1; }
+
+int32_t katsu_f16_drop_call(katsu_cuda_ctx *ctx) {
+    ctx->f16_set ^= 1;
+    return KATSU_OK;
+}
+
+KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) { return slots(ctx, ctx->f16_set) + slot; }
+
+KatsuF16Call katsu_f16_call(const katsu_cuda_ctx *ctx, const KatsuF16Info *a, const KatsuF16Info *b, const KatsuF16Info *c) {
+    return KatsuF16Call{{a, b, c}, ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28};
 }
 
 int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count) {
     AmaxParams p;
     p.segments = count;
-    p.span = ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28;
     unsigned at = 0;
     for (int i = 0; i < count; ++i) {
         AmaxSegment &s = p.seg[i];
         s.src = jobs[i].src;
         s.count = jobs[i].count;
         s.info = jobs[i].info;
-        s.acc = static_cast<AmaxAcc *>(ctx->f16_state) + i;
         // a warp takes eight groups of 128 at once; at most eight resident blocks per SM
         size_t blocks = katsu_div_up(jobs[i].count, size_t(128) * 8 * (THREADS / 32));
         if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
@@ -396,6 +389,7 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
     StageParams p;
     p.call = call;
     p.narrow_planes = katsu_f16_narrow_planes(ctx);
+    p.clear = slots(ctx, ctx->f16_set ^ 1);
     p.jobs = count;
     size_t at = 0;
     for (int i = 0; i < count; ++i) {
