@@ -64,6 +64,9 @@ int32_t katsu_scratch(katsu_cuda_ctx *ctx, size_t floats, float **out);
 // Stream-ordered allocation from the context's pool.
 int32_t katsu_pool_alloc(katsu_cuda_ctx *ctx, size_t bytes, void **out);
 
+// Whether the context's stream is being captured into a graph.
+bool katsu_capturing(const katsu_cuda_ctx *ctx);
+
 // cudaStreamSynchronize plus the status word of the bounded device-side waits: KATSU_ERR_TIMEOUT
 // (once; the word is cleared) when a wait gave up in any launch since the last check.
 int32_t katsu_sync_and_check(katsu_cuda_ctx *ctx);

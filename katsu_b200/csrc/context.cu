@@ -36,11 +36,14 @@ int32_t katsu_prepare_kernel(katsu_cuda_ctx *ctx, const void *kernel, size_t sme
     static std::unordered_map<const void *, size_t> *prepared = new std::unordered_map<const void *, size_t>[64];
     const std::lock_guard<std::mutex> hold(lock);
     std::unordered_map<const void *, size_t> &of_device = prepared[ctx->device & 63];
-    auto it = of_device.find(kernel);
+    const auto it = of_device.find(kernel);
     if (it != of_device.end() && it->second >= smem) return KATSU_OK;
     if (smem) KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KATSU_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    of_device[kernel] = smem;
+    try {
+        of_device[kernel] = smem;
+    } catch (...) {  // no host memory for the entry: set again by the next launch
+    }
     return KATSU_OK;
 }
 
@@ -50,9 +53,14 @@ int32_t katsu_prepare_kernel(katsu_cuda_ctx *ctx, const void *kernel, size_t sme
 // memory inside a step (the small CNN's step took 3 to 40 ms that way, 2 ms of it kernels).  So a freed block stays
 // whole and goes to the next request of nearly its size.  All use of a context's blocks is on its one stream, so reuse
 // needs no event, and one host thread drives a context.  At most an eighth of the device's memory is held; an allocation
-// that fails gives everything held back and tries again; shutdown gives everything back.
+// (the scratch block's too) that fails gives everything held back and tries again; shutdown gives everything back.
+struct KatsuBlock {
+    size_t bytes;
+    bool held;  // freed by the caller and not handed out again
+};
+
 struct KatsuBlockCache {
-    std::unordered_map<void *, size_t> sizes;  // of every block this context has handed out or holds
+    std::unordered_map<void *, KatsuBlock> blocks;  // every block this context has handed out or holds
     std::multimap<size_t, void *> held;
     size_t held_bytes = 0, most_bytes = 0;
 };
@@ -62,17 +70,24 @@ static size_t block_bytes(size_t bytes) {
     return (bytes + grain - 1) / grain * grain;
 }
 
+bool katsu_capturing(const katsu_cuda_ctx *ctx) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(ctx->stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+}
+
 static void give_back_blocks(katsu_cuda_ctx *ctx) {
     KatsuBlockCache &cache = *ctx->blocks;
     for (auto &entry : cache.held) {
-        cache.sizes.erase(entry.second);
+        cache.blocks.erase(entry.second);
         cudaFreeAsync(entry.second, ctx->stream);
     }
     cache.held.clear();
     cache.held_bytes = 0;
 }
 
+// While the stream is being captured the cache stays out of it: what a capture allocates belongs to its graph.
 static int32_t take_block(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
+    if (katsu_capturing(ctx)) return katsu_pool_alloc(ctx, bytes, out);
     KatsuBlockCache &cache = *ctx->blocks;
     const size_t want = block_bytes(bytes);
     auto it = cache.held.lower_bound(want);
@@ -80,36 +95,53 @@ static int32_t take_block(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
         *out = it->second;
         cache.held_bytes -= it->first;
         cache.held.erase(it);
+        cache.blocks.find(*out)->second.held = false;
         return KATSU_OK;
     }
-    int32_t rc = katsu_pool_alloc(ctx, want, out);
-    if (rc != KATSU_OK && !cache.held.empty()) {
-        give_back_blocks(ctx);
-        cudaStreamSynchronize(ctx->stream);
-        rc = katsu_pool_alloc(ctx, want, out);
+    KATSU_TRY(katsu_pool_alloc(ctx, want, out));
+    try {
+        cache.blocks[*out] = KatsuBlock{want, false};
+    } catch (...) {  // no host memory for the entry: the block goes straight back to the pool when it is freed
     }
-    if (rc == KATSU_OK) cache.sizes[*out] = want;
-    return rc;
+    return KATSU_OK;
 }
 
-// False when the block is not one of this context's (another context of the device handed it out).
-static bool keep_block(katsu_cuda_ctx *ctx, void *ptr) {
+// *kept = false when the block has to go to the driver (another context of the device handed it out, a capture runs, or
+// the cache is full).  A block that the caller has freed already is refused, as the driver refuses it.
+static int32_t keep_block(katsu_cuda_ctx *ctx, void *ptr, bool *kept) {
+    *kept = false;
     KatsuBlockCache &cache = *ctx->blocks;
-    auto it = cache.sizes.find(ptr);
-    if (it == cache.sizes.end()) return false;
-    const size_t bytes = it->second;
-    if (cache.held_bytes + bytes > cache.most_bytes) {
-        cache.sizes.erase(it);
-        return false;
+    auto it = cache.blocks.find(ptr);
+    if (it == cache.blocks.end()) return KATSU_OK;
+    if (it->second.held) return katsu_set_error(KATSU_ERR_CUDA, "block %p is freed twice", ptr);
+    if (katsu_capturing(ctx)) return KATSU_OK;
+    const size_t bytes = it->second.bytes;
+    try {
+        if (cache.held_bytes + bytes <= cache.most_bytes) {
+            cache.held.emplace(bytes, ptr);
+            cache.held_bytes += bytes;
+            it->second.held = *kept = true;
+            return KATSU_OK;
+        }
+    } catch (...) {
     }
-    cache.held.emplace(bytes, ptr);
-    cache.held_bytes += bytes;
-    return true;
+    cache.blocks.erase(it);
+    return KATSU_OK;
+}
+
+static cudaError_t pool_malloc(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
+    return ctx->pool != nullptr ? cudaMallocFromPoolAsync(out, bytes, (cudaMemPool_t)ctx->pool, ctx->stream)
+                                : cudaMallocAsync(out, bytes, ctx->stream);
 }
 
 int32_t katsu_pool_alloc(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
-    cudaError_t err = ctx->pool != nullptr ? cudaMallocFromPoolAsync(out, bytes, (cudaMemPool_t)ctx->pool, ctx->stream)
-                                           : cudaMallocAsync(out, bytes, ctx->stream);
+    cudaError_t err = pool_malloc(ctx, bytes, out);
+    if (err != cudaSuccess && !ctx->blocks->held.empty() && !katsu_capturing(ctx)) {
+        cudaGetLastError();
+        give_back_blocks(ctx);
+        cudaStreamSynchronize(ctx->stream);
+        err = pool_malloc(ctx, bytes, out);
+    }
     if (err != cudaSuccess) {
         cudaGetLastError();
         *out = nullptr;
@@ -317,7 +349,9 @@ extern "C" int32_t katsu_cuda_free(katsu_cuda_ctx *ctx, float *ptr) {
     if (ptr == nullptr) return KATSU_OK;
     // Stream-ordered: work already queued on this context's stream may still use the block;
     // work queued on another context must have been synchronised by the caller.
-    if (!keep_block(ctx, ptr)) KATSU_CUDA_TRY(cudaFreeAsync(ptr, ctx->stream));
+    bool kept = false;
+    KATSU_TRY(keep_block(ctx, ptr, &kept));
+    if (!kept) KATSU_CUDA_TRY(cudaFreeAsync(ptr, ctx->stream));
     return KATSU_OK;
 }
 
