@@ -30,6 +30,7 @@ struct katsu_cuda_ctx {
     // 1 KiB of device memory: what the magnitude pass found of a call's operands (f16_split.cuh, first half), ticket of the sum (streaming.cu, at 512).
     void *f16_state;
     int f16_set;  // set of operand slots of the current call
+    bool f16_captured;  // the current call is being captured into a graph
     // Buffer written by katsu_cuda_flush_l2.
     float *flush;
     size_t flush_floats;

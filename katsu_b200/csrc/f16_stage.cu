@@ -88,11 +88,15 @@ __global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ A
     if (most) atomicMax(&sg.info->inverted_least, 0x7fffffffu - least);
 }
 
+__global__ void clear_kernel(KatsuF16Info *info) {
+    if (threadIdx.x < KATSU_INFO_SLOTS) info[threadIdx.x] = KatsuF16Info{0, 0};
+}
+
 // ---- fp16 planes ------------------------------------------------------------------------------------------------
 struct StageParams {
     KatsuF16Call call;
     int narrow_planes;
-    KatsuF16Info *clear;  // the other set of slots
+    KatsuF16Info *clear;  // the other set of slots, or null
     KatsuStageJob job[KATSU_STAGE_JOBS];
     unsigned first_block[KATSU_STAGE_JOBS], blocks[KATSU_STAGE_JOBS];
     int jobs;
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ 
     out.wide = katsu_f16_wide(p.call);
     out.planes = p.narrow_planes + (out.wide ? 1 : 0);
     out.scale = out.wide ? 1.f : __uint_as_float(unsigned(127 + katsu_f16_exp(own)) << 23);
-    if (blockIdx.x == 0 && threadIdx.x < KATSU_INFO_SLOTS) p.clear[threadIdx.x] = KatsuF16Info{0, 0};
+    if (p.clear && blockIdx.x == 0 && threadIdx.x < KATSU_INFO_SLOTS) p.clear[threadIdx.x] = KatsuF16Info{0, 0};
     if (block == 0 && threadIdx.x == 0 && j.info_copy) *j.info_copy = own;
     if (j.only_if_mixed && !(out.wide && katsu_f16_narrow(own, p.call.span))) return;
     if (j.kind == KATSU_STAGE_NHWC) {
@@ -351,14 +355,19 @@ static KatsuF16Info *slots(const katsu_cuda_ctx *ctx, int set) {
     return reinterpret_cast<KatsuF16Info *>(static_cast<char *>(ctx->f16_state) + set * 64);
 }
 
-void katsu_f16_new_call(katsu_cuda_ctx *ctx) { ctx->f16_set ^= 1; }
+// Set 2 is that of captured calls, which clear it themselves: a graph is replayed with the set it was captured with, at
+// any point between other calls.
+void katsu_f16_new_call(katsu_cuda_ctx *ctx) {
+    ctx->f16_captured = katsu_capturing(ctx);
+    if (!ctx->f16_captured) ctx->f16_set ^= 1;
+}
 
 int32_t katsu_f16_drop_call(katsu_cuda_ctx *ctx) {
-    ctx->f16_set ^= 1;
+    if (!ctx->f16_captured) ctx->f16_set ^= 1;
     return KATSU_OK;
 }
 
-KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) { return slots(ctx, ctx->f16_set) + slot; }
+KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) { return slots(ctx, ctx->f16_captured ? 2 : ctx->f16_set) + slot; }
 
 KatsuF16Call katsu_f16_call(const katsu_cuda_ctx *ctx, const KatsuF16Info *a, const KatsuF16Info *b, const KatsuF16Info *c) {
     return KatsuF16Call{{a, b, c}, ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28};
@@ -381,6 +390,7 @@ int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count)
         s.blocks = (unsigned)blocks;
         at += s.blocks;
     }
+    if (ctx->f16_captured) KATSU_LAUNCH(ctx, clear_kernel, 1, 32, 0, katsu_f16_slot(ctx, 0));
     KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)amax_kernel, 0));
     return katsu_launch_chained(ctx, amax_kernel, at, THREADS, 0, 1, p);
 }
@@ -389,7 +399,7 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
     StageParams p;
     p.call = call;
     p.narrow_planes = katsu_f16_narrow_planes(ctx);
-    p.clear = slots(ctx, ctx->f16_set ^ 1);
+    p.clear = ctx->f16_captured ? nullptr : slots(ctx, ctx->f16_set ^ 1);
     p.jobs = count;
     size_t at = 0;
     for (int i = 0; i < count; ++i) {
