@@ -10,6 +10,7 @@
 namespace {
 
 constexpr int THREADS = 256;
+constexpr int STAGE_BLOCKS = 5;  // resident staging blocks per SM
 
 // ---- largest magnitude ------------------------------------------------------------------------------------------
 struct AmaxSegment {
@@ -42,35 +43,45 @@ __global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ A
     const unsigned long long stride = (unsigned long long)sg.blocks * (THREADS / 32);
     const bool vec = (reinterpret_cast<uintptr_t>(sg.src) & 15u) == 0;
     unsigned most = 0, least = 0x7fffffffu;
-    auto load = [&](unsigned long long g) -> unsigned {
-        unsigned long long at = g * 128;
-        unsigned m = 0;
-        if (at + 128 <= sg.count && vec) {
-            m = max4(__ldg(reinterpret_cast<const float4 *>(sg.src + at) + lane));
-        } else {
-            if (at + 128 > sg.count) at = sg.count > 128 ? sg.count - 128 : 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const unsigned long long e = at + lane + 32 * i;
-                if (e < sg.count) m = max(m, magnitude(__ldg(sg.src + e)));
-            }
-        }
-        return m;
-    };
     auto take = [&](unsigned m) {
         m = __reduce_max_sync(0xffffffffu, m);
         most = max(most, m);
-        if (m != 0) least = min(least, m);
+        least = min(least, m ? m : 0x7fffffffu);
     };
-    unsigned long long g = (unsigned long long)(blockIdx.x - sg.first_block) * (THREADS / 32) + warp;
-    for (; g + 7 * stride < groups; g += 8 * stride) {  // eight 16-byte loads in flight per thread
-        unsigned m[8];
+    auto load = [&](unsigned long long g) -> unsigned {  // any group
+        unsigned long long at = g * 128;
+        if (at + 128 > sg.count) at = sg.count > 128 ? sg.count - 128 : 0;
+        unsigned m = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) m[i] = load(g + i * stride);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) take(m[i]);
+        for (int i = 0; i < 4; ++i) {
+            const unsigned long long e = at + lane + 32 * i;
+            if (e < sg.count) m = max(m, magnitude(__ldg(sg.src + e)));
+        }
+        return m;
+    };
+    // Warps walk from the tensor's end to its front: the staging pass starts at the front, which then is what L2 holds.
+    // `left` groups are not yet read by anybody from this warp's place on; its next one is left - 1.
+    long long left = (long long)groups - ((long long)(blockIdx.x - sg.first_block) * (THREADS / 32) + warp);
+    const long long step = (long long)stride;
+    if ((sg.count & 127) != 0 && left == (long long)groups) {  // the ragged last group
+        take(load(groups - 1));
+        left -= step;
     }
-    for (; g < groups; g += stride) take(load(g));
+    if (vec) {
+        // Eight 16-byte loads in flight per thread, with no branch between them: with the range checks of load() around
+        // each the compiler kept one in flight (103 M floats: 100 us).
+        const float4 *src = reinterpret_cast<const float4 *>(sg.src) + lane;
+        for (; left > 7 * step; left -= 8 * step) {
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(src + (left - 1 - i * step) * 32);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) take(max4(v[i]));
+        }
+        for (; left > 0; left -= step) take(max4(__ldg(src + (left - 1) * 32)));
+    } else {
+        for (; left > 0; left -= step) take(load(left - 1));
+    }
 
     __shared__ unsigned sh_most[THREADS / 32], sh_least[THREADS / 32];
     if (lane == 0) {
@@ -167,70 +178,93 @@ __device__ __forceinline__ void zero8(const Writer &w, size_t at) {
 // bank conflicts: a warp writes one or two channel rows, and reads 8 channel groups of 4 pixels (CT = 64) or 4 groups of
 // 8 pixels (CT = 32).  Few instructions a value matter here: with a thread per channel pair, and a division per pixel and
 // channel, this pass was bound by instruction issue (0.20 ms for 103 M values, 4.1 TB/s).
+//
+// A block walks over tiles `block`, `block + blocks` ..., the loads of the next one in flight while it writes the present
+// one.  (One tile to a block, with its wait for the scale and for the loads in front of every store, took 164 us for 103 M
+// values into two planes.)
 template <int CT>
-__device__ void stage_nhwc_tiles(const KatsuStageJob &j, const Writer &out, unsigned block, float *tile) {
+__device__ void stage_nhwc_tiles(const KatsuStageJob &j, const Writer &out, unsigned block, unsigned blocks, float *tile) {
     constexpr int PT = 4096 / CT, GROUPS = CT / 8, XOR = 32 / GROUPS;
-    const int hw = j.h * j.w, ptiles = (hw + PT - 1) / PT, ctiles = (j.c + CT - 1) / CT;
-    const unsigned n = block / unsigned(ptiles * ctiles), rest = block - n * unsigned(ptiles * ctiles);
-    const int pt = rest / unsigned(ctiles);
-    const int p0 = pt * PT, c0 = (rest - pt * ctiles) * CT;
-    const float *src = j.src + (size_t(n) * j.c + c0) * hw + p0;
-    const int channels = min(j.c - c0, CT), pixels = min(hw - p0, PT);
-    if ((hw & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15u) == 0) {
-        // a float4 a thread: PT / 4 threads to a channel
-        const int quad = threadIdx.x % (PT / 4), row0 = threadIdx.x / (PT / 4);
-        constexpr int STEP = THREADS / (PT / 4);
-        float4 v[CT / STEP];
+    const int hw = j.h * j.w;
+    const unsigned ptiles = (hw + PT - 1) / PT, ctiles = (j.c + CT - 1) / CT, tiles = unsigned(j.n) * ptiles * ctiles;
+    const bool vec = (hw & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15u) == 0;
+    // vec: a float4 a thread, PT / 4 threads to a channel; else a float a thread, PT threads to a channel
+    constexpr int VSTEP = THREADS / (PT / 4), STEP = THREADS / PT;
+    const int quad = threadIdx.x % (PT / 4), vrow = threadIdx.x / (PT / 4);
+    const int col0 = threadIdx.x % PT, row0 = threadIdx.x / PT;
+    float v[16];
+    unsigned n = 0;
+    int p0 = 0, c0 = 0;
+    auto load = [&](unsigned t) {
+        n = t / (ptiles * ctiles);
+        const unsigned rest = t - n * (ptiles * ctiles), pt = rest / ctiles;
+        p0 = int(pt) * PT;
+        c0 = int(rest - pt * ctiles) * CT;
+        const float *src = j.src + (size_t(n) * j.c + c0) * hw + p0;
+        const int channels = min(j.c - c0, CT), pixels = min(hw - p0, PT);
+        if (vec) {
 #pragma unroll
-        for (int i = 0; i < CT / STEP; ++i) {
-            const int row = row0 + STEP * i;
-            v[i] = (row < channels && quad * 4 < pixels) ? __ldg(reinterpret_cast<const float4 *>(src + size_t(row) * hw) + quad)
-                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+            for (int i = 0; i < 4; ++i) {
+                const int row = vrow + VSTEP * i;
+                const float4 q = (row < channels && quad * 4 < pixels)
+                                     ? __ldg(reinterpret_cast<const float4 *>(src + size_t(row) * hw) + quad)
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
+            }
+        } else {
 #pragma unroll
-        for (int i = 0; i < CT / STEP; ++i) {
-            const int row = row0 + STEP * i;
-            const int col = (quad * 4) ^ ((row >> 3) * XOR);
-            *reinterpret_cast<float4 *>(tile + row * PT + col) = v[i];
+            for (int i = 0; i < 16; ++i) {
+                const int row = row0 + STEP * i;
+                v[i] = (row < channels && col0 < pixels) ? __ldg(src + size_t(row) * hw + col0) : 0.f;
+            }
         }
-    } else {
-        const int col0 = threadIdx.x % PT, row0 = threadIdx.x / PT;
-        constexpr int STEP = THREADS / PT;
-        float v[CT / STEP];
-#pragma unroll
-        for (int i = 0; i < CT / STEP; ++i) {
-            const int row = row0 + STEP * i;
-            v[i] = (row < channels && col0 < pixels) ? __ldg(src + size_t(row) * hw + col0) : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < CT / STEP; ++i) {
-            const int row = row0 + STEP * i;
-            tile[row * PT + (col0 ^ ((row >> 3) * XOR))] = v[i];
-        }
-    }
-    __syncthreads();
+    };
     const int g = threadIdx.x % GROUPS, first = threadIdx.x / GROUPS;
-    if (c0 + g * 8 >= j.cp) return;
-    constexpr int STEP = THREADS / GROUPS;
-    int y = (p0 + first) / j.w, x = (p0 + first) - y * j.w;
     const float *column = tile + g * 8 * PT;
+    constexpr int PSTEP = THREADS / GROUPS;
+    unsigned t = block;
+    if (t < tiles) load(t);
+    for (; t < tiles; t += blocks) {
+        if (vec) {
 #pragma unroll
-    for (int i = 0; i < PT / STEP; ++i) {
-        const int p = first + STEP * i;
-        if (p >= pixels) break;
-        const float *from = column + (p ^ (g * XOR));
-        float v[8];
+            for (int i = 0; i < 4; ++i) {
+                const int row = vrow + VSTEP * i;
+                *reinterpret_cast<float4 *>(tile + row * PT + ((quad * 4) ^ ((row >> 3) * XOR))) =
+                    make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+        } else {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = from[u * PT];
-        const size_t at = ((size_t(n) * j.h + y) * (j.w + j.gap) + x) * j.cp + c0 + g * 8;
-        write8(out, at, v);
-        if (x == j.w - 1)
-            for (int q = 1; q <= j.gap; ++q) zero8(out, at + size_t(q) * j.cp);
-        x += STEP;
-        while (x >= j.w) {
-            x -= j.w;
-            ++y;
+            for (int i = 0; i < 16; ++i) {
+                const int row = row0 + STEP * i;
+                tile[row * PT + (col0 ^ ((row >> 3) * XOR))] = v[i];
+            }
         }
+        const int channel = c0 + g * 8, from0 = p0 + first, pixels = min(hw - p0, PT);
+        const size_t image = size_t(n) * j.h;
+        __syncthreads();
+        if (t + blocks < tiles) load(t + blocks);
+        if (channel < j.cp) {
+            int y = from0 / j.w, x = from0 - y * j.w;
+#pragma unroll
+            for (int i = 0; i < PT / PSTEP; ++i) {
+                const int p = first + PSTEP * i;
+                if (p >= pixels) break;
+                const float *from = column + (p ^ (g * XOR));
+                float o[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) o[u] = from[u * PT];
+                const size_t at = ((image + y) * (j.w + j.gap) + x) * j.cp + channel;
+                write8(out, at, o);
+                if (x == j.w - 1)
+                    for (int q = 1; q <= j.gap; ++q) zero8(out, at + size_t(q) * j.cp);
+                x += PSTEP;
+                while (x >= j.w) {
+                    x -= j.w;
+                    ++y;
+                }
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -311,7 +345,7 @@ __device__ void stage_weights(const KatsuStageJob &j, const Writer &out, unsigne
     }
 }
 
-__global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ StageParams p) {
+__global__ void __launch_bounds__(THREADS, STAGE_BLOCKS) stage_kernel(const __grid_constant__ StageParams p) {
     __shared__ __align__(16) float tile[4096];
     launch_next();
     launch_wait();
@@ -340,8 +374,8 @@ __global__ void __launch_bounds__(THREADS) stage_kernel(const __grid_constant__ 
             for (int i = threadIdx.x * 8; i < j.tail; i += THREADS * 8) zero8(out, end + i);
         }
         if (j.c <= 16) stage_nhwc_narrow(j, out, block, p.blocks[ji]);
-        else if (tile_channels(j.c) == 32) stage_nhwc_tiles<32>(j, out, block, tile);
-        else stage_nhwc_tiles<64>(j, out, block, tile);
+        else if (tile_channels(j.c) == 32) stage_nhwc_tiles<32>(j, out, block, p.blocks[ji], tile);
+        else stage_nhwc_tiles<64>(j, out, block, p.blocks[ji], tile);
     } else if (j.kind == KATSU_STAGE_ROWS) {
         stage_rows(j, out, block, p.blocks[ji]);
     } else {
@@ -410,6 +444,8 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
         if (j.kind == KATSU_STAGE_NHWC && j.c > 16) {
             const size_t ct = tile_channels(j.c);
             blocks = size_t(j.n) * katsu_div_up(hw, 4096 / ct) * katsu_div_up((size_t)j.c, ct);
+            if (blocks > 0x3fffffff) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "operand too large to stage");
+            if (blocks > size_t(ctx->num_sms) * STAGE_BLOCKS) blocks = size_t(ctx->num_sms) * STAGE_BLOCKS;
         } else {
             const size_t units = j.kind == KATSU_STAGE_NHWC ? size_t(j.n) * hw * (j.cp / 8)
                                  : j.kind == KATSU_STAGE_ROWS ? size_t(j.n) * (j.cp / 8)
@@ -417,6 +453,8 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
             blocks = katsu_div_up(units, (size_t)THREADS);
             if (blocks > size_t(ctx->num_sms) * 64) blocks = size_t(ctx->num_sms) * 64;
         }
+        // (as many blocks would do nothing but start and end when the copy is not needed: 30 us for 25 000)
+        if (j.only_if_mixed && blocks > (size_t)ctx->num_sms) blocks = (size_t)ctx->num_sms;
         p.first_block[i] = (unsigned)at;
         p.blocks[i] = (unsigned)blocks;
         at += blocks;

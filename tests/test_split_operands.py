@@ -56,6 +56,23 @@ def test_convolution_edges(ctx, oracle, shape):
         assert max(errors) <= bar, (shape, mode, errors)
 
 
+# more tiles of 64 x 64 or 32 channels x 128 pixels than staging blocks run at a time (5 to an SM; one to an SM for the copy
+# of x beside the caller's), pixels a multiple of 4 and not
+@pytest.mark.parametrize("shape", [(12, 70, 47, 45, 24, 1, 1, 1, 0), (12, 70, 48, 45, 24, 1, 1, 1, 0), (48, 28, 47, 45, 24, 1, 1, 1, 0)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("staged", [False, True], ids=["plain", "staged"])
+def test_staging_blocks_take_several_tiles(ctx, oracle, shape, staged):
+    n, c, h, w, k = shape[:5]
+    if staged:
+        shape = (n, c // 4 * 4, *shape[2:])  # what the caller can stage
+        c = shape[1]
+    rng = np.random.default_rng(n + c)
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c, n * k * h * w))
+    if staged:
+        g[:g.size // n] *= np.float32(1e-9)  # wide: the copy beside the caller's is written
+    assert max(conv_errors(ctx, oracle, shape, x, wt, g, staged, "g" if staged else None)) <= REL_L2_TOL
+
+
 @pytest.mark.parametrize("staged", [False, True], ids=["plain", "staged"])
 @pytest.mark.parametrize("small", ["x", "g"])
 def test_one_image_far_below_the_others(ctx, oracle, small, staged):
