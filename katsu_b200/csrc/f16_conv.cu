@@ -106,6 +106,7 @@ struct Classes {
     short off_h[KATSU_F16_MAX_ROWS], ky[KATSU_F16_MAX_ROWS];
     int taps_x[KATSU_F16_MAX_CLASSES], off_x[KATSU_F16_MAX_CLASSES], kx_last[KATSU_F16_MAX_CLASSES];
     int lower_h, first_x, most_rel_x, most_taps;
+    int span_h, span_x;  // rows and columns of g that the pixels (s jy + py, s jx + px) of one (jy, jx) receive from
     size_t grid_h, grid_w, left, right;  // zero pixels that g's rows need on either side
 };
 
@@ -130,7 +131,10 @@ Classes classes_of(const Shape &g) {
         }
     }
     q.row_begin[st] = rows;
-    for (int i = 0; i < rows; ++i) q.off_h[i] = (short)(q.off_h[i] - q.lower_h);
+    for (int i = 0; i < rows; ++i) {
+        q.off_h[i] = (short)(q.off_h[i] - q.lower_h);
+        if (q.off_h[i] >= q.span_h) q.span_h = q.off_h[i] + 1;
+    }
     q.first_x = 0x7fff;
     int last_x = -0x7fff;
     for (int px = 0; px < st; ++px) {
@@ -151,6 +155,7 @@ Classes classes_of(const Shape &g) {
         if (q.taps_x[px] == 0) q.off_x[px] = q.first_x;
         if (q.off_x[px] - q.first_x > q.most_rel_x) q.most_rel_x = q.off_x[px] - q.first_x;
     }
+    q.span_x = last_x - q.first_x + 1;
     q.left = q.first_x < 0 ? (size_t)-q.first_x : 0;
     const int right = (int)q.grid_w - 1 + last_x - (int)(g.ow - 1);
     q.right = right > 0 ? (size_t)right : 0;
@@ -313,20 +318,32 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     KatsuF16Problem pd = {};
     const KatsuF16Box box_dx = katsu_f16_box(128, false, 1, q.grid_w, q.grid_h, n);
     pixel_fields(&pd, g, box_dx);
+    // At stride 2 the pixels of an x-parity pair are stored together (store_pairs).  With few input channels all four classes
+    // are columns of one contraction over the span_h x span_x pixels of g they receive from, with zero weights where a class
+    // has no tap: those pixels are then loaded once and not once per class and tap, and a tile is one pass of the pipeline
+    // instead of four short ones.  The zeros cost the tensor pipe (16 tap products for 9 at 3 x 3), so the line is where the
+    // columns of all classes fit 128, whose products take no longer than their operands' fill: 32 channels.  With more, the
+    // two classes of a pair run one after the other on tiles of at most 128 columns and the sums of both are held.
+    const size_t class_cols = 2 * katsu_round_up(c, 16);
+    const bool merged = stride == 2 && class_cols <= 64;
     int width = 0;
-    for (size_t i = 0; i < stride; ++i) {
-        const int cols = q.taps_x[i] * (int)kp;
+    for (size_t i = 0; i < (merged ? 1 : stride); ++i) {
+        const int cols = (merged ? q.span_x : q.taps_x[i]) * (int)kp;
         pd.b_col[i] = width;
         pd.chunks[i] = (short)((cols + 63) / 64);
         pd.steps_last[i] = (short)((cols - 64 * (pd.chunks[i] - 1) + 15) / 16);
-        pd.off_w[i] = (short)(q.off_x[i] - q.first_x);
+        pd.off_w[i] = merged ? 0 : (short)(q.off_x[i] - q.first_x);
         width += pd.chunks[i] * 64;
     }
     long long kb_dx = 0;
-    for (size_t py = 0; py < stride; ++py)
-        for (size_t px = 0; px < stride; ++px) kb_dx += (long long)(q.row_begin[py + 1] - q.row_begin[py]) * pd.chunks[px];
+    if (merged) kb_dx = (long long)q.span_h * pd.chunks[0];
+    else
+        for (size_t py = 0; py < stride; ++py)
+            for (size_t px = 0; px < stride; ++px) kb_dx += (long long)(q.row_begin[py + 1] - q.row_begin[py]) * pd.chunks[px];
+    const size_t dx_columns = merged ? 2 * class_cols : c, dx_planes = merged ? (size_t)q.span_h : r;
     const size_t dx_count = n * c * h * wd;
-    const KatsuF16Plan plan_dx = katsu_f16_plan(ctx, KATSU_F16_CONV, box_dx.blocks * 128, (int)c, kb_dx, double(dx_count));
+    const KatsuF16Plan plan_dx = katsu_f16_plan(ctx, KATSU_F16_CONV, box_dx.blocks * 128, (int)dx_columns, kb_dx, double(dx_count),
+                                                stride == 2 ? 128 : 256);
     // dW
     const size_t gpr = katsu_div_up(s * cp, (size_t)64), dw_lanes = r * gpr * 64, dw_count = dw_lanes * k;
     const KatsuF16Box box_dw = katsu_f16_box(64, true, (int)stride, ow, oh, n);
@@ -343,15 +360,15 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         }
         void *gs = arena.take(staged_bytes(ctx, n, k, oh, ow, gap, tail));
         void *xs = dw ? arena.take(staged_bytes(ctx, n, c, h, wd, pad, 0)) : nullptr;
-        const KatsuF16Planes ws = dx ? arena.planes(r * c * width, planes) : KatsuF16Planes{nullptr, 0};
+        const KatsuF16Planes ws = dx ? arena.planes(dx_planes * dx_columns * width, planes) : KatsuF16Planes{nullptr, 0};
         float *partial_dx = dx && plan_dx.splits > 1 ? arena.floats(size_t(plan_dx.splits) * dx_count) : nullptr;
         float *partial_dw = dw ? arena.floats(size_t(plan_dw.splits) * dw_count) : nullptr;
         if (!pass) continue;
         const Staged sg = staged_at(gs, n, k, oh, ow, gap, tail), own = staged_at(xs, n, c, h, wd, pad, 0);
         KatsuF16Maps md, mw;
-        if (dx && (!katsu_f16_window_maps(md.a, sg.planes, q.first_x * (long long)kp, planes, size_t(q.most_taps) * kp,
-                                          q.grid_w + q.most_rel_x, oh, n, kp, sg.row(), sg.image(), 1, 64, box_dx) ||
-                   !katsu_f16_rows_maps(md.b, ws, planes, width, c, r, width, c * width, plan_dx.bn / 2)))
+        if (dx && (!katsu_f16_window_maps(md.a, sg.planes, q.first_x * (long long)kp, planes,
+                                          size_t(merged ? q.span_x : q.most_taps) * kp, q.grid_w + (merged ? 0 : q.most_rel_x), oh, n, kp, sg.row(), sg.image(), 1, 64, box_dx) ||
+                   !katsu_f16_rows_maps(md.b, ws, planes, width, dx_columns, dx_planes, width, dx_columns * width, plan_dx.bn / 2)))
             return katsu_f16_drop_call(ctx);
         if (dw && (!x_window_maps(ctx, mw.a, prestaged ? held : own, g, box_dw) ||
                    (prestaged && !x_window_maps(ctx, mw.a_second, own, g, box_dw)) ||
@@ -374,9 +391,13 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             amax[na++] = {w, k * c * r * s, iw};
             KatsuStageJob &jw = jobs[nj++];
             jw = weights_job(w, ws, g, kp, width, iw);
-            jw.backward = 1;
+            jw.backward = merged ? 2 : 1;
             jw.classes = jw.stride = (int)stride;
-            for (size_t i = 0; i < stride; ++i) {
+            jw.class_cols = (int)class_cols;
+            jw.span_h = q.span_h; jw.span_x = q.span_x;
+            jw.lower_h = q.lower_h; jw.first_x = q.first_x;
+            jw.pad = (int)pad;
+            for (size_t i = 0; i < (merged ? 0 : stride); ++i) {
                 jw.col_begin[i] = pd.b_col[i];
                 jw.kx_last[i] = q.kx_last[i];
                 jw.class_taps[i] = q.taps_x[i];
@@ -396,11 +417,19 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.m_total = box_dx.blocks * 128;
             p.n_total = (int)c;
             p.col_stride = (long long)(h * wd);
-            p.classes_y = p.classes_x = p.step = (int)stride;
-            for (size_t i = 0; i <= stride; ++i) p.row_begin[i] = q.row_begin[i];
-            for (int i = 0; i < q.row_begin[stride]; ++i) {
-                p.off_h[i] = q.off_h[i];
-                p.b_row[i] = q.ky[i];
+            p.step = (int)stride;
+            if (merged) {
+                p.class_cols = (int)class_cols;
+                p.row_begin[1] = q.span_h;
+                for (int i = 0; i < q.span_h; ++i) p.off_h[i] = p.b_row[i] = (short)i;
+            } else {
+                p.classes_y = p.classes_x = (int)stride;
+                p.pair_x = stride == 2 ? 1 : 0;
+                for (size_t i = 0; i <= stride; ++i) p.row_begin[i] = q.row_begin[i];
+                for (int i = 0; i < q.row_begin[stride]; ++i) {
+                    p.off_h[i] = q.off_h[i];
+                    p.b_row[i] = q.ky[i];
+                }
             }
             p.in_step = 1;
             p.lower_h = q.lower_h;

@@ -135,6 +135,34 @@ __device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d
     }
 }
 
+// The two neighbouring pixels of a stride-2 parity pair, for N channels from the one at `d` on: one 8-byte store where the
+// result allows it.  Stored class by class, every 32-byte sector of dX went out half full twice, and these stores were
+// half of the kernel's time (128 x 128 x 112 x 112: 981 us, 516 without them).
+template <int N, int STEP>
+__device__ __forceinline__ void store_pairs(const KatsuF16Problem &p, float *d, bool ok0, bool ok1, int live, const float *a,
+                                            const float *b, float factor) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (i < live) {
+            float2 v = make_float2(a[i * STEP] * factor, b[i * STEP] * factor);
+            if (p.pair_vec) {
+                if (ok0) {
+                    if (p.accumulate) {
+                        const float2 old = *reinterpret_cast<const float2 *>(d);
+                        v.x += old.x;
+                        v.y += old.y;
+                    }
+                    *reinterpret_cast<float2 *>(d) = v;
+                }
+            } else {
+                if (ok0) d[0] = p.accumulate ? d[0] + v.x : v.x;
+                if (ok1) d[1] = p.accumulate ? d[1] + v.y : v.y;
+            }
+        }
+        d += p.col_stride;
+    }
+}
+
 template <int NARROW, KatsuF16Kind KIND>
 __global__ void __launch_bounds__(THREADS, 1)
 f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant__ KatsuF16Problem p) {
@@ -357,18 +385,35 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                 img += q2;
                 in_box = q2 < p.nb && img < p.n_img;
             }
+            const bool pairs_of_x = KIND == KATSU_F16_CONV && p.pair_x;
+            float run[4][32];  // sums of the drains; of pairs: [0, 1], and in [2, 3] those of the class px = 0 before
             for (int py = 0; py < p.classes_y && alive; ++py)
                 for (int px = 0; px < p.classes_x && alive; ++px) {
                     int kb0, kb1;
                     k_range(p, class_kblocks<KIND>(p, py, px), t.split, &kb0, &kb1);
-                    bool valid = in_box && m < p.m_total;
+                    const bool in_result = in_box && m < p.m_total;
+                    bool valid = in_result;
                     long long at = m;
+                    int y = 0, x = 0;
                     if (KIND == KATSU_F16_CONV) {
-                        const int y = p.step * jy + py, x = p.step * jx + px;
+                        y = p.step * jy + py, x = p.step * jx + px;
                         valid = valid && y < p.out_h && x < p.out_w;
                         at = img * p.img_stride + (long long)y * p.out_w + x;
                     }
-                    float *dst = p.out + t.split * p.split_stride + at + n0 * p.col_stride;
+                    float *dst = p.out + t.split * p.split_stride + at;
+                    // columns n0 + c0 .. + 31 of this lane
+                    auto put = [&](int c0, const float (&v)[32], float bias) {
+                        const int col = n0 + c0;
+                        if (KIND == KATSU_F16_CONV && p.class_cols) {
+                            // (a last column tile may reach past the classes)
+                            const int q = col / p.class_cols, channel = (col - q * p.class_cols) >> 1;
+                            const bool ok = in_result && q < 2 && y + q < p.out_h && x < p.out_w;
+                            store_pairs<16, 2>(p, dst + q * p.out_w + channel * p.col_stride, ok, ok && x + 1 < p.out_w,
+                                               p.n_total - channel, v, v + 1, factor);
+                        } else {
+                            store_columns(p, dst + col * p.col_stride, valid, col, v, factor, bias);
+                        }
+                    };
                     auto bias_of = [&](int c0) {
                         const int col = n0 + c0 + lane;
                         return p.bias && col < p.n_total ? __ldg(p.bias + col) : 0.f;
@@ -386,7 +431,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             else mbar_arrive_cluster(map_to_rank(&acc_empty[b], 0));
                         }
                     };
-                    if (kb1 - kb0 <= drain) {
+                    if (!pairs_of_x && kb1 - kb0 <= drain) {
                         // one accumulator holds it all: 32 columns at a time, no sums in registers
                         float bias[4];
 #pragma unroll
@@ -404,7 +449,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) v[i] = 0.f;
                             }
-                            store_columns(p, dst + c0 * p.col_stride, valid, n0 + c0, v, factor, bias[c]);
+                            put(c0, v, bias[c]);
                         }
                         if (kb1 > kb0) {
                             release_acc(q & 1);
@@ -412,11 +457,17 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         }
                         continue;
                     }
-                    float run[4][32];
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) run[c][i] = 0.f;
+                        for (int i = 0; i < 32; ++i) {
+                            if (c < 2) {
+                                if (pairs_of_x) run[2 + c][i] = run[c][i];
+                                run[c][i] = 0.f;
+                            } else if (!pairs_of_x) {
+                                run[c][i] = 0.f;
+                            }
+                        }
                     for (int kb = kb0; kb < kb1; kb += drain, ++q) {
                         const uint32_t acc = wait_acc(q & 1);
                         if (!alive) break;
@@ -432,10 +483,22 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         release_acc(q & 1);
                     }
                     if (!alive) break;
+                    if (pairs_of_x) {
+                        if (px == 0) continue;
+                        const bool ok = in_result && y < p.out_h && x - 1 < p.out_w;
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const int c0 = (2 * c + group) * 32;
+                            if (c0 < p.bn)
+                                store_pairs<32, 1>(p, dst - 1 + (n0 + c0) * p.col_stride, ok, valid, p.n_total - n0 - c0, run[2 + c],
+                                                   run[c], factor);
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int c0 = (2 * c + group) * 32;
-                        if (c0 < p.bn) store_columns(p, dst + c0 * p.col_stride, valid, n0 + c0, run[c], factor, bias_of(c0));
+                        if (c0 < p.bn) put(c0, run[c], bias_of(c0));
                     }
                 }
         }
@@ -475,13 +538,13 @@ int32_t launch(katsu_cuda_ctx *ctx, const KatsuF16Maps &maps, const KatsuF16Prob
 // passes * 4 * bn / 2 clocks and the fill of (128 + bn / 2) * 128 bytes per part at about 60 bytes a clock; an item costs
 // its pipeline start and its stores besides; splits pay for writing and folding their slabs.
 KatsuF16Plan katsu_f16_plan(const katsu_cuda_ctx *ctx, KatsuF16Kind kind, long long m_total, int n_total,
-                            long long kblocks, double out_floats) {
+                            long long kblocks, double out_floats, int most_bn) {
     const int parts = ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1, passes = parts == 2 ? 3 : 1;
     const double pairs = ctx->num_sms / 2;
     const long long m_tiles = (m_total + 2 * BM - 1) / (2 * BM);
     KatsuF16Plan best = {0, 1};
     double best_cost = 0;
-    for (int bn = 32; bn <= 256; bn += 32) {
+    for (int bn = 32; bn <= most_bn; bn += 32) {
         if (kind == KATSU_F16_CONV_DW && bn != 64 && bn != 128 && bn != 256) continue;
         const long long tiles = m_tiles * ((n_total + bn - 1) / bn);
         const double pipe = passes * 4 * bn / 2.0, fill = (BM + bn / 2) * 128.0 * parts / 60.0;
@@ -515,7 +578,7 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
     p.bn = plan.bn;
     p.splits = plan.splits;
     p.m_tiles = (int)((p.m_total + 2 * BM - 1) / (2 * BM));
-    p.n_tiles = (p.n_total + plan.bn - 1) / plan.bn;
+    p.n_tiles = ((p.class_cols ? 2 * p.class_cols : p.n_total) + plan.bn - 1) / plan.bn;
     long long most = 0;  // k-blocks of the longest class
     if (kind == KATSU_F16_CONV_DW) {
         most = p.blocks;
@@ -538,6 +601,7 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
         p.bias = nullptr;
         p.relu = 0;
     }
+    p.pair_vec = p.out_w % 2 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 7) == 0;
     p.status = ctx->status;
     const long long items = (long long)p.m_tiles * p.n_tiles * p.splits;
     if (items > 0x3fffffff) return katsu_set_error(KATSU_ERR_UNSUPPORTED, "too many tiles");

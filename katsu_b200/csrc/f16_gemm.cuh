@@ -44,6 +44,9 @@ struct KatsuF16Problem {
     long long blocks;
     int in_step, lower_h;
     int out_h, out_w, step;
+    // CONV with step 2.  class_cols, if not 0: one contraction for all four parity classes, columns (py, channel, px),
+    // class_cols to a py.  Else pair_x: the classes px = 0 and 1 are stored together (bn <= 128).  pair_vec: as float2.
+    int class_cols, pair_x, pair_vec;
     long long img_stride;
     // ---- dW: lanes are 64-wide column groups, groups_per_row to a filter row
     int groups, groups_per_row;
@@ -64,7 +67,7 @@ struct KatsuF16Plan {
     int bn, splits;
 };
 KatsuF16Plan katsu_f16_plan(const katsu_cuda_ctx *ctx, KatsuF16Kind kind, long long m_total, int n_total,
-                            long long kblocks, double out_floats);
+                            long long kblocks, double out_floats, int most_bn = 256);
 
 // Starts the kernel; with plan.splits > 1 the results go to `partial` (splits slabs of split_stride floats in the
 // layout of `out`) and the caller folds them.

@@ -80,7 +80,9 @@ struct KatsuF16Planes {
 //   ROWS     src [n][c] -> [n][cp]
 //   WEIGHTS  src [k][c][r][s] -> [r][rows][width]; backward = 0: rows are k and column kx * cp + c is tap kx;
 //            backward = 1: rows are c and the columns of x-parity class j start at col_begin[j], tap t of the class
-//            (kx = kx_last[j] - t * stride) holding cp columns, channel k innermost.
+//            (kx = kx_last[j] - t * stride) holding cp columns, channel k innermost;
+//            backward = 2 (stride 2): -> [span_h][(py, c, px)][width], class_cols rows to a py, column t * cp + k of a row in
+//            plane dy is tap (py + pad - 2 * (lower_h + dy), px + pad - 2 * (first_x + t)), zero where there is no such tap.
 struct KatsuStageJob {
     int kind;
     const float *src;
@@ -91,6 +93,7 @@ struct KatsuStageJob {
     int n, c, h, w, gap, cp, tail;
     int k, r, s, width, backward, classes, stride;
     int col_begin[8], kx_last[8], class_taps[8];
+    int class_cols, span_h, span_x, pad, lower_h, first_x;  // backward = 2
 };
 
 // Largest magnitude and usability of up to three operands, one launch.

@@ -312,19 +312,33 @@ __device__ void stage_rows(const KatsuStageJob &j, const Writer &out, unsigned b
     }
 }
 
+// Rows and planes of staged weights.
+__host__ __device__ inline int weight_rows(const KatsuStageJob &j) {
+    return j.backward == 2 ? 2 * j.class_cols : j.backward ? j.c : j.k;
+}
+__host__ __device__ inline int weight_planes(const KatsuStageJob &j) { return j.backward == 2 ? j.span_h : j.r; }
+
 // Eight columns of one weight row to a thread; cp and every class's first column are multiples of 8.
 __device__ void stage_weights(const KatsuStageJob &j, const Writer &out, unsigned block, unsigned blocks) {
-    const int rows = j.backward ? j.c : j.k, inner = j.backward ? j.k : j.c;
+    const int rows = weight_rows(j), inner = j.backward ? j.k : j.c;
     const unsigned eights = j.width / 8, taps = j.r * j.s;
-    const size_t total = size_t(j.r) * rows * eights;
+    const size_t total = size_t(weight_planes(j)) * rows * eights;
     const size_t step = j.backward ? size_t(j.c) * taps : taps;  // between channels of the contraction
     for (size_t i = size_t(block) * THREADS + threadIdx.x; i < total; i += size_t(blocks) * THREADS) {
         const int col = int(i % eights) * 8;
         const size_t rest = i / eights;
-        const int row = int(rest % rows), ky = int(rest / rows);
+        int row = int(rest % rows), ky = int(rest / rows);
         int kx, ch;
         bool live;
-        if (j.backward) {
+        if (j.backward == 2) {
+            const int py = row / j.class_cols, px = row & 1, t = col / j.cp;
+            row = (row - py * j.class_cols) >> 1;
+            ch = col - t * j.cp;
+            ky = py + j.pad - 2 * (j.lower_h + ky);
+            kx = px + j.pad - 2 * (j.first_x + t);
+            live = row < j.c && t < j.span_x && ky >= 0 && ky < j.r && kx >= 0 && kx < j.s;
+            if (!live) ky = kx = row = 0;
+        } else if (j.backward) {
             int q = 0;
             while (q + 1 < j.classes && col >= j.col_begin[q + 1]) ++q;
             const int t = (col - j.col_begin[q]) / j.cp;
@@ -449,7 +463,7 @@ int32_t katsu_f16_stage(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Kat
         } else {
             const size_t units = j.kind == KATSU_STAGE_NHWC ? size_t(j.n) * hw * (j.cp / 8)
                                  : j.kind == KATSU_STAGE_ROWS ? size_t(j.n) * (j.cp / 8)
-                                                              : size_t(j.r) * (j.backward ? j.c : j.k) * (j.width / 8);
+                                                              : size_t(weight_planes(j)) * weight_rows(j) * (j.width / 8);
             blocks = katsu_div_up(units, (size_t)THREADS);
             if (blocks > size_t(ctx->num_sms) * 64) blocks = size_t(ctx->num_sms) * 64;
         }

@@ -56,6 +56,36 @@ def test_convolution_edges(ctx, oracle, shape):
         assert max(errors) <= bar, (shape, mode, errors)
 
 
+# Strides: dX of all four parity classes in one contraction (at most 32 channels at stride 2) and just past that line, x pairs
+# stored together and, with odd widths, apart; filters that leave a class without taps, that are not square, that reach over
+# several pixels of g; images whose rows the forward pass takes as two dimensions (height a multiple of the stride) and not;
+# dW with one and with two column groups to a load.
+STRIDED = [(3, 32, 15, 18, 40, 3, 3, 2, 1), (2, 17, 16, 16, 24, 1, 1, 2, 0), (2, 33, 16, 18, 40, 3, 3, 2, 1), (3, 20, 16, 13, 130, 5, 3, 2, 2),
+           (2, 4, 18, 30, 20, 7, 7, 2, 3), (5, 12, 2, 40, 24, 3, 3, 2, 1), (2, 140, 14, 11, 24, 3, 3, 2, 1), (2, 24, 18, 21, 40, 3, 3, 3, 1),
+           (2, 40, 15, 11, 24, 4, 4, 3, 2), (2, 128, 12, 10, 192, 3, 3, 2, 1)]
+
+
+@pytest.mark.parametrize("shape", STRIDED, ids=lambda s: "x".join(map(str, s)))
+def test_strided_edges(ctx, oracle, shape):
+    """Both modes, and dX added to what is there."""
+    n, c, h, w, k, r, s, stride, pad = shape
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    rng = np.random.default_rng(sum(shape))
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, n * k * oh * ow))
+    before = rng.standard_normal(x.size).astype(np.float32)
+    dx64 = oracle.conv2d_backward_f64(x, wt, g, [n, c, h, w], [k, c, r, s], stride, pad)[0].reshape(-1) + before
+    for mode, bar in BARS:
+        ctx.set_precision(mode)
+        try:
+            errors = conv_errors(ctx, oracle, shape, x, wt, g)
+            with DeviceArrays(ctx, x=x, w=wt, g=g, dx=before) as d:
+                ctx.conv2d_bwd(d["x"], d["w"], d["g"], d["dx"], None, *shape, accumulate=1)
+                errors.append(rel_l2(d.get("dx"), dx64))
+        finally:
+            ctx.set_precision(0)
+        assert max(errors) <= bar, (shape, mode, errors)
+
+
 # more tiles of 64 x 64 or 32 channels x 128 pixels than staging blocks run at a time (5 to an SM; one to an SM for the copy
 # of x beside the caller's), pixels a multiple of 4 and not
 @pytest.mark.parametrize("shape", [(12, 70, 47, 45, 24, 1, 1, 1, 0), (12, 70, 48, 45, 24, 1, 1, 1, 0), (48, 28, 47, 45, 24, 1, 1, 1, 0)],
