@@ -95,9 +95,10 @@ bool held_x(const katsu_cuda_ctx *ctx, const Shape &g, const KatsuF16Info **info
 }
 
 // x as the window operand of forward and dW.
-bool x_window_maps(const katsu_cuda_ctx *ctx, CUtensorMap *maps, const Staged &x, const Shape &g, const KatsuF16Box &box) {
+bool x_window_maps(const katsu_cuda_ctx *ctx, CUtensorMap *maps, const Staged &x, const Shape &g, const KatsuF16Box &box,
+                   bool pairs) {
     return katsu_f16_window_maps(maps, x.planes, -(long long)(g.pad * x.cp), katsu_f16_narrow_planes(ctx) + 1, g.s * x.cp, g.ow,
-                                 g.h, g.n, g.stride * x.cp, x.row(), x.image(), (int)g.stride, 64, box);
+                                 g.h, g.n, g.stride * x.cp, x.row(), x.image(), (int)g.stride, 64, box, pairs);
 }
 
 // The taps of dX by parity class.
@@ -226,8 +227,8 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         if (!pass) continue;
         const Staged own = staged_at(xs, n, c, h, wd, pad, 0);
         KatsuF16Maps maps;
-        if (!x_window_maps(ctx, maps.a, prestaged ? held : own, g, box) ||
-            (prestaged && !x_window_maps(ctx, maps.a_second, own, g, box)) ||
+        if (!x_window_maps(ctx, maps.a, prestaged ? held : own, g, box, false) ||
+            (prestaged && !x_window_maps(ctx, maps.a_second, own, g, box, false)) ||
             !katsu_f16_rows_maps(maps.b, ws, planes, width, k, r, width, k * width, plan.bn / 2))
             return katsu_f16_drop_call(ctx);
         *handled = 1;
@@ -351,6 +352,11 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     if (box_dx.blocks > 0x7fffffff || box_dw.blocks > 0x7fffffff) return katsu_f16_drop_call(ctx);
     const KatsuF16Plan plan_dw = katsu_f16_plan(ctx, KATSU_F16_CONV_DW, (long long)dw_lanes, (int)k, kb_dw, double(dw_count));
 
+    // dW: two 64-column groups to a load, where no pair of groups holds padding or parts of two filter rows.  A load costs the
+    // copy unit about 150 clocks whatever it brings, and with four to a k-block of 512 pipe clocks they set the pace in TF32
+    // mode (256 x 256 channels, 128 x 56 x 56: 623 -> 449 us).
+    const bool a_pairs = (s * cp) % 128 == 0, b_pairs = plan_dw.bn == 256 && kp % 64 == 0;
+
     KatsuArena arena = {nullptr, 0};
     for (int pass = 0; pass < 2; ++pass) {
         if (pass) {
@@ -370,10 +376,10 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
                                           size_t(merged ? q.span_x : q.most_taps) * kp, q.grid_w + (merged ? 0 : q.most_rel_x), oh, n, kp, sg.row(), sg.image(), 1, 64, box_dx) ||
                    !katsu_f16_rows_maps(md.b, ws, planes, width, dx_columns, dx_planes, width, dx_columns * width, plan_dx.bn / 2)))
             return katsu_f16_drop_call(ctx);
-        if (dw && (!x_window_maps(ctx, mw.a, prestaged ? held : own, g, box_dw) ||
-                   (prestaged && !x_window_maps(ctx, mw.a_second, own, g, box_dw)) ||
+        if (dw && (!x_window_maps(ctx, mw.a, prestaged ? held : own, g, box_dw, a_pairs) ||
+                   (prestaged && !x_window_maps(ctx, mw.a_second, own, g, box_dw, a_pairs)) ||
                    !katsu_f16_window_maps(mw.b, sg.planes, 0, planes, kp, ow, oh, n, kp, sg.row(), sg.image(), 1,
-                                          plan_dw.bn >= 128 ? 64 : 32, box_dw)))
+                                          plan_dw.bn >= 128 ? 64 : 32, box_dw, b_pairs)))
             return katsu_f16_drop_call(ctx);
         *handled = 1;
         const KatsuF16Call call = katsu_f16_call(ctx, ig, dx ? iw : nullptr, dw ? info : nullptr);
@@ -456,6 +462,8 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.lower_h = -(int)pad;
             p.groups = (int)(r * gpr);
             p.groups_per_row = (int)gpr;
+            p.a_pairs = a_pairs;
+            p.b_pairs = b_pairs;
             KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_CONV_DW, mw, p, plan_dw, partial_dw, (long long)dw_count));
             KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)f16_dw_fold_kernel, 0));
             KATSU_TRY(katsu_launch_chained(ctx, f16_dw_fold_kernel, (unsigned)katsu_div_up(dw_count, (size_t)32), 256, 0, 1,

@@ -258,19 +258,32 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             int n, oy, ox;
                             box_origin(p, i, &n, &oy, &ox);
                             const int per_load = half >= 64 ? 64 : 32;
+                            const int first = (2 * t.mt + int(rank)) * 2;  // of this block's two column groups
                             for (int part = 0; part < planes; ++part) {
+                                if (p.a_pairs) {
+                                    const int ky = first / p.groups_per_row;
+                                    const bool live = first < p.groups;  // past the last one: an image that does not exist
+                                    tma_load_5d_pair(st + part * A_BYTES, map_a + part, bar, 0, ox,
+                                                     oy * p.in_step + p.lower_h + (live ? ky : 0), live ? n : p.n_img,
+                                                     live ? first - ky * p.groups_per_row : 0);
+                                } else {
 #pragma unroll
-                                for (int g = 0; g < 2; ++g) {
-                                    const int group = (2 * t.mt + int(rank)) * 2 + g;
-                                    const int ky = group / p.groups_per_row, j = group - ky * p.groups_per_row;
-                                    const bool live = group < p.groups;  // past the last one: an image that does not exist
-                                    tma_load_4d_pair(st + part * A_BYTES + g * (A_BYTES / 2), map_a + part, bar,
-                                                     live ? j * 64 : 0, ox, oy * p.in_step + p.lower_h + (live ? ky : 0),
-                                                     live ? n : p.n_img);
+                                    for (int g = 0; g < 2; ++g) {
+                                        const int group = first + g;
+                                        const int ky = group / p.groups_per_row, j = group - ky * p.groups_per_row;
+                                        const bool live = group < p.groups;
+                                        tma_load_4d_pair(st + part * A_BYTES + g * (A_BYTES / 2), map_a + part, bar,
+                                                         live ? j * 64 : 0, ox, oy * p.in_step + p.lower_h + (live ? ky : 0),
+                                                         live ? n : p.n_img);
+                                    }
                                 }
-                                for (int c = 0; c < half; c += per_load)
-                                    tma_load_4d_pair(st + b_off + part * b_bytes + c * BK * 2,
-                                                     map_b + part, bar, n0 + c, ox, oy, n);
+                                if (p.b_pairs) {
+                                    tma_load_5d_pair(st + b_off + part * b_bytes, map_b + part, bar, 0, ox, oy, n, n0 >> 6);
+                                } else {
+                                    for (int c = 0; c < half; c += per_load)
+                                        tma_load_4d_pair(st + b_off + part * b_bytes + c * BK * 2,
+                                                         map_b + part, bar, n0 + c, ox, oy, n);
+                                }
                             }
                         }
                         if (++s == stages) {
@@ -642,15 +655,15 @@ bool katsu_f16_rows_maps(CUtensorMap *maps, const KatsuF16Planes &planes, int co
 
 bool katsu_f16_window_maps(CUtensorMap *maps, const KatsuF16Planes &planes, long long offset, int count, size_t channels,
                            size_t width, size_t height, size_t images, size_t w_pitch, size_t h_pitch, size_t n_pitch,
-                           int step_h, int box_channels, const KatsuF16Box &box) {
+                           int step_h, int box_channels, const KatsuF16Box &box, bool pairs) {
     katsu_tensor_map_encode_fn encode = katsu_tensor_map_encoder();
     if (encode == nullptr) return false;
-    cuuint64_t dims[4] = {channels, width, height, images};
-    cuuint64_t strides[3] = {w_pitch * 2, h_pitch * 2, n_pitch * 2};
-    cuuint32_t gbox[4] = {(cuuint32_t)box_channels, (cuuint32_t)box.bw, (cuuint32_t)((box.bh - 1) * step_h + 1), (cuuint32_t)box.nb};
-    cuuint32_t estr[4] = {1, 1, (cuuint32_t)step_h, 1};
+    cuuint64_t dims[5] = {pairs ? 64 : channels, width, height, images, channels / 64};
+    cuuint64_t strides[4] = {w_pitch * 2, h_pitch * 2, n_pitch * 2, 128};
+    cuuint32_t gbox[5] = {(cuuint32_t)box_channels, (cuuint32_t)box.bw, (cuuint32_t)((box.bh - 1) * step_h + 1), (cuuint32_t)box.nb, 2};
+    cuuint32_t estr[5] = {1, 1, (cuuint32_t)step_h, 1, 1};
     for (int i = 0; i < count; ++i)
-        if (encode(maps + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, planes.base + offset + i * (long long)planes.stride, dims, strides,
+        if (encode(maps + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, pairs ? 5 : 4, planes.base + offset + i * (long long)planes.stride, dims, strides,
                    gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    box_channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)

@@ -50,6 +50,7 @@ struct KatsuF16Problem {
     long long img_stride;
     // ---- dW: lanes are 64-wide column groups, groups_per_row to a filter row
     int groups, groups_per_row;
+    int a_pairs, b_pairs;  // the maps are of the `pairs` form: one load brings two column groups
     int a_bytes;  // bytes of one loaded A part of a k-block
     // filled in by the launcher
     int bn, m_tiles, n_tiles, splits, kb_per_split;
@@ -90,9 +91,10 @@ KatsuF16Box katsu_f16_box(int lanes, bool exact, int step_h, size_t width, size_
 // Tensor maps over fp16 planes.  rows_map: [d2][rows][cols] with pitches in elements, box 64 x box_rows x 1, 128-byte
 // swizzle.  window_map: {channels, width, height, images} with pitches in elements, box of box_channels x a pixel box whose
 // rows are step_h apart.
-// One map per plane.
+// One map per plane.  `pairs` (channels a multiple of 64): the groups of 64 channels are a fifth dimension and a box holds
+// two of them, one behind the other.
 bool katsu_f16_rows_maps(CUtensorMap *maps, const KatsuF16Planes &planes, int count, size_t cols, size_t rows, size_t d2, size_t row_pitch,
                         size_t d2_pitch, int box_rows);
 bool katsu_f16_window_maps(CUtensorMap *maps, const KatsuF16Planes &planes, long long offset, int count, size_t channels, size_t width, size_t height,
                           size_t images, size_t w_pitch, size_t h_pitch, size_t n_pitch, int step_h, int box_channels,
-                          const KatsuF16Box &box);
+                          const KatsuF16Box &box, bool pairs = false);

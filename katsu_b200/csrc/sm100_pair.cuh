@@ -115,4 +115,13 @@ __device__ __forceinline__ void tma_load_4d_pair(void *smem_dst, const CUtensorM
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_addr, int c0, int c1,
+                                                 int c2, int c3, int c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], "
+        "[%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+        : "memory");
+}
+
 }  // namespace sm100
