@@ -441,7 +441,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.lower_h = q.lower_h;
             p.out_h = (int)h; p.out_w = (int)wd;
             p.img_stride = (long long)(c * h * wd);
-            KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_CONV, md, p, plan_dx, partial_dx, (long long)dx_count));
+            KATSU_TRY(katsu_f16_launch(ctx, stride == 2 ? KATSU_F16_CONV_DX2 : KATSU_F16_CONV, md, p, plan_dx, partial_dx, (long long)dx_count));
             if (plan_dx.splits > 1)
                 KATSU_TRY(katsu_f16_fold(ctx, partial_dx, dx, dx_count, plan_dx.splits, accumulate, nullptr, 1, 1, 0));
         }

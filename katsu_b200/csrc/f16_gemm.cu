@@ -166,7 +166,7 @@ __device__ __forceinline__ void store_pairs(const KatsuF16Problem &p, float *d, 
 template <int NARROW, KatsuF16Kind KIND>
 __global__ void __launch_bounds__(THREADS, 1)
 f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant__ KatsuF16Problem p) {
-    constexpr bool MN = KIND == KATSU_F16_CONV_DW;
+    constexpr bool MN = KIND == KATSU_F16_CONV_DW, CONV = KIND == KATSU_F16_CONV || KIND == KATSU_F16_CONV_DX2;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2];
@@ -221,7 +221,30 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
             const long long m0 = (2ll * t.mt + rank) * BM;
             const int n0 = t.nt * p.bn + int(rank) * half;
             int img = 0, jy = 0, jx = 0;  // CONV: first pixel of this block's lanes
-            if (KIND == KATSU_F16_CONV) box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
+            if (CONV) box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
+            // CONV_DW: this block's two column groups; past the last one an image that does not exist
+            int group_y[2] = {0, 0}, group_x[2] = {0, 0};
+            bool group_live[2] = {false, false};
+            if (MN) {
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    const int group = (2 * t.mt + int(rank)) * 2 + g;
+                    if (group >= p.groups) continue;
+                    group_live[g] = true;
+                    group_y[g] = group / p.groups_per_row;
+                    group_x[g] = group - group_y[g] * p.groups_per_row;
+                }
+            }
+            auto tma_a = [&](unsigned char *to, const CUtensorMap *map, uint32_t bar, int n, int y, int x) {
+                if (p.a_pairs) {
+                    tma_load_5d_pair(to, map, bar, 0, x, y + group_y[0], group_live[0] ? n : p.n_img, group_x[0]);
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 2; ++g)
+                        tma_load_4d_pair(to + g * (A_BYTES / 2), map, bar, group_x[g] * 64, x, y + group_y[g],
+                                         group_live[g] ? n : p.n_img);
+                }
+            };
             for (int py = 0; py < p.classes_y && ok; ++py)
                 for (int px = 0; px < p.classes_x && ok; ++px) {
                     int kb0, kb1;
@@ -243,7 +266,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                                 tma_load_3d_pair(st + part * A_BYTES, map_a + part, bar, i * BK, int(m0), 0);
                                 tma_load_3d_pair(st + b_off + part * b_bytes, map_b + part, bar, i * BK, n0, 0);
                             }
-                        } else if (KIND == KATSU_F16_CONV) {
+                        } else if (CONV) {
                             for (int part = 0; part < planes; ++part) {
                                 tma_load_4d_pair(st + part * A_BYTES, map_a + part, bar, chunk * BK, jx + p.off_w[px],
                                                  jy * p.in_step + p.lower_h + p.off_h[row], img);
@@ -258,25 +281,8 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             int n, oy, ox;
                             box_origin(p, i, &n, &oy, &ox);
                             const int per_load = half >= 64 ? 64 : 32;
-                            const int first = (2 * t.mt + int(rank)) * 2;  // of this block's two column groups
                             for (int part = 0; part < planes; ++part) {
-                                if (p.a_pairs) {
-                                    const int ky = first / p.groups_per_row;
-                                    const bool live = first < p.groups;  // past the last one: an image that does not exist
-                                    tma_load_5d_pair(st + part * A_BYTES, map_a + part, bar, 0, ox,
-                                                     oy * p.in_step + p.lower_h + (live ? ky : 0), live ? n : p.n_img,
-                                                     live ? first - ky * p.groups_per_row : 0);
-                                } else {
-#pragma unroll
-                                    for (int g = 0; g < 2; ++g) {
-                                        const int group = first + g;
-                                        const int ky = group / p.groups_per_row, j = group - ky * p.groups_per_row;
-                                        const bool live = group < p.groups;
-                                        tma_load_4d_pair(st + part * A_BYTES + g * (A_BYTES / 2), map_a + part, bar,
-                                                         live ? j * 64 : 0, ox, oy * p.in_step + p.lower_h + (live ? ky : 0),
-                                                         live ? n : p.n_img);
-                                    }
-                                }
+                                tma_a(st + part * A_BYTES, map_a + part, bar, n, oy * p.in_step + p.lower_h, ox);
                                 if (p.b_pairs) {
                                     tma_load_5d_pair(st + b_off + part * b_bytes, map_b + part, bar, 0, ox, oy, n, n0 >> 6);
                                 } else {
@@ -389,7 +395,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
             const int n0 = t.nt * p.bn;
             int img = 0, jy = 0, jx = 0;
             bool in_box = true;
-            if (KIND == KATSU_F16_CONV) {
+            if (CONV) {
                 const int r = quarter * 32 + lane;
                 box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
                 const int q1 = r / p.bw, q2 = q1 / p.bh;
@@ -398,7 +404,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                 img += q2;
                 in_box = q2 < p.nb && img < p.n_img;
             }
-            const bool pairs_of_x = KIND == KATSU_F16_CONV && p.pair_x;
+            const bool pairs_of_x = KIND == KATSU_F16_CONV_DX2 && p.pair_x;
             float run[4][32];  // sums of the drains; of pairs: [0, 1], and in [2, 3] those of the class px = 0 before
             for (int py = 0; py < p.classes_y && alive; ++py)
                 for (int px = 0; px < p.classes_x && alive; ++px) {
@@ -408,7 +414,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                     bool valid = in_result;
                     long long at = m;
                     int y = 0, x = 0;
-                    if (KIND == KATSU_F16_CONV) {
+                    if (CONV) {
                         y = p.step * jy + py, x = p.step * jx + px;
                         valid = valid && y < p.out_h && x < p.out_w;
                         at = img * p.img_stride + (long long)y * p.out_w + x;
@@ -417,7 +423,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                     // columns n0 + c0 .. + 31 of this lane
                     auto put = [&](int c0, const float (&v)[32], float bias) {
                         const int col = n0 + c0;
-                        if (KIND == KATSU_F16_CONV && p.class_cols) {
+                        if (KIND == KATSU_F16_CONV_DX2 && p.class_cols) {
                             // (a last column tile may reach past the classes)
                             const int q = col / p.class_cols, channel = (col - q * p.class_cols) >> 1;
                             const bool ok = in_result && q < 2 && y + q < p.out_h && x < p.out_w;
@@ -622,10 +628,12 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
     if (parts == 2) {
         if (kind == KATSU_F16_GEMM) return launch<2, KATSU_F16_GEMM>(ctx, maps, p, pairs);
         if (kind == KATSU_F16_CONV) return launch<2, KATSU_F16_CONV>(ctx, maps, p, pairs);
+        if (kind == KATSU_F16_CONV_DX2) return launch<2, KATSU_F16_CONV_DX2>(ctx, maps, p, pairs);
         return launch<2, KATSU_F16_CONV_DW>(ctx, maps, p, pairs);
     }
     if (kind == KATSU_F16_GEMM) return launch<1, KATSU_F16_GEMM>(ctx, maps, p, pairs);
     if (kind == KATSU_F16_CONV) return launch<1, KATSU_F16_CONV>(ctx, maps, p, pairs);
+    if (kind == KATSU_F16_CONV_DX2) return launch<1, KATSU_F16_CONV_DX2>(ctx, maps, p, pairs);
     return launch<1, KATSU_F16_CONV_DW>(ctx, maps, p, pairs);
 }
 

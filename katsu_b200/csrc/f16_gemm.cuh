@@ -11,6 +11,7 @@ constexpr int KATSU_F16_MAX_CLASSES = 8;  // parity classes per axis
 enum KatsuF16Kind {
     KATSU_F16_GEMM,     // A and B are K-major matrices
     KATSU_F16_CONV,     // A is a convolution window over a channels-innermost tensor (forward, dX), B taps x rows
+    KATSU_F16_CONV_DX2,  // CONV with the stores of dX at stride 2, whose code slows the others' epilogue
     KATSU_F16_CONV_DW,  // contraction over pixels, both operands MN-major
 };
 
@@ -44,7 +45,7 @@ struct KatsuF16Problem {
     long long blocks;
     int in_step, lower_h;
     int out_h, out_w, step;
-    // CONV with step 2.  class_cols, if not 0: one contraction for all four parity classes, columns (py, channel, px),
+    // CONV_DX2, step 2.  class_cols, if not 0: one contraction for all four parity classes, columns (py, channel, px),
     // class_cols to a py.  Else pair_x: the classes px = 0 and 1 are stored together (bn <= 128).  pair_vec: as float2.
     int class_cols, pair_x, pair_vec;
     long long img_stride;

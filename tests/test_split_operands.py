@@ -58,8 +58,7 @@ def test_convolution_edges(ctx, oracle, shape):
 
 # Strides: dX of all four parity classes in one contraction (at most 32 channels at stride 2) and just past that line, x pairs
 # stored together and, with odd widths, apart; filters that leave a class without taps, that are not square, that reach over
-# several pixels of g; images whose rows the forward pass takes as two dimensions (height a multiple of the stride) and not;
-# dW with one and with two column groups to a load.
+# several pixels of g; dW with one and with two column groups to a load.
 STRIDED = [(3, 32, 15, 18, 40, 3, 3, 2, 1), (2, 17, 16, 16, 24, 1, 1, 2, 0), (2, 33, 16, 18, 40, 3, 3, 2, 1), (3, 20, 16, 13, 130, 5, 3, 2, 2),
            (2, 4, 18, 30, 20, 7, 7, 2, 3), (5, 12, 2, 40, 24, 3, 3, 2, 1), (2, 140, 14, 11, 24, 3, 3, 2, 1), (2, 24, 18, 21, 40, 3, 3, 3, 1),
            (2, 40, 15, 11, 24, 4, 4, 3, 2), (2, 128, 12, 10, 192, 3, 3, 2, 1)]
