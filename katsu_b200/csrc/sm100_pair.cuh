@@ -44,33 +44,10 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t colum
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
 }
 
-// D[tmem of both blocks] (+)= A[tmem of both blocks] * B[halves in both blocks' shared memory]; issued by one
-// thread of the leader block for the pair.
-__device__ __forceinline__ void mma_tf32_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                                 bool accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n"
-        "}\n"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate ? 1u : 0u)
-        : "memory");
-}
-
 // Arrives on the barrier at shared-window address `addr` (this block's or the peer's) once every MMA issued so far
 // by this thread has completed.
 __device__ __forceinline__ void mma_commit_pair(uint32_t addr) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(addr) : "memory");
-}
-
-// This block's own tile into its own shared memory; the bytes are counted on the barrier at `bar_addr`, which
-// may belong to the pair's leader.
-__device__ __forceinline__ void tma_load_2d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_addr, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1)
-        : "memory");
 }
 
 __device__ __forceinline__ void tma_load_3d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_addr, int c0, int c1,
@@ -81,20 +58,9 @@ __device__ __forceinline__ void tma_load_3d_pair(void *smem_dst, const CUtensorM
         : "memory");
 }
 
-// D[tmem of both blocks] (+)= A[both blocks' shared memory, 128 rows each] * B[halves in both blocks' shared memory].
-__device__ __forceinline__ void mma_tf32_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                              bool accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n"
-        "}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate ? 1u : 0u)
-        : "memory");
-}
-
-// 16-bit operands (fp16, f32 accumulator), same operand layout as above: 2 SMs, 256 x N x 16 per instruction.
+// D[tmem of both blocks] (+)= A[both blocks' shared memory, 128 rows each] * B[halves in both blocks' shared memory], 16-bit
+// operands, f32 accumulator: 256 x N x 16 per instruction; issued by one thread of the leader block.  The TMA loads below bring
+// a block's own tile into its own shared memory; the bytes are counted on the barrier at `bar_addr`, which may be the leader's.
 __device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                              bool accumulate) {
     asm volatile(
