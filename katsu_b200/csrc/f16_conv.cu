@@ -31,9 +31,17 @@ bool geometry_ok(const katsu_cuda_ctx *ctx, const Shape &g) {
     return g.n * g.h * (g.w + gap) < 0x7fffffff && g.n * g.oh * (g.ow + gap) < 0x7fffffff && g.h * g.w < 0x3fffffff;
 }
 
-// Multiply-adds from which the passes in front pay against the direct kernels.
+// At least 16 channels on both sides, in multiples of 4.
+bool regular(const Shape &g) {
+    return g.c >= 16 && g.k >= 16 && g.c % 4 == 0 && g.k % 4 == 0 && g.n * g.oh * g.ow >= 64;
+}
+
+// Where the passes in front pay against the direct kernels.  The three launches take about 18 us whatever the size.  A direct
+// kernel's time is one thread's chain of c * r * s (dX: k * r * s) multiply-adds: at 16 channels and 3 x 3 already 39 us forward
+// and 45 us dX (16 x 8 x 8, 150 000 multiply-adds; 18.6 and 18.5 us here), so regular layers come here at any size.  Others
+// do from 1e6 multiply-adds on.
 bool worth_it(const Shape &g) {
-    return double(g.n) * g.oh * g.ow * double(g.k) * g.c * g.r * g.s >= 1e6;
+    return regular(g) || double(g.n) * g.oh * g.ow * double(g.k) * g.c * g.r * g.s >= 1e6;
 }
 
 // A staged tensor: its planes start at pixel (0, 0) of image 0; element pitches.

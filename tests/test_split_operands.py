@@ -163,3 +163,19 @@ def test_non_finite_values_reach_exactly_their_outputs(ctx, oracle, mode):
     finite = np.isfinite(y64)
     assert not finite.all() and np.array_equal(np.isfinite(y), finite)
     assert rel_l2(y[finite], y64[finite]) <= BARS[mode][1]
+
+
+@pytest.mark.parametrize("shape", [(1, 16, 8, 8, 16, 3, 3, 1, 1), (1, 16, 14, 14, 24, 3, 3, 1, 1), (2, 24, 13, 13, 32, 3, 3, 2, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_small_regular_layers_stay_on_the_tensor_cores(ctx, oracle, shape):
+    """Below 1e6 multiply-adds too: a direct kernel's chain of c * r * s multiply-adds takes two to three times as long."""
+    n, c, h, w, k, r, s, stride, pad = shape
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    rng = np.random.default_rng(sum(shape))
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, n * k * oh * ow))
+    with DeviceArrays(ctx, x=x, w=wt) as d:
+        d.alloc("y", g.size)
+        before = ctx.launch_count()
+        ctx.conv2d_fwd(d["x"], d["w"], d["y"], *shape)
+        assert ctx.launch_count() - before >= 3  # magnitudes, planes, product; a direct kernel is one launch
+    assert max(conv_errors(ctx, oracle, shape, x, wt, g)) <= REL_L2_TOL
