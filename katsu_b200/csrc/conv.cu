@@ -135,10 +135,7 @@ extern "C" int32_t katsu_cuda_conv2d_staged_floats(katsu_cuda_ctx *ctx, size_t n
     KATSU_TRY(geometry(c, h, wd, k, r, s, stride, pad, &g));
     *floats = 0;
     if (n == 0) return KATSU_OK;
-    // layers of at least 16 channels on both sides, in multiples of 4; others are staged inside the calls
-    if (c < 16 || k < 16 || (c & 3) != 0 || (k & 3) != 0 || n * g.oh * g.ow < 64 ||
-        !katsu_f16_conv_geometry(ctx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow))
-        return KATSU_OK;
+    if (!katsu_f16_conv_takes_copy(ctx, n, c, h, wd, k, r, s, stride, pad, g.oh, g.ow)) return KATSU_OK;
     // (never less than one or two f32 copies of x, what callers that size buffers by hand have been told)
     const size_t copy = n * c * h * wd * (ctx->precision == KATSU_MODE_3XTF32 ? 2 : 1);
     *floats = katsu_div_up(katsu_f16_conv_staged_bytes(ctx, n, c, h, wd), sizeof(float));

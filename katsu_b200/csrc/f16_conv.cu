@@ -44,6 +44,12 @@ bool worth_it(const Shape &g) {
     return regular(g) || double(g.n) * g.oh * g.ow * double(g.k) * g.c * g.r * g.s >= 1e6;
 }
 
+// Whether forward and dW read x through a copy that the caller holds: regular layers whose padding the gaps between the
+// copy's rows provide.
+bool takes_copy(const katsu_cuda_ctx *ctx, const Shape &g) {
+    return geometry_ok(ctx, g) && regular(g) && g.pad <= (size_t)STAGED_GAP;
+}
+
 // A staged tensor: its planes start at pixel (0, 0) of image 0; element pitches.
 struct Staged {
     KatsuF16Planes planes;
@@ -93,9 +99,10 @@ KatsuStageJob weights_job(const float *w, const KatsuF16Planes &to, const Shape 
     return j;
 }
 
-// The caller's staged copy of x; false when the call has none that fits.
+// The caller's staged copy of x.  False when the call has none, or is of a shape that uses none: what the pointer then
+// refers to was never written.
 bool held_x(const katsu_cuda_ctx *ctx, const Shape &g, const KatsuF16Info **info, Staged *out) {
-    if (ctx->x_prestaged == nullptr || g.pad > (size_t)STAGED_GAP) return false;
+    if (ctx->x_prestaged == nullptr || !takes_copy(ctx, g)) return false;
     char *base = const_cast<char *>(reinterpret_cast<const char *>(ctx->x_prestaged));
     *info = reinterpret_cast<const KatsuF16Info *>(base);
     *out = staged_at(base + STAGED_HEADER, g.n, g.c, g.h, g.w, STAGED_GAP, 0);
@@ -199,9 +206,9 @@ int32_t katsu_f16_conv_stage(katsu_cuda_ctx *ctx, const float *x, void *staged, 
     return katsu_f16_stage(ctx, katsu_f16_call(ctx, info, nullptr, nullptr), &job, 1);
 }
 
-bool katsu_f16_conv_geometry(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
-                             size_t s, size_t stride, size_t pad, size_t oh, size_t ow) {
-    return geometry_ok(ctx, Shape{n, c, h, w, k, r, s, stride, pad, oh, ow});
+bool katsu_f16_conv_takes_copy(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
+                               size_t s, size_t stride, size_t pad, size_t oh, size_t ow) {
+    return takes_copy(ctx, Shape{n, c, h, w, k, r, s, stride, pad, oh, ow});
 }
 
 int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, const float *bias, int relu, float *y,

@@ -140,8 +140,8 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
                              size_t m, size_t k, size_t n, int accumulate, int *handled);
 
 // The fp16 path of the convolutions (f16_conv.cu), *handled as above.
-bool katsu_f16_conv_geometry(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
-                             size_t s, size_t stride, size_t pad, size_t oh, size_t ow);
+bool katsu_f16_conv_takes_copy(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w, size_t k, size_t r,
+                               size_t s, size_t stride, size_t pad, size_t oh, size_t ow);
 size_t katsu_f16_conv_staged_bytes(const katsu_cuda_ctx *ctx, size_t n, size_t c, size_t h, size_t w);
 int32_t katsu_f16_conv_stage(katsu_cuda_ctx *ctx, const float *x, void *staged, size_t n, size_t c, size_t h, size_t w);
 int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, const float *bias, int relu, float *y,

@@ -45,6 +45,31 @@ def test_staged_calls_match_the_plain_calls_bit_for_bit(ctx, oracle, shape, mode
         ctx.set_precision(0)
 
 
+@pytest.mark.parametrize("shape", [(4, 64, 14, 14, 64, 7, 7, 1, 3), (2, 64, 15, 15, 64, 9, 5, 1, 4)], ids=lambda s: "x".join(map(str, s)))
+def test_no_copy_is_asked_for_that_no_kernel_reads(ctx, shape):
+    """A padding wider than the gaps between the copy's rows: the layer stages x inside its calls."""
+    assert ctx.conv2d_staged_floats(*shape) == 0
+
+
+@pytest.mark.parametrize("shape", [(4, 12, 20, 20, 48, 3, 3, 1, 1), (4, 64, 20, 20, 12, 3, 3, 1, 1), (2, 35, 18, 18, 40, 3, 3, 1, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_a_pointer_given_with_a_shape_that_has_no_copy_is_not_read(ctx, oracle, shape):
+    """The size of its copy is 0 floats: whatever the pointer refers to (here NaNs) was not written by katsu_cuda_conv2d_stage."""
+    n, c, h, w, k, r, s, stride, pad = shape
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    rng = np.random.default_rng(sum(shape))
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, n * k * oh * ow))
+    assert ctx.conv2d_staged_floats(*shape) == 0
+    with DeviceArrays(ctx, x=x, w=wt, g=g) as d:
+        for name, size in (("y", g.size), ("dw", wt.size), ("y2", g.size), ("dw2", wt.size), ("other", 16 * x.size)):
+            d.alloc(name, size, fill=np.nan)
+        ctx.conv2d_fwd(d["x"], d["w"], d["y"], *shape)
+        ctx.conv2d_bwd(d["x"], d["w"], d["g"], None, d["dw"], *shape, 0)
+        ctx.conv2d_fwd_staged(d["x"], d["other"], d["w"], None, d["y2"], *shape, 0)
+        ctx.conv2d_bwd_staged(d["x"], d["other"], d["w"], d["g"], None, 1.0, None, d["dw2"], *shape, 0)
+        assert np.array_equal(d.get("y"), d.get("y2")) and np.array_equal(d.get("dw"), d.get("dw2"))
+
+
 def test_shapes_that_stage_nothing_report_zero(ctx):
     assert ctx.conv2d_staged_floats(4, 3, 32, 32, 16, 3, 3, 1, 1) == 0     # stem kernels
     assert ctx.conv2d_staged_floats(2, 7, 13, 11, 9, 3, 3, 1, 1) == 0      # direct kernels
