@@ -23,6 +23,7 @@ struct katsu_cuda_ctx {
     // it are serialised by stream order.
     float *scratch;
     size_t scratch_floats;
+    bool scratch_captured;  // a captured graph refers to this block (katsu_scratch)
     // set by the *_staged entry points for the duration of one call: the caller's channels-innermost copy
     // of x (f16_conv.cu), written by katsu_cuda_conv2d_stage; the forward and dW launches use it instead of
     // staging x themselves

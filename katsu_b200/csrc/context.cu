@@ -8,6 +8,7 @@
 #include <mutex>
 #include <new>
 #include <unordered_map>
+#include <vector>
 
 #include "common.cuh"
 #include "launch.cuh"
@@ -63,6 +64,7 @@ struct KatsuBlockCache {
     std::unordered_map<void *, KatsuBlock> blocks;  // every block this context has handed out or holds
     std::multimap<size_t, void *> held;
     size_t held_bytes = 0, most_bytes = 0;
+    std::vector<void *> retired;  // earlier scratch blocks that captured graphs refer to
 };
 
 static size_t block_bytes(size_t bytes) {
@@ -151,19 +153,44 @@ int32_t katsu_pool_alloc(katsu_cuda_ctx *ctx, size_t bytes, void **out) {
     return KATSU_OK;
 }
 
+// A graph's kernels and tensor maps hold the address of the scratch block that they were captured with, for as long as the
+// caller keeps the graph.  So a block that a capture has used is never given back before shutdown, and a block that a capture
+// asks for is allocated beside it: allocated on the capturing stream it would belong to the graph, and be there only while
+// the graph runs.  One block is kept back for every growth behind a capture.
 int32_t katsu_scratch(katsu_cuda_ctx *ctx, size_t floats, float **out) {
+    const bool capturing = katsu_capturing(ctx);
     if (floats > ctx->scratch_floats) {
+        const size_t want = floats < (size_t(1) << 20) ? (size_t(1) << 20) : floats;
+        void *p = nullptr;
+        if (capturing || ctx->scratch_captured) {
+            try {
+                ctx->blocks->retired.reserve(ctx->blocks->retired.size() + 1);
+            } catch (...) {
+                return katsu_set_error(KATSU_ERR_ALLOC, "out of host memory");
+            }
+        }
+        if (capturing) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            KATSU_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t err = cudaMalloc(&p, want * sizeof(float));
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (err != cudaSuccess) {
+                cudaGetLastError();
+                return katsu_set_error(KATSU_ERR_ALLOC, "scratch of %zu bytes: %s", want * sizeof(float), cudaGetErrorString(err));
+            }
+        }
         // Stream-ordered: launches already queued keep the old block until they have run, and the
         // new one comes from the context's pool, so growing the scratch does not stall the device.
-        if (ctx->scratch) KATSU_CUDA_TRY(cudaFreeAsync(ctx->scratch, ctx->stream));
+        if (ctx->scratch && (capturing || ctx->scratch_captured)) ctx->blocks->retired.push_back(ctx->scratch);
+        else if (ctx->scratch) KATSU_CUDA_TRY(cudaFreeAsync(ctx->scratch, ctx->stream));
         ctx->scratch = nullptr;
         ctx->scratch_floats = 0;
-        size_t want = floats < (size_t(1) << 20) ? (size_t(1) << 20) : floats;
-        void *p = nullptr;
-        KATSU_TRY(katsu_pool_alloc(ctx, want * sizeof(float), &p));
+        ctx->scratch_captured = false;
+        if (!capturing) KATSU_TRY(katsu_pool_alloc(ctx, want * sizeof(float), &p));
         ctx->scratch = (float *)p;
         ctx->scratch_floats = want;
     }
+    if (capturing) ctx->scratch_captured = true;
     *out = ctx->scratch;
     return KATSU_OK;
 }
@@ -276,9 +303,10 @@ extern "C" int32_t katsu_cuda_shutdown(katsu_cuda_ctx *ctx) {
     KATSU_TRY(katsu_bind(ctx));
     cudaStreamSynchronize(ctx->stream);
     if (ctx->comm) katsu_comm_destroy_impl(ctx);
-    if (ctx->scratch) cudaFreeAsync(ctx->scratch, ctx->stream);
     give_back_blocks(ctx);
     cudaStreamSynchronize(ctx->stream);
+    if (ctx->scratch) cudaFree(ctx->scratch);
+    for (void *block : ctx->blocks->retired) cudaFree(block);
     if (ctx->flush) cudaFree(ctx->flush);
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->f16_state) cudaFree(ctx->f16_state);
