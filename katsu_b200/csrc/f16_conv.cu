@@ -199,7 +199,7 @@ int32_t katsu_f16_conv_stage(katsu_cuda_ctx *ctx, const float *x, void *staged, 
     katsu_f16_new_call(ctx);
     KatsuF16Info *info = katsu_f16_slot(ctx, KATSU_INFO_A);
     const Staged p = staged_at(static_cast<char *>(staged) + STAGED_HEADER, n, c, h, w, STAGED_GAP, 0);
-    const KatsuAmaxJob amax = {x, n * c * h * w, info};
+    const KatsuAmaxJob amax = katsu_amax_planes(x, n, c, h * w, info);
     KATSU_TRY(katsu_f16_amax(ctx, &amax, 1));
     KatsuStageJob job = nhwc_job(x, p, c, 0, info);
     job.info_copy = static_cast<KatsuF16Info *>(staged);
@@ -248,7 +248,7 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             return katsu_f16_drop_call(ctx);
         *handled = 1;
         const KatsuF16Call call = katsu_f16_call(ctx, info, iw, nullptr);
-        KatsuAmaxJob amax[2] = {{w, k * c * r * s, iw}, {x, n * c * h * wd, ix}};
+        KatsuAmaxJob amax[2] = {katsu_amax_matrix(w, k, c * r * s, iw), katsu_amax_planes(x, n, c, h * wd, ix)};
         KATSU_TRY(katsu_f16_amax(ctx, amax, prestaged ? 1 : 2));
         KatsuStageJob jobs[2] = {nhwc_job(x, own, c, 0, info), weights_job(w, ws, g, cp, width, iw)};
         jobs[0].only_if_mixed = prestaged ? 1 : 0;
@@ -401,15 +401,15 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         KatsuAmaxJob amax[3];
         KatsuStageJob jobs[3];
         int na = 0, nj = 0;
-        amax[na++] = {gr, n * k * oh * ow, ig};
+        amax[na++] = katsu_amax_planes(gr, n, k, oh * ow, ig);
         jobs[nj++] = nhwc_job(gr, sg, k, tail, ig);
         if (dw) {
-            if (!prestaged) amax[na++] = {x, n * c * h * wd, ix};
+            if (!prestaged) amax[na++] = katsu_amax_planes(x, n, c, h * wd, ix);
             jobs[nj] = nhwc_job(x, own, c, 0, info);
             jobs[nj++].only_if_mixed = prestaged ? 1 : 0;
         }
         if (dx) {
-            amax[na++] = {w, k * c * r * s, iw};
+            amax[na++] = katsu_amax_matrix(w, k, c * r * s, iw);
             KatsuStageJob &jw = jobs[nj++];
             jw = weights_job(w, ws, g, kp, width, iw);
             jw.backward = merged ? 2 : 1;

@@ -118,7 +118,7 @@ int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b
         if (!pass) continue;
         *handled = 1;
         const KatsuF16Call call = katsu_f16_call(ctx, ia, ib, nullptr);
-        const KatsuAmaxJob amax[2] = {{a, m * k, ia}, {b, k * n, ib}};
+        const KatsuAmaxJob amax[2] = {katsu_amax_matrix(a, m, k, ia), katsu_amax_matrix(b, k, n, ib)};
         KATSU_TRY(katsu_f16_amax(ctx, amax, 2));
         const KatsuStageJob jobs[2] = {transposed_job(b, k, n, q.lanes, ib), rows_job(a, m, k, q.columns, ia)};
         KATSU_TRY(katsu_f16_stage(ctx, call, jobs, 2));
@@ -170,14 +170,14 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
         KatsuAmaxJob amax[3];
         KatsuStageJob jobs[4];
         int na = 0, nj = 0;
-        amax[na++] = {g, m * n, ig};
+        amax[na++] = katsu_amax_matrix(g, m, n, ig);
         if (da) {
-            amax[na++] = {b, k * n, ib};
+            amax[na++] = katsu_amax_matrix(b, k, n, ib);
             jobs[nj++] = rows_job(b, k, n, qa.lanes, ib);
             jobs[nj++] = rows_job(g, m, n, qa.columns, ig);
         }
         if (db) {
-            amax[na++] = {a, m * k, ia};
+            amax[na++] = katsu_amax_matrix(a, m, k, ia);
             jobs[nj++] = transposed_job(g, m, n, qb.lanes, ig);
             jobs[nj++] = transposed_job(a, m, k, qb.columns, ia);
         }

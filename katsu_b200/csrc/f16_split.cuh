@@ -7,10 +7,15 @@
 // 2^-(exp_a + exp_b) is applied to the f32 sums, so the scale itself costs no rounding.
 //
 // What fp16 lacks is range.  Below 2^-14 it goes subnormal: an element's error never exceeds 2^-25 of the scaled
-// range = 2^-39 of the tensor's largest magnitude.  The pass that finds that magnitude therefore also finds the
-// SMALLEST maximum over all groups of 128 consecutive elements that are not all zero, and a tensor counts as narrow
-// only if every group's maximum is within 2^17 of the tensor's (two planes) or 2^28 (one plane): then no element's
-// error exceeds 2^-22 (2^-11) of the largest magnitude in its own neighbourhood, which is the bar of the TF32 forms.
+// range = 2^-39 of the tensor's largest magnitude (2^-26 - 2^-25 with one plane: 11 bits down to 2^-28).  An output that
+// depends on small elements alone (a column of b, an input channel of w, a dim region of an image) would lose what TF32
+// parts keep, so the pass that finds the largest magnitude also finds the SMALLEST maximum over groups of elements that
+// are not all zero, along both axes of the tensor: up to 128 neighbours in a row, and up to 16 rows of a column (a row of
+// a matrix, of weights [k][c * r * s], or a channel's plane of an image).  A tensor counts as narrow only if every group's
+// maximum is within 2^17 of the tensor's (two planes) or 2^28 (one plane): then no element's error exceeds 2^-22 (2^-11)
+// of the largest magnitude around it in its row, and in its column.  Within such a neighbourhood of 16 x 128 elements of
+// mixed sizes the small ones do have fewer bits than TF32 parts would give them.  (Groups of single elements would keep
+// those too, but every normally distributed tensor of more than a few thousand elements holds one below 2^-17.)
 //
 // If one operand of a call has a wider range, or holds infinities or NaNs, all of the call's operands are written as
 // bf16 planes instead: each the leading 8 significand bits of what the planes before it left, three of them (two in
@@ -57,12 +62,24 @@ __device__ __forceinline__ bool katsu_f16_wide(const KatsuF16Call &call) {
     return !(katsu_f16_narrow(v[0], call.span) && katsu_f16_narrow(v[1], call.span) && katsu_f16_narrow(v[2], call.span));
 }
 
-// One operand whose magnitude is to be found.
+// One operand whose magnitude is to be found: matrices [images][rows][cols], none of the sizes 0.
 struct KatsuAmaxJob {
     const float *src;
-    size_t count;
+    unsigned images, rows, cols;
+    bool columns;  // groups along columns too
     KatsuF16Info *info;
 };
+
+static inline KatsuAmaxJob katsu_amax_matrix(const float *src, size_t rows, size_t cols, KatsuF16Info *info) {
+    return {src, 1, (unsigned)rows, (unsigned)cols, true, info};
+}
+
+// An image tensor [n][c][pixels]; without pixels beside each other a matrix [n][c].  With one channel a group along a
+// column would be a single pixel.
+static inline KatsuAmaxJob katsu_amax_planes(const float *src, size_t n, size_t c, size_t pixels, KatsuF16Info *info) {
+    if (pixels == 1) return katsu_amax_matrix(src, n, c, info);
+    return {src, (unsigned)n, (unsigned)c, (unsigned)pixels, c > 1, info};
+}
 
 enum KatsuStageKind { KATSU_STAGE_NHWC, KATSU_STAGE_ROWS, KATSU_STAGE_WEIGHTS };
 

@@ -13,11 +13,14 @@ constexpr int THREADS = 256;
 constexpr int STAGE_BLOCKS = 5;  // resident staging blocks per SM
 
 // ---- largest magnitude ------------------------------------------------------------------------------------------
+constexpr int AMAX_BLOCKS = 3;   // resident blocks per SM
+constexpr int AMAX_ROWS = 16;    // rows of a strip at most
+
 struct AmaxSegment {
-    const float *src;
-    unsigned long long count;
-    KatsuF16Info *info;
+    KatsuAmaxJob job;
+    unsigned strips, strip_rows, col_tiles;  // of a matrix
     unsigned first_block, blocks;
+    int vec;  // 128 columns to a tile, a float4 to a lane; else 32
 };
 
 struct AmaxParams {
@@ -26,62 +29,80 @@ struct AmaxParams {
 };
 
 __device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-__device__ __forceinline__ unsigned max4(float4 v) {
-    return max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w)));
+
+// Magnitudes of ROWS rows of a tile, W columns to a lane, all loads in flight before the first use and no branch between
+// them (with a range check around each load the compiler kept one in flight: 100 us for 103 M floats).  Rows past the last
+// are the last one again, which changes no maximum.
+template <int ROWS, int W>
+__device__ __forceinline__ void amax_rows(const float *src, size_t pitch, unsigned rows, unsigned &most, unsigned &least,
+                                          unsigned (&column)[W]) {
+    unsigned v[ROWS][W];
+#pragma unroll
+    for (unsigned i = 0; i < ROWS; ++i) {
+        const float *at = src + size_t(min(i, rows - 1)) * pitch;
+        if (W == 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(at));
+            v[i][0] = magnitude(q.x);
+            v[i][W > 1 ? 1 : 0] = magnitude(q.y);
+            v[i][W > 2 ? 2 : 0] = magnitude(q.z);
+            v[i][W > 3 ? 3 : 0] = magnitude(q.w);
+        } else {
+            v[i][0] = magnitude(__ldg(at));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        unsigned m = v[i][0];
+#pragma unroll
+        for (int u = 0; u < W; ++u) {
+            column[u] = max(column[u], v[i][u]);
+            if (u) m = max(m, v[i][u]);
+        }
+        m = __reduce_max_sync(0xffffffffu, m);
+        most = max(most, m);
+        least = min(least, m ? m : 0x7fffffffu);
+    }
 }
 
-// A group is the 128 consecutive floats that a warp reads at once; the last group of a tensor reaches back so that
-// it is a full one.  Magnitudes compare as their bit patterns, which puts infinities and NaNs above every number.
-__global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ AmaxParams p) {
+template <int W>
+__device__ __forceinline__ void amax_tiles(const AmaxSegment &sg, unsigned first, unsigned stride, unsigned &most, unsigned &least) {
+    const KatsuAmaxJob &j = sg.job;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long tiles = (unsigned long long)j.images * sg.strips * sg.col_tiles;
+    unsigned least_column = 0x7fffffffu;
+    // From the tensor's end to its front: the staging pass starts at the front, which then is what L2 holds.
+    for (unsigned long long left = tiles - min((unsigned long long)first, tiles); left > 0; left -= min((unsigned long long)stride, left)) {
+        const unsigned long long rest = (left - 1) / sg.col_tiles;
+        const unsigned tile = unsigned(left - 1 - rest * sg.col_tiles);
+        const unsigned long long image = rest / sg.strips;
+        const unsigned row = unsigned(rest - image * sg.strips) * sg.strip_rows, rows = min(sg.strip_rows, j.rows - row);
+        // the last tile reaches back so that it is a full one; lanes past a narrow row read its last columns again
+        unsigned col = tile * (32 * W);
+        if (col + 32 * W > j.cols) col = j.cols > 32 * W ? j.cols - 32 * W : 0;
+        col = min(col + lane * W, j.cols - W);
+        const float *src = j.src + (size_t(image) * j.rows + row) * j.cols + col;
+        unsigned column[W] = {};
+        if (rows <= 4) amax_rows<4, W>(src, j.cols, rows, most, least, column);
+        else if (rows <= 8) amax_rows<8, W>(src, j.cols, rows, most, least, column);
+        else amax_rows<AMAX_ROWS, W>(src, j.cols, rows, most, least, column);
+#pragma unroll
+        for (int u = 0; u < W; ++u) least_column = min(least_column, column[u] ? column[u] : 0x7fffffffu);
+    }
+    if (j.columns) least = min(least, __reduce_min_sync(0xffffffffu, least_column));
+}
+
+// Magnitudes compare as their bit patterns, which puts infinities and NaNs above every number.
+__global__ void __launch_bounds__(THREADS, AMAX_BLOCKS) amax_kernel(const __grid_constant__ AmaxParams p) {
     launch_next();
     launch_wait();
     int si = 0;
     while (si + 1 < p.segments && blockIdx.x >= p.seg[si + 1].first_block) ++si;
     const AmaxSegment &sg = p.seg[si];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned long long groups = (sg.count + 127) / 128;
-    const unsigned long long stride = (unsigned long long)sg.blocks * (THREADS / 32);
-    const bool vec = (reinterpret_cast<uintptr_t>(sg.src) & 15u) == 0;
+    const unsigned first = (blockIdx.x - sg.first_block) * (THREADS / 32) + warp, stride = sg.blocks * (THREADS / 32);
     unsigned most = 0, least = 0x7fffffffu;
-    auto take = [&](unsigned m) {
-        m = __reduce_max_sync(0xffffffffu, m);
-        most = max(most, m);
-        least = min(least, m ? m : 0x7fffffffu);
-    };
-    auto load = [&](unsigned long long g) -> unsigned {  // any group
-        unsigned long long at = g * 128;
-        if (at + 128 > sg.count) at = sg.count > 128 ? sg.count - 128 : 0;
-        unsigned m = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const unsigned long long e = at + lane + 32 * i;
-            if (e < sg.count) m = max(m, magnitude(__ldg(sg.src + e)));
-        }
-        return m;
-    };
-    // Warps walk from the tensor's end to its front: the staging pass starts at the front, which then is what L2 holds.
-    // `left` groups are not yet read by anybody from this warp's place on; its next one is left - 1.
-    long long left = (long long)groups - ((long long)(blockIdx.x - sg.first_block) * (THREADS / 32) + warp);
-    const long long step = (long long)stride;
-    if ((sg.count & 127) != 0 && left == (long long)groups) {  // the ragged last group
-        take(load(groups - 1));
-        left -= step;
-    }
-    if (vec) {
-        // Eight 16-byte loads in flight per thread, with no branch between them: with the range checks of load() around
-        // each the compiler kept one in flight (103 M floats: 100 us).
-        const float4 *src = reinterpret_cast<const float4 *>(sg.src) + lane;
-        for (; left > 7 * step; left -= 8 * step) {
-            float4 v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __ldg(src + (left - 1 - i * step) * 32);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) take(max4(v[i]));
-        }
-        for (; left > 0; left -= step) take(max4(__ldg(src + (left - 1) * 32)));
-    } else {
-        for (; left > 0; left -= step) take(load(left - 1));
-    }
+    if (sg.vec) amax_tiles<4>(sg, first, stride, most, least);
+    else amax_tiles<1>(sg, first, stride, most, least);
 
     __shared__ unsigned sh_most[THREADS / 32], sh_least[THREADS / 32];
     if (lane == 0) {
@@ -95,8 +116,8 @@ __global__ void __launch_bounds__(THREADS) amax_kernel(const __grid_constant__ A
         least = min(least, sh_least[i]);
     }
     // no result is waited for: the kernels behind this one read the slots when it has ended
-    atomicMax(&sg.info->most, most);
-    if (most) atomicMax(&sg.info->inverted_least, 0x7fffffffu - least);
+    atomicMax(&sg.job.info->most, most);
+    if (most) atomicMax(&sg.job.info->inverted_least, 0x7fffffffu - least);
 }
 
 __global__ void clear_kernel(KatsuF16Info *info) {
@@ -427,13 +448,14 @@ int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count)
     unsigned at = 0;
     for (int i = 0; i < count; ++i) {
         AmaxSegment &s = p.seg[i];
-        s.src = jobs[i].src;
-        s.count = jobs[i].count;
-        s.info = jobs[i].info;
-        // a warp takes eight groups of 128 at once; at most eight resident blocks per SM
-        size_t blocks = katsu_div_up(jobs[i].count, size_t(128) * 8 * (THREADS / 32));
-        if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
-        if (blocks < 1) blocks = 1;
+        s.job = jobs[i];
+        s.vec = (jobs[i].cols & 3) == 0 && (reinterpret_cast<uintptr_t>(jobs[i].src) & 15u) == 0;
+        s.strips = (jobs[i].rows + AMAX_ROWS - 1) / AMAX_ROWS;
+        s.strip_rows = (jobs[i].rows + s.strips - 1) / s.strips;  // even strips: no group of a row or two at the end
+        s.strips = (jobs[i].rows + s.strip_rows - 1) / s.strip_rows;
+        s.col_tiles = (jobs[i].cols + (s.vec ? 127 : 31)) / (s.vec ? 128 : 32);
+        size_t blocks = katsu_div_up(size_t(jobs[i].images) * s.strips * s.col_tiles, (size_t)(THREADS / 32));
+        if (blocks > size_t(ctx->num_sms) * AMAX_BLOCKS) blocks = size_t(ctx->num_sms) * AMAX_BLOCKS;
         s.first_block = at;
         s.blocks = (unsigned)blocks;
         at += s.blocks;

@@ -122,6 +122,83 @@ def test_one_image_far_below_the_others(ctx, oracle, small, staged):
         assert max(errors) <= bar, (small, staged, mode, errors)
 
 
+# Parts of an operand far below the rest that no run of 128 neighbours in memory is made of: the error of the outputs that
+# depend on that part alone.  Sizes at which the part lies inside the first tile of the magnitude pass and in its last,
+# ragged one, rows short and long, aligned and not.
+@pytest.mark.parametrize("size", [(300, 700, 515), (515, 516, 512), (2000, 100, 600), (420, 33, 3100)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("scale", [1e-6, 1e-8, 1e-12])
+def test_small_rows_and_columns_of_matrices(ctx, oracle, size, scale):
+    m, k, n = size
+    rng = np.random.default_rng(11)
+    whole = [rng.standard_normal(v).astype(np.float32) for v in ((m, k), (k, n), (m, n))]
+    for mode, bar in BARS:
+        ctx.set_precision(mode)
+        try:
+            # operand, its small row or column, the output that it reaches alone, at which row or column of it
+            for which, axis, output in ((0, 0, 0), (0, 1, 2), (1, 0, 1), (1, 1, 0), (2, 0, 1), (2, 1, 2)):
+                operands = [v.copy() for v in whole]
+                length = operands[which].shape[axis]
+                for at in (3, length - 1):
+                    operands[which] = whole[which].copy()
+                    part = (at, slice(None)) if axis == 0 else (slice(None), at)
+                    operands[which][part] *= np.float32(scale)
+                    a, b, g = operands
+                    a64, b64, g64 = (v.astype(np.float64) for v in operands)
+                    want = (a64 @ b64, g64 @ b64.T, a64.T @ g64)[output]
+                    with DeviceArrays(ctx, a=a, b=b, g=g) as d:
+                        d.alloc("out", want.size, fill=np.nan)
+                        if output == 0:
+                            ctx.matmul_fwd(d["a"], d["b"], d["out"], m, k, n)
+                        else:
+                            da, db = (d["out"], None) if output == 1 else (None, d["out"])
+                            ctx.matmul_bwd(d["a"], d["b"], d["g"], da, db, m, k, n, 0)
+                        got = d.get("out").reshape(want.shape)
+                    # an output row for a small row of a or g and a small column of a (row of db) or row of b (column of da)
+                    out_axis = {(0, 0): 0, (0, 1): 0, (1, 0): 1, (1, 1): 1, (2, 0): 0, (2, 1): 1}[which, axis]
+                    part = (at, slice(None)) if out_axis == 0 else (slice(None), at)
+                    assert rel_l2(got[part], want[part]) <= bar, (mode, which, axis, at)
+        finally:
+            ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("shape", [(4, 48, 7, 7, 40, 3, 3, 1, 1), (3, 33, 14, 15, 30, 3, 3, 1, 1), (4, 64, 12, 12, 64, 1, 1, 1, 0), (6, 3, 40, 40, 24, 5, 5, 2, 2),
+                                   (200, 64, 1, 1, 128, 1, 1, 1, 0)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("scale", [1e-6, 1e-8, 1e-12])
+def test_small_channels_and_regions(ctx, oracle, shape, scale):
+    n, c, h, w, k, r, s, stride, pad = shape
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    xs, ws, gs = (n, c, h, w), (k, c, r, s), (n, k, oh, ow)
+    rng = np.random.default_rng(12)
+    whole = [rng.standard_normal(v).astype(np.float32) for v in (xs, ws, gs)]
+    every = slice(None)
+    dim = (every, every, every, slice(0, max(0, (w // 2 - s + pad) // stride + 1)))  # outputs whose window lies in the left half
+    parts = [(0, (every, c - 1), 2, (every, c - 1)), (0, (1,), 0, (1,)), (0, (every, every, every, slice(0, w // 2)), 0, dim),
+             (1, (every, 2), 1, (every, 2)), (1, (k - 1,), 0, (every, k - 1)), (2, (every, 5), 2, (5,)), (2, (n - 1,), 1, (n - 1,))]
+    for mode, bar in BARS:
+        ctx.set_precision(mode)
+        try:
+            for which, part, output, reached in parts:
+                if which == 0 and len(part) == 4 and w == 1:
+                    continue
+                t = [v.copy() for v in whole]
+                t[which][part] *= np.float32(scale)
+                x, wt, g = (v.reshape(-1) for v in t)
+                y64 = oracle.conv2d_forward_f64(x, wt, list(xs), list(ws), stride, pad)
+                dx64, dw64 = oracle.conv2d_backward_f64(x, wt, g, list(xs), list(ws), stride, pad)
+                want = (y64.reshape(gs), dx64.reshape(xs), dw64.reshape(ws))[output]
+                with DeviceArrays(ctx, x=x, w=wt, g=g) as d:
+                    d.alloc("out", want.size, fill=np.nan)
+                    if output == 0:
+                        ctx.conv2d_fwd(d["x"], d["w"], d["out"], *shape)
+                    else:
+                        dx, dw = (d["out"], None) if output == 1 else (None, d["out"])
+                        ctx.conv2d_bwd(d["x"], d["w"], d["g"], dx, dw, *shape, 0)
+                    got = d.get("out").reshape(want.shape)
+                assert rel_l2(got[reached], want[reached]) <= bar, (mode, which, part)
+        finally:
+            ctx.set_precision(0)
+
+
 @pytest.mark.parametrize("scale", [1e-30, 1e-5, 1e25])
 def test_magnitudes_of_whole_tensors(ctx, oracle, scale):
     """A common factor of a whole operand, up to where its fp16 scale would leave f32."""
