@@ -264,6 +264,7 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         p.a_second = prestaged ? 1 : 0;
         p.m_total = box.blocks * 128;
         p.n_total = (int)k;
+        p.f32_terms = regular(g) ? 0 : (long long)(c * r * s);
         p.col_stride = (long long)(oh * ow);
         p.row_begin[1] = (int)r;
         for (size_t i = 0; i < r; ++i) p.off_h[i] = p.b_row[i] = (short)i;
@@ -436,6 +437,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.gscale = gscale;
             p.gfactor = gfactor;
             p.m_total = box_dx.blocks * 128;
+            p.f32_terms = regular(g) ? 0 : (long long)katsu_div_up(k * r * s, stride * stride);
             p.n_total = (int)c;
             p.col_stride = (long long)(h * wd);
             p.step = (int)stride;
@@ -471,6 +473,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.gscale = gscale;
             p.gfactor = gfactor;
             p.m_total = (long long)dw_lanes;
+            p.f32_terms = regular(g) ? 0 : 1;  // the direct kernel's sums over pixels are split into short ones
             p.n_total = (int)k;
             p.col_stride = (long long)dw_lanes;
             p.in_step = (int)stride;

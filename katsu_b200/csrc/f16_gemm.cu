@@ -22,8 +22,10 @@
 //
 // Passes.  Narrow operands (fp16): hi*hi in TF32 mode (NARROW = 1), lo*hi + hi*lo + hi*hi in 3xTF32 mode (NARROW = 2).
 // Wide operands (bf16): the three largest products of two planes, or the six largest of three.  The tensor core's f32
-// accumulation loses about 3e-8 per accumulation step, so in 3xTF32 mode an accumulator receives at most 192 steps before
-// eight epilogue warps fold it into f32 registers while the other one fills.
+// accumulation loses about 2e-8 of the sum per step, always towards zero, so the loss grows with the steps; in 3xTF32 mode
+// eight epilogue warps fold an accumulator into f32 registers every p.drain k-blocks (katsu_f16_launch has the rule) while
+// others fill.  A `fine` problem takes the small products of a k-block first, whose steps lose little, then the four steps of
+// hi*hi, at 4 to 10 % more time than products in the order of the steps (which use A's rows twice in a row).
 //
 // What bounds it: at 256 x 256 a k-block is 12 (4) MMAs of 128 clocks against 64 (32) KiB of operand fill per block,
 // the ratio of the TF32 kernels at twice their rate.
@@ -43,6 +45,7 @@ namespace {
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 8;
+constexpr int MAX_ACCS = 4;
 constexpr int THREADS = 320;
 constexpr uint32_t kLayoutSw64 = 4;
 constexpr int RASTER_M = 16;
@@ -169,7 +172,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     constexpr bool MN = KIND == KATSU_F16_CONV_DW, CONV = KIND == KATSU_F16_CONV || KIND == KATSU_F16_CONV_DX2;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[MAX_ACCS], acc_empty[MAX_ACCS];
     __shared__ uint32_t tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -185,7 +188,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
             mbar_init(&full[s], 1);    // the leader's: its own expect_tx arrival, both blocks' bytes
             mbar_init(&empty[s], 1);   // each block's own copy, released by the leader's commit
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < MAX_ACCS; ++b) {
             mbar_init(&acc_full[b], 1);    // each block's own copy
             mbar_init(&acc_empty[b], 16);  // the leader's: eight epilogue warps of each block
         }
@@ -205,8 +208,10 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     const KatsuF16Info info_a = katsu_f16_load(p.info_a), info_b = katsu_f16_load(p.info_b);
     const bool wide = katsu_f16_wide(p.call);
     const int planes = NARROW + (wide ? 1 : 0);
-    // k-blocks between two drains: 192 accumulation steps in 3xTF32 mode, up to 12 288 in TF32 mode (4e-4 of 2e-3)
-    const int drain = NARROW == 2 ? (wide ? 8 : 16) : 1024;
+    // k-blocks between two drains: in TF32 mode up to 12 288 accumulation steps (4e-4 of 2e-3)
+    const int drain = NARROW == 2 ? (wide ? (p.drain + 1) / 2 : p.drain) : 1024;
+    // accumulators that take turns; hand-over q is the one q & (2^acc_bits - 1), acc_cols columns apart
+    const int acc_bits = p.bn <= 128 ? 2 : 1, acc_mask = (1 << acc_bits) - 1, acc_cols = 512 >> acc_bits;
     const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
     const int stages = min(MAX_STAGES, SMEM_RING / stage_bytes);
 
@@ -322,12 +327,12 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                     int chunk = (!MN && kb1 > kb0) ? kb0 % chunks : 0;
                     const int last = MN ? BK / 16 : p.steps_last[px];
                     for (int kb = kb0; kb < kb1 && ok; ++q) {
-                        const int b = q & 1;
-                        if (!mbar_wait_warp(&acc_empty[b], ((q >> 1) & 1) ^ 1, p.status, 172)) { ok = false; break; }
+                        const int b = q & acc_mask;
+                        if (!mbar_wait_warp_ready(&acc_empty[b], ((q >> acc_bits) & 1) ^ 1, p.status, 172)) { ok = false; break; }
                         tc_fence_after_sync();
-                        const uint32_t acc = tmem_base + uint32_t(b) * 256;
+                        const uint32_t acc = tmem_base + uint32_t(b * acc_cols);
                         const int kb_end = min(kb + drain, kb1);
-                        bool first = true;
+                        bool add = false;
                         for (; kb < kb_end; ++kb) {
                             if (!mbar_wait_warp_ready(&full[s], phase, p.status, 173)) { ok = false; break; }
                             tc_fence_after_sync();
@@ -337,40 +342,45 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             const uint64_t b0 = smem_desc(st + b_off, lbo, b_sbo, b_layout);
                             const int steps = (!MN && chunk == chunks - 1) ? last : BK / 16;
                             if (issue) {
+                                // plane pa of A times plane pb of B, all steps of the k-block
+                                auto product = [&](uint32_t pa, uint32_t pb) {
+                                    const uint64_t ap = a0 + pa * (A_BYTES >> 4), bp = b0 + pb * (uint32_t(b_bytes) >> 4);
 #pragma unroll
-                                for (int j = 0; j < BK / 16; ++j) {
-                                    if (j < steps) {
-                                        const uint64_t ad = a0 + j * (a_step >> 4), bd = b0 + j * (b_step >> 4);
-                                        const uint32_t na = A_BYTES >> 4, nb = b_bytes >> 4;  // to the next plane
-                                        const bool add = !(first && j == 0);
-                                        if (NARROW == 2) {
-                                            if (wide) {
-                                                mma_f16_pair(acc, ad + 2 * na, bd, idesc, add);
-                                                mma_f16_pair(acc, ad + na, bd + nb, idesc, true);
-                                                mma_f16_pair(acc, ad, bd + 2 * nb, idesc, true);
+                                    for (int j = 0; j < BK / 16; ++j) {
+                                        if (j < steps) {
+                                            mma_f16_pair(acc, ap + j * (a_step >> 4), bp + j * (b_step >> 4), idesc, add);
+                                            add = true;
+                                        }
+                                    }
+                                };
+                                if (NARROW == 2 && wide) {
+                                    product(2, 0);
+                                    product(1, 1);
+                                    product(0, 2);
+                                }
+                                if (NARROW == 2 && p.fine) {
+                                    product(1, 0);
+                                    product(0, 1);
+                                    product(0, 0);
+                                } else {
+#pragma unroll
+                                    for (int j = 0; j < BK / 16; ++j) {
+                                        if (j < steps) {
+                                            const uint64_t ad = a0 + j * (a_step >> 4), bd = b0 + j * (b_step >> 4);
+                                            if (NARROW == 2 || wide) {
+                                                mma_f16_pair(acc, ad + (A_BYTES >> 4), bd, idesc, add);
+                                                mma_f16_pair(acc, ad, bd + (uint32_t(b_bytes) >> 4), idesc, true);
                                             }
-                                            mma_f16_pair(acc, ad + na, bd, idesc, add || wide);
-                                            mma_f16_pair(acc, ad, bd + nb, idesc, true);
-                                            mma_f16_pair(acc, ad, bd, idesc, true);
-                                        } else {
-                                            if (wide) {
-                                                mma_f16_pair(acc, ad + na, bd, idesc, add);
-                                                mma_f16_pair(acc, ad, bd + nb, idesc, true);
-                                            }
-                                            mma_f16_pair(acc, ad, bd, idesc, add || wide);
+                                            mma_f16_pair(acc, ad, bd, idesc, add || NARROW == 2 || wide);
+                                            add = true;
                                         }
                                     }
                                 }
                                 // every release goes to this block's barrier and to the peer's copy of it
-                                mma_commit_pair(smem_u32(&empty[s]));
-                                mma_commit_pair(map_to_rank(&empty[s], 1));
-                                if (kb == kb_end - 1) {
-                                    mma_commit_pair(smem_u32(&acc_full[b]));
-                                    mma_commit_pair(map_to_rank(&acc_full[b], 1));
-                                }
+                                if (kb == kb_end - 1) mma_commit_both(&acc_full[b]);
+                                mma_commit_both(&empty[s]);
                             }
                             __syncwarp();
-                            first = false;
                             if (!MN && ++chunk == chunks) chunk = 0;
                             if (++s == stages) {
                                 s = 0;
@@ -438,9 +448,9 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         return p.bias && col < p.n_total ? __ldg(p.bias + col) : 0.f;
                     };
                     auto wait_acc = [&](int b) -> uint32_t {
-                        alive = mbar_wait_warp(&acc_full[b], (q >> 1) & 1, p.status, 174);
+                        alive = mbar_wait_warp(&acc_full[b], (q >> acc_bits) & 1, p.status, 174);
                         tc_fence_after_sync();
-                        return tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b) * 256;
+                        return tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * acc_cols);
                     };
                     auto release_acc = [&](int b) {
                         tc_fence_before_sync();
@@ -455,7 +465,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         float bias[4];
 #pragma unroll
                         for (int c = 0; c < 4; ++c) bias[c] = bias_of((2 * c + group) * 32);
-                        const uint32_t acc = kb1 > kb0 ? wait_acc(q & 1) : 0;
+                        const uint32_t acc = kb1 > kb0 ? wait_acc(q & acc_mask) : 0;
                         if (!alive) break;
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
@@ -471,7 +481,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             put(c0, v, bias[c]);
                         }
                         if (kb1 > kb0) {
-                            release_acc(q & 1);
+                            release_acc(q & acc_mask);
                             ++q;
                         }
                         continue;
@@ -488,18 +498,19 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             }
                         }
                     for (int kb = kb0; kb < kb1; kb += drain, ++q) {
-                        const uint32_t acc = wait_acc(q & 1);
+                        const uint32_t acc = wait_acc(q & acc_mask);
                         if (!alive) break;
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
                             if (2 * c + group < col_chunks) {
                                 float v[32];
                                 tmem_ld_32x32(acc + (2 * c + group) * 32, v);
+                                if (2 * c + group + 2 >= col_chunks) release_acc(q & acc_mask);
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) run[c][i] += v[i];
                             }
                         }
-                        release_acc(q & 1);
+                        if (group >= col_chunks) release_acc(q & acc_mask);
                     }
                     if (!alive) break;
                     if (pairs_of_x) {
@@ -610,6 +621,15 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
                 if (kb > most) most = kb;
             }
     }
+    // 3xTF32 mode: k-blocks to an accumulator, and with it the error against 64-bit sums of normally distributed values: 1 fine
+    // 1.5e-7, 1 2.6e-7, 2 4.8e-7, 5 1.2e-6, 16 3.6e-6.  The lines lie where that is below the error of other arithmetic of this
+    // mode's grade: kernels that cut operands into TF32 parts have 4.6e-7 to 8e-7 up to 8 k-blocks, 1.4e-6 and 1.6e-6 at 9
+    // and 13, 4e-6 from 16 on, and 5e-7 to 4e-6 in dW; f32 multiply-adds 1.8e-8 times the root of their number (2.9e-7 for
+    // 256 terms, 5.1e-7 for 800).  A drain costs more the shorter a tile's k-loop is (4096^3: 351 us with 16, 359 with 4, 375
+    // with 2, 411 with 1; 64 channels, 8 x 56 x 56: 26.3, 27.9, 29.4, 31.4).
+    p.fine = p.f32_terms > 0 && p.f32_terms < 256;
+    if (p.f32_terms > 0) p.drain = p.f32_terms < 800 ? 1 : 2;
+    else p.drain = kind == KATSU_F16_CONV_DW || most < 9 ? 2 : most < 16 ? 5 : 16;
     p.kb_per_split = (int)((most + plan.splits - 1) / plan.splits);
     if (p.kb_per_split < 1) p.kb_per_split = 1;
     p.split_stride = 0;

@@ -20,6 +20,9 @@ struct KatsuF16Problem {
     float *out;
     const float *bias;  // per column, or null
     int relu, accumulate;
+    // Terms of one sum where TF32 parts would not do for 3xTF32 mode, because the shape can have f32 multiply-adds (rows that
+    // are not whole 16-byte units, few channels); 0 elsewhere.
+    long long f32_terms;
     KatsuF16Call call;
     const KatsuF16Info *info_a, *info_b;
     // A's planes come from the second set of maps when the call is wide and A's own copy, made before the call, is not
@@ -54,7 +57,7 @@ struct KatsuF16Problem {
     int a_pairs, b_pairs;  // the maps are of the `pairs` form: one load brings two column groups
     int a_bytes;  // bytes of one loaded A part of a k-block
     // filled in by the launcher
-    int bn, m_tiles, n_tiles, splits, kb_per_split;
+    int bn, m_tiles, n_tiles, splits, kb_per_split, drain, fine;
     long long split_stride;
     int *status;
 };

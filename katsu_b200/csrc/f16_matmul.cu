@@ -47,6 +47,7 @@ struct Product {
     size_t n_lanes, n_columns, k;
     float *out;
     int accumulate;
+    bool regular;
     KatsuF16Plan plan;
 };
 
@@ -60,6 +61,7 @@ int32_t run(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Product &q, flo
     KatsuF16Problem p = {};
     p.out = q.out;
     p.accumulate = q.accumulate;
+    p.f32_terms = q.regular ? 0 : (long long)q.k;
     p.call = call;
     p.info_a = q.info_lanes;
     p.info_b = q.info_columns;
@@ -78,6 +80,12 @@ int32_t run(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Product &q, flo
         KATSU_TRY(katsu_f16_fold(ctx, partial, q.out, count, q.plan.splits, q.accumulate,
                                  nullptr, 1, 1, 0));
     return KATSU_OK;
+}
+
+// Products of matrices whose rows are whole 16-byte units at 16-byte addresses, and no sliver: those that TF32 parts suit.
+bool regular(const float *a, const float *b, const float *c, size_t m, size_t n, size_t k) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+    return (at & 15u) == 0 && m >= 64 && n >= 32 && k >= 32;
 }
 
 KatsuF16Plan plan_for(const katsu_cuda_ctx *ctx, size_t n_lanes, size_t n_columns, size_t k) {
@@ -101,6 +109,7 @@ int32_t katsu_f16_matmul_fwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     q.n_columns = m;
     q.k = k;
     q.out = c;
+    q.regular = k % 4 == 0 && n % 4 == 0 && regular(a, b, c, m, n, k);
     katsu_f16_new_call(ctx);
     KatsuF16Info *ia = katsu_f16_slot(ctx, KATSU_INFO_A), *ib = katsu_f16_slot(ctx, KATSU_INFO_B);
     q.info_lanes = ib;
@@ -138,10 +147,12 @@ int32_t katsu_f16_matmul_bwd(katsu_cuda_ctx *ctx, const float *a, const float *b
     qa.plan = plan_for(ctx, k, m, n);
     qa.n_lanes = k; qa.n_columns = m; qa.k = n;
     qa.out = da; qa.accumulate = accumulate;
+    qa.regular = n % 4 == 0 && regular(g, b, da, m, k, n);
     qa.info_lanes = ib; qa.info_columns = ig;
     qb.plan = plan_for(ctx, n, k, m);
     qb.n_lanes = n; qb.n_columns = k; qb.k = m;
     qb.out = db;
+    qb.regular = k % 4 == 0 && n % 4 == 0 && regular(a, g, db, k, n, m);
     // da == db (the same parent on both edges): the second product adds to the first whatever `accumulate` says
     qb.accumulate = da != nullptr && da == db ? 1 : accumulate;
     qb.info_lanes = ig; qb.info_columns = ia;

@@ -50,6 +50,13 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t addr) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(addr) : "memory");
 }
 
+// The same on the barrier at this place in both blocks of the pair.
+__device__ __forceinline__ void mma_commit_both(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((unsigned short)3)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tma_load_3d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_addr, int c0, int c1,
                                                  int c2) {
     asm volatile(

@@ -256,3 +256,36 @@ def test_small_regular_layers_stay_on_the_tensor_cores(ctx, oracle, shape):
         ctx.conv2d_fwd(d["x"], d["w"], d["y"], *shape)
         assert ctx.launch_count() - before >= 3  # magnitudes, planes, product; a direct kernel is one launch
     assert max(conv_errors(ctx, oracle, shape, x, wt, g)) <= REL_L2_TOL
+
+
+# What a 3xTF32 result may lose to the tensor core's accumulation, beside the 22 bits of its operands (6e-8): a step truncates
+# the sum by 2e-8 of it on average, and 12 steps (3 products) of 64 terms go to an accumulator before it is added to f32 sums,
+# or 24.  Taken small products first, 4 of the 12 count.  Twice the measured errors of 1.5e-7, 2.6e-7 and 4.8e-7 at most.
+FINE, ONE, TWO = 6e-8 + 4 * 4e-8, 6e-8 + 12 * 2.5e-8, 6e-8 + 24 * 2.5e-8
+
+
+@pytest.mark.parametrize("size, bars", [((333, 1001, 777), (TWO, ONE, ONE)), ((2050, 67, 1030), (FINE, TWO, TWO)), ((200, 300, 3001), (ONE, TWO, FINE)),
+                                        ((1024, 128, 512), (TWO, TWO, REL_L2_TOL)), ((512, 512, 512), (TWO, TWO, TWO))], ids=str)
+def test_accumulation_error_of_products(ctx, oracle, size, bars):
+    m, k, n = size
+    rng = np.random.default_rng(m)
+    a, b, g = (rng.standard_normal(v).astype(np.float32) for v in ((m, k), (k, n), (m, n)))
+    a64, b64, g64 = (v.astype(np.float64) for v in (a, b, g))
+    with DeviceArrays(ctx, a=a, b=b, g=g) as d:
+        d.alloc("c", m * n), d.alloc("da", m * k), d.alloc("db", k * n)
+        ctx.matmul_fwd(d["a"], d["b"], d["c"], m, k, n)
+        ctx.matmul_bwd(d["a"], d["b"], d["g"], d["da"], d["db"], m, k, n, 0)
+        errors = rel_l2(d.get("c"), a64 @ b64), rel_l2(d.get("da"), g64 @ b64.T), rel_l2(d.get("db"), a64.T @ g64)
+    assert all(e <= bar for e, bar in zip(errors, bars)), (errors, bars)
+
+
+@pytest.mark.parametrize("shape, bars", [((4, 35, 31, 25, 70, 5, 3, 2, 1), (ONE, ONE, FINE)), ((4, 3, 40, 40, 32, 5, 5, 1, 2), (FINE, TWO, FINE)),
+                                         ((2, 129, 14, 14, 67, 3, 3, 1, 1), (TWO, ONE, FINE)), ((4, 32, 32, 32, 64, 3, 3, 2, 1), (TWO, TWO, TWO)),
+                                         ((8, 96, 14, 14, 96, 1, 1, 1, 0), (TWO, TWO, TWO))], ids=str)
+def test_accumulation_error_of_layers(ctx, oracle, shape, bars):
+    n, c, h, w, k, r, s, stride, pad = shape
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    rng = np.random.default_rng(sum(shape))
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, n * k * oh * ow))
+    errors = conv_errors(ctx, oracle, shape, x, wt, g)
+    assert all(e <= bar for e, bar in zip(errors, bars)), (errors, bars)
