@@ -115,7 +115,7 @@ __device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d
         }
         return;
     }
-    const float floor = p.relu ? 0.f : -INFINITY;
+    const float floor = p.relu ? 0.f : NAN;  // max(v, NaN) is v; max(NaN, 0) is 0: a ReLU cuts a NaN off, as in every kernel
 #pragma unroll
     for (int i0 = 0; i0 < 32; i0 += 8) {
         float o[8];
@@ -131,7 +131,7 @@ __device__ __forceinline__ void store_columns(const KatsuF16Problem &p, float *d
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            if (o[i] < floor) o[i] = floor;  // (a NaN stays one)
+            o[i] = fmaxf(o[i], floor);
             if (valid && (all || i0 + i < live)) *d = o[i];
             d += stride;
         }

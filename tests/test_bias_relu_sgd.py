@@ -124,3 +124,20 @@ def test_c_abi_entry_points(ctx, oracle):
         before = d.get("w")
         ctx.call("katsu_cuda_sgd_step", d["w"], d["g"], 0.25, w.size)
         assert np.array_equal(d.get("w"), before - (np.float32(0.25) * g[:w.size]).astype(np.float32))
+
+
+# stem kernel, direct kernel, tensor-core product in one piece and in several that are folded
+@pytest.mark.parametrize("shape", [(2, 3, 16, 16, 16, 3, 3, 1, 1), (1, 5, 6, 6, 7, 3, 3, 1, 1), (16, 64, 20, 20, 64, 3, 3, 1, 1), (1, 512, 7, 7, 64, 3, 3, 1, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_relu_cuts_off_nan_in_every_kernel(ctx, shape):
+    """max(., 0) of a NaN is 0, whatever kernel and split the shape gets; the backward mask treats it as cut off."""
+    n, c, h, w, k, r, s, stride, pad = shape
+    rng = np.random.default_rng(sum(shape))
+    x, wt, b = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, k))
+    x[x.size // 2] = np.nan
+    with DeviceArrays(ctx, x=x, w=wt, b=b) as d:
+        d.alloc("plain", n * k * h * w), d.alloc("relu", n * k * h * w)
+        ctx.conv2d_fwd_staged(d["x"], None, d["w"], d["b"], d["plain"], *shape, 0)
+        ctx.conv2d_fwd_staged(d["x"], None, d["w"], d["b"], d["relu"], *shape, 1)
+        plain, relu = d.get("plain"), d.get("relu")
+    assert np.isnan(plain).any() and np.array_equal(relu, np.fmax(plain, 0))
