@@ -178,6 +178,20 @@ Classes classes_of(const Shape &g) {
     return q;
 }
 
+// Where results have to be summed again that meet an infinity or NaN and a product that is not theirs (f16_exact.cuh): for layers
+// that can run on the direct kernels, which have no such products, and where the classes of a strided dX share products.
+KatsuF16Raw raw_of(KatsuF16Raw::Form form, const float *a, const float *b, const Shape &g, bool shared, const float *gscale, float gfactor) {
+    KatsuF16Raw q = {};
+    q.form = shared || !regular(g) ? form : KatsuF16Raw::NONE;
+    q.a = a;
+    q.b = b;
+    q.n = (int)g.n; q.c = (int)g.c; q.h = (int)g.h; q.w = (int)g.w; q.k = (int)g.k; q.r = (int)g.r; q.s = (int)g.s;
+    q.stride = (int)g.stride; q.pad = (int)g.pad; q.oh = (int)g.oh; q.ow = (int)g.ow;
+    q.gscale = gscale;
+    q.gfactor = gfactor;
+    return q;
+}
+
 void pixel_fields(KatsuF16Problem *p, const Shape &g, const KatsuF16Box &box) {
     p->n_img = (int)g.n;
     p->gfactor = 1.f;
@@ -256,6 +270,7 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         KatsuF16Problem p = {};
         pixel_fields(&p, g, box);
         p.out = y;
+        p.raw = raw_of(KatsuF16Raw::FORWARD, x, w, g, false, nullptr, 1.f);
         p.bias = bias;
         p.relu = relu;
         p.call = call;
@@ -276,7 +291,7 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         p.img_stride = (long long)(k * oh * ow);
         KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_CONV, maps, p, plan, partial, (long long)out_count));
         if (plan.splits > 1)
-            KATSU_TRY(katsu_f16_fold(ctx, partial, y, out_count, plan.splits, 0, bias, k, oh * ow, relu));
+            KATSU_TRY(katsu_f16_fold(ctx, p.raw, partial, y, out_count, plan.splits, 0, bias, k, oh * ow, relu));
     }
     return KATSU_OK;
 }
@@ -286,7 +301,7 @@ namespace {
 // dw[k][c][ky][kx] (+)= sum over splits of partial[split][k][(ky, column group, column)].  A
 // block handles 32 elements in the partials' order, eight thread groups each add every eighth split.
 __global__ void __launch_bounds__(256)
-f16_dw_fold_kernel(const float *__restrict__ partial, float *dw, int k, int c, int r, int s, int cp, int groups_per_row, int splits, int accumulate) {
+f16_dw_fold_kernel(const __grid_constant__ KatsuF16Raw raw, const float *__restrict__ partial, float *dw, int k, int c, int r, int s, int cp, int groups_per_row, int splits, int accumulate) {
     __shared__ float sums[8][32];
     launch_next();
     launch_wait();
@@ -307,6 +322,7 @@ f16_dw_fold_kernel(const float *__restrict__ partial, float *dw, int k, int c, i
     const int ky = m / (groups_per_row * 64), col = m - ky * groups_per_row * 64;
     const int kx = col / cp, cc = col - kx * cp;
     if (kx >= s || cc >= c) return;
+    if (raw.form != KatsuF16Raw::NONE && !katsu_is_number(total) && katsu_f16_mixed(raw, ky, kx)) total = katsu_f16_exact(raw, o, cc, ky, kx);
     float *dst = dw + ((size_t(o) * c + cc) * r + ky) * s + kx;
     *dst = accumulate ? *dst + total : total;
 }
@@ -434,6 +450,8 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.call = call;
             p.info_a = ig;
             p.info_b = iw;
+            // (the last 16-wide step of a class of fewer taps reaches into the next pixel where kp is no multiple of 16)
+            p.raw = raw_of(KatsuF16Raw::DX, gr, w, g, merged || (stride > 1 && kp % 16 != 0), gscale, gfactor);
             p.gscale = gscale;
             p.gfactor = gfactor;
             p.m_total = box_dx.blocks * 128;
@@ -460,7 +478,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             p.img_stride = (long long)(c * h * wd);
             KATSU_TRY(katsu_f16_launch(ctx, stride == 2 ? KATSU_F16_CONV_DX2 : KATSU_F16_CONV, md, p, plan_dx, partial_dx, (long long)dx_count));
             if (plan_dx.splits > 1)
-                KATSU_TRY(katsu_f16_fold(ctx, partial_dx, dx, dx_count, plan_dx.splits, accumulate, nullptr, 1, 1, 0));
+                KATSU_TRY(katsu_f16_fold(ctx, p.raw, partial_dx, dx, dx_count, plan_dx.splits, accumulate, nullptr, 1, 1, 0));
         }
         if (dw) {
             KatsuF16Problem p = {};
@@ -485,7 +503,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
             KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_CONV_DW, mw, p, plan_dw, partial_dw, (long long)dw_count));
             KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)f16_dw_fold_kernel, 0));
             KATSU_TRY(katsu_launch_chained(ctx, f16_dw_fold_kernel, (unsigned)katsu_div_up(dw_count, (size_t)32), 256, 0, 1,
-                                           partial_dw, dw, (int)k, (int)c, (int)r, (int)s, (int)cp, (int)gpr, plan_dw.splits,
+                                           raw_of(KatsuF16Raw::DW, x, gr, g, false, gscale, gfactor), partial_dw, dw, (int)k, (int)c, (int)r, (int)s, (int)cp, (int)gpr, plan_dw.splits,
                                            accumulate));
         }
     }

@@ -166,6 +166,31 @@ __device__ __forceinline__ void store_pairs(const KatsuF16Problem &p, float *d, 
     }
 }
 
+// The mixed results (f16_exact.cuh) that this thread has stored, or left out (`left_out`), for the tile of its pixel (img, jy, jx).
+__device__ __noinline__ void repair_tile(const KatsuF16Problem &p, int img, int jy, int jx, int n0, int group, bool left_out) {
+    for (int py = 0; py < p.classes_y; ++py)
+        for (int px = 0; px < p.classes_x; ++px)
+            for (int i = 0; i < 128; ++i) {  // alternate 32-column chunks, as they are stored
+                const int col = n0 + ((i >> 5) * 2 + group) * 32 + (i & 31);
+                if (col >= n0 + p.bn) break;
+                int channel = col, y = p.step * jy + py, x = p.step * jx + px;
+                if (p.class_cols) {
+                    const int q = col / p.class_cols;
+                    if (q > 1) break;
+                    channel = (col - q * p.class_cols) >> 1;
+                    y += q;
+                    x += col & 1;
+                }
+                if (channel >= p.n_total || y >= p.out_h || x >= p.out_w || !katsu_f16_mixed(p.raw, y, x)) continue;
+                float *d = p.out + img * p.img_stride + (long long)y * p.out_w + x + channel * p.col_stride;
+                if (!left_out && katsu_is_number(*d)) continue;
+                float v = katsu_f16_exact(p.raw, img, channel, y, x);
+                if (p.bias) v += __ldg(p.bias + channel);
+                if (p.accumulate) v += *d;
+                *d = p.relu ? fmaxf(v, 0.f) : v;
+            }
+}
+
 template <int NARROW, KatsuF16Kind KIND>
 __global__ void __launch_bounds__(THREADS, 1)
 f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant__ KatsuF16Problem p) {
@@ -208,6 +233,10 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     const KatsuF16Info info_a = katsu_f16_load(p.info_a), info_b = katsu_f16_load(p.info_b);
     const bool wide = katsu_f16_wide(p.call);
     const int planes = NARROW + (wide ? 1 : 0);
+    // Mixed results are summed again (f16_exact.cuh).  What is added to, or ends in a ReLU, cannot be told from what it should be
+    // once it is stored, so such a call does not store them first.  Parts of a split contraction are looked at when they are folded.
+    const bool repairs = CONV && p.raw.form != KatsuF16Raw::NONE && p.splits == 1 && !(katsu_f16_finite(info_a) && katsu_f16_finite(info_b));
+    const bool left_out = repairs && (p.accumulate || p.relu);
     // k-blocks between two drains: in TF32 mode up to 12 288 accumulation steps (4e-4 of 2e-3)
     const int drain = NARROW == 2 ? (wide ? (p.drain + 1) / 2 : p.drain) : 1024;
     // accumulators that take turns; hand-over q is the one q & (2^acc_bits - 1), acc_cols columns apart
@@ -217,7 +246,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 
     if (warp == 8 && lane == 0) {
         // ---- TMA producer: this block's lanes of A and half of B's columns; bytes counted on the leader's barrier ----
-        const CUtensorMap *map_a = p.a_second && wide && katsu_f16_narrow(info_a, p.call.span) ? maps.a_second : maps.a, *map_b = maps.b;
+        const CUtensorMap *map_a = p.a_second && wide && katsu_f16_own_copy(p.call, info_a) ? maps.a_second : maps.a, *map_b = maps.b;
         bool ok = true;
         int s = 0;
         uint32_t phase = 1;  // a fresh barrier counts as released
@@ -404,7 +433,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
             const long long m = (2ll * t.mt + rank) * BM + quarter * 32 + lane;
             const int n0 = t.nt * p.bn;
             int img = 0, jy = 0, jx = 0;
-            bool in_box = true;
+            bool in_result = m < p.m_total;
             if (CONV) {
                 const int r = quarter * 32 + lane;
                 box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
@@ -412,7 +441,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                 jx += r - q1 * p.bw;
                 jy += q1 - q2 * p.bh;
                 img += q2;
-                in_box = q2 < p.nb && img < p.n_img;
+                in_result = in_result && q2 < p.nb && img < p.n_img && !(KIND == KATSU_F16_CONV_DX2 && left_out);
             }
             const bool pairs_of_x = KIND == KATSU_F16_CONV_DX2 && p.pair_x;
             float run[4][32];  // sums of the drains; of pairs: [0, 1], and in [2, 3] those of the class px = 0 before
@@ -420,13 +449,13 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                 for (int px = 0; px < p.classes_x && alive; ++px) {
                     int kb0, kb1;
                     k_range(p, class_kblocks<KIND>(p, py, px), t.split, &kb0, &kb1);
-                    const bool in_result = in_box && m < p.m_total;
                     bool valid = in_result;
                     long long at = m;
                     int y = 0, x = 0;
                     if (CONV) {
                         y = p.step * jy + py, x = p.step * jx + px;
                         valid = valid && y < p.out_h && x < p.out_w;
+                        if (KIND == KATSU_F16_CONV && left_out) valid = valid && !katsu_f16_mixed(p.raw, y, x);
                         at = img * p.img_stride + (long long)y * p.out_w + x;
                     }
                     float *dst = p.out + t.split * p.split_stride + at;
@@ -533,6 +562,17 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                 }
         }
     }
+    if (CONV && repairs && warp < 8) {
+        // (behind the pipeline: no wait of the other warps runs out meanwhile)
+        for (int item = pair; item < items; item += pairs) {
+            const Tile t = tile_of(item, p);
+            int img, jy, jx;
+            box_origin(p, 2ll * t.mt + rank, &img, &jy, &jx);
+            const int r = (warp & 3) * 32 + lane, q1 = r / p.bw, q2 = q1 / p.bh;
+            if (q2 < p.nb && img + q2 < p.n_img)
+                repair_tile(p, img + q2, jy + q1 - q2 * p.bh, jx + r - q1 * p.bw, t.nt * p.bn, warp >> 2, left_out);
+        }
+    }
     // Neither block leaves (or gives its tensor memory back) while the other may still signal its barriers,
     // read its half of B or hold accumulators: every path above ends here.
     tc_fence_before_sync();
@@ -542,13 +582,14 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
 }
 
 __global__ void __launch_bounds__(256)
-f16_fold_kernel(const float *__restrict__ partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels, size_t plane, int relu) {
+f16_fold_kernel(const __grid_constant__ KatsuF16Raw raw, const float *__restrict__ partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels, size_t plane, int relu) {
     launch_next();
     launch_wait();
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
         float s = 0.f;
 #pragma unroll 8
         for (int q = 0; q < splits; ++q) s += __ldg(partial + size_t(q) * count + i);
+        if (raw.form != KatsuF16Raw::NONE && !katsu_is_number(s)) s = katsu_f16_exact_element(raw, i, s);
         if (bias) s += __ldg(bias + (i / plane) % channels);
         if (relu) s = fmaxf(s, 0.f);
         out[i] = accumulate ? out[i] + s : s;
@@ -657,12 +698,12 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
     return launch<1, KATSU_F16_CONV_DW>(ctx, maps, p, pairs);
 }
 
-int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const float *partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels,
-                       size_t plane, int relu) {
+int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const KatsuF16Raw &raw, const float *partial, float *out, size_t count, int splits,
+                       int accumulate, const float *bias, size_t channels, size_t plane, int relu) {
     size_t blocks = katsu_div_up(count, (size_t)256);
     if (blocks > size_t(ctx->num_sms) * 8) blocks = size_t(ctx->num_sms) * 8;
     KATSU_TRY(katsu_prepare_kernel(ctx, (const void *)f16_fold_kernel, 0));
-    return katsu_launch_chained(ctx, f16_fold_kernel, (unsigned)blocks, 256, 0, 1, partial, out, count, splits, accumulate, bias,
+    return katsu_launch_chained(ctx, f16_fold_kernel, (unsigned)blocks, 256, 0, 1, raw, partial, out, count, splits, accumulate, bias,
                                 channels, plane, relu);
 }
 

@@ -3,6 +3,7 @@
 
 #include <cuda.h>
 
+#include "f16_exact.cuh"
 #include "f16_split.cuh"
 
 constexpr int KATSU_F16_MAX_ROWS = 49;    // filter rows over all y-parity classes
@@ -25,10 +26,11 @@ struct KatsuF16Problem {
     long long f32_terms;
     KatsuF16Call call;
     const KatsuF16Info *info_a, *info_b;
-    // A's planes come from the second set of maps when the call is wide and A's own copy, made before the call, is not
+    // A's planes come from the second set of maps when the copy made before the call is not one for it (katsu_f16_own_copy)
     int a_second;
     const float *gscale;  // device scalar or null, times gfactor
     float gfactor;
+    KatsuF16Raw raw;
     long long m_total;    // lanes: matrix rows, pixels of the grid, or dW rows
     int n_total;          // columns
     long long col_stride;
@@ -80,8 +82,8 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
                          const KatsuF16Plan &plan, float *partial, long long split_stride);
 
 // out[i] (+)= act(sum over splits of partial[split][i] + bias[(i / plane) % channels]).
-int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const float *partial, float *out, size_t count, int splits, int accumulate, const float *bias, size_t channels,
-                       size_t plane, int relu);
+int32_t katsu_f16_fold(katsu_cuda_ctx *ctx, const KatsuF16Raw &raw, const float *partial, float *out, size_t count, int splits,
+                       int accumulate, const float *bias, size_t channels, size_t plane, int relu);
 
 // Pixel boxes over a width x height x images grid: the factors of a box of at most `lanes` pixels (exactly `lanes`, in
 // powers of two, when `exact`) that waste the fewest lanes.

@@ -77,7 +77,7 @@ int32_t run(katsu_cuda_ctx *ctx, const KatsuF16Call &call, const Product &q, flo
     const size_t count = q.n_lanes * q.n_columns;
     KATSU_TRY(katsu_f16_launch(ctx, KATSU_F16_GEMM, maps, p, q.plan, partial, (long long)count));
     if (q.plan.splits > 1)
-        KATSU_TRY(katsu_f16_fold(ctx, partial, q.out, count, q.plan.splits, q.accumulate,
+        KATSU_TRY(katsu_f16_fold(ctx, p.raw, partial, q.out, count, q.plan.splits, q.accumulate,
                                  nullptr, 1, 1, 0));
     return KATSU_OK;
 }

@@ -22,6 +22,10 @@
 // TF32 mode), no scale.  bf16 has the exponents of f32, and three planes hold all 24 bits.  The products kept are
 // those down to 2^-16 (six; three in TF32 mode), at the cost of 3xTF32.  The choice is made on the device, by every
 // kernel of the call from the same KatsuF16Info values; no value crosses to the host.
+//
+// In a call with an infinity or NaN every plane but the last is cut strictly below the value, so that each part of a nonzero
+// value is nonzero and of its sign, and an infinity is one in every plane: its products with the other operand's parts are
+// then all the infinity of the product, where 0 * inf would be NaN.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -60,6 +64,21 @@ __device__ __forceinline__ bool katsu_f16_wide(const KatsuF16Call &call) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) v[i] = call.info[i] ? katsu_f16_load(call.info[i]) : KatsuF16Info{0, 0};
     return !(katsu_f16_narrow(v[0], call.span) && katsu_f16_narrow(v[1], call.span) && katsu_f16_narrow(v[2], call.span));
+}
+
+__device__ __forceinline__ bool katsu_f16_finite(KatsuF16Info info) { return info.most < 0x7f800000u; }
+__device__ __forceinline__ bool katsu_f16_finite(const KatsuF16Call &call) {
+    unsigned most = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (call.info[i]) most = max(most, katsu_f16_load(call.info[i]).most);
+    return most < 0x7f800000u;
+}
+
+// Whether a wide call needs planes of its own for an operand of which a copy has been made by itself: the copy holds fp16
+// planes, or planes that are not made to stand beside an infinity.
+__device__ __forceinline__ bool katsu_f16_own_copy(const KatsuF16Call &call, KatsuF16Info info) {
+    return katsu_f16_narrow(info, call.span) || (katsu_f16_finite(info) && !katsu_f16_finite(call));
 }
 
 // One operand whose magnitude is to be found: matrices [images][rows][cols], none of the sizes 0.
@@ -106,7 +125,7 @@ struct KatsuStageJob {
     KatsuF16Planes to;
     const KatsuF16Info *info;
     KatsuF16Info *info_copy;  // where to leave a copy of it, or null
-    int only_if_mixed;  // 1: written only when this operand is narrow and the call is not (a narrow copy exists already)
+    int only_if_mixed;  // 1: a copy of this operand exists already; written only when the call is wide and cannot use it
     int n, c, h, w, gap, cp, tail;
     int k, r, s, width, backward, classes, stride;
     int col_begin[8], kx_last[8], class_taps[8];

@@ -139,7 +139,7 @@ struct Writer {
     KatsuF16Planes to;
     float scale;
     int planes;  // planes of the form in use
-    bool wide;
+    bool wide, finite;
 };
 
 // Two scaled values as packed hi and lo halves.  Two values to a conversion: with one each, the conversion pipe and not
@@ -152,21 +152,21 @@ __device__ __forceinline__ void split_narrow(float a, float b, unsigned *hi, uns
     *lo = *reinterpret_cast<const unsigned *>(&l);
 }
 
-// The leading 8 significand bits of v as a bf16 pattern in the upper half of a word, and what is left of v.  An infinity
-// or NaN is its first plane alone.
-__device__ __forceinline__ unsigned peel(float *v) {
+// The leading 8 significand bits of v as a bf16 pattern in the upper half of a word, and what is left of v.  `below`: of the
+// largest value below v's.  An infinity or NaN is one in every plane.
+__device__ __forceinline__ unsigned peel(float *v, bool below) {
     unsigned bits = __float_as_uint(*v);
     if ((bits & 0x7f800000u) == 0x7f800000u) {
         if (bits & 0x007fffffu) bits |= 0x00400000u;  // a NaN stays one without its lower bits
-        *v = 0.f;
         return bits & 0xffff0000u;
     }
+    if (below && (bits & 0x7fffffffu) != 0) bits -= 1;
     bits &= 0xffff0000u;
     *v -= __uint_as_float(bits);
     return bits;
 }
 
-__device__ __forceinline__ unsigned peel2(float *a, float *b) { return (peel(a) >> 16) | peel(b); }
+__device__ __forceinline__ unsigned peel2(float *a, float *b, bool below) { return (peel(a, below) >> 16) | peel(b, below); }
 
 // Eight consecutive elements at `at` (16-byte aligned).
 __device__ __forceinline__ void write8(const Writer &w, size_t at, float (&v)[8]) {
@@ -180,11 +180,12 @@ __device__ __forceinline__ void write8(const Writer &w, size_t at, float (&v)[8]
         if (w.planes == 2) *reinterpret_cast<uint4 *>(w.to.base + w.to.stride + at) = lo;
     } else {
         for (int i = 0; i < w.planes; ++i) {
+            const bool below = !w.finite && i + 1 < w.planes;
             uint4 o;
-            o.x = peel2(&v[0], &v[1]);
-            o.y = peel2(&v[2], &v[3]);
-            o.z = peel2(&v[4], &v[5]);
-            o.w = peel2(&v[6], &v[7]);
+            o.x = peel2(&v[0], &v[1], below);
+            o.y = peel2(&v[2], &v[3], below);
+            o.z = peel2(&v[4], &v[5], below);
+            o.w = peel2(&v[6], &v[7], below);
             *reinterpret_cast<uint4 *>(w.to.base + i * w.to.stride + at) = o;
         }
     }
@@ -392,11 +393,12 @@ __global__ void __launch_bounds__(THREADS, STAGE_BLOCKS) stage_kernel(const __gr
     out.to = j.to;
     const KatsuF16Info own = katsu_f16_load(j.info);
     out.wide = katsu_f16_wide(p.call);
+    out.finite = katsu_f16_finite(p.call);
     out.planes = p.narrow_planes + (out.wide ? 1 : 0);
     out.scale = out.wide ? 1.f : __uint_as_float(unsigned(127 + katsu_f16_exp(own)) << 23);
     if (p.clear && blockIdx.x == 0 && threadIdx.x < KATSU_INFO_SLOTS) p.clear[threadIdx.x] = KatsuF16Info{0, 0};
     if (block == 0 && threadIdx.x == 0 && j.info_copy) *j.info_copy = own;
-    if (j.only_if_mixed && !(out.wide && katsu_f16_narrow(own, p.call.span))) return;
+    if (j.only_if_mixed && !(out.wide && katsu_f16_own_copy(p.call, own))) return;
     if (j.kind == KATSU_STAGE_NHWC) {
         if (block == 0) {
             // zero pixels in front of the first row, zeros behind the last

@@ -242,6 +242,113 @@ def test_non_finite_values_reach_exactly_their_outputs(ctx, oracle, mode):
     assert rel_l2(y[finite], y64[finite]) <= BARS[mode][1]
 
 
+def kinds(values):
+    """0 a number, 1 and 2 the infinities, 3 NaN."""
+    values = np.asarray(values).reshape(-1)
+    return np.where(np.isnan(values), 3, np.where(values == np.inf, 1, np.where(values == -np.inf, 2, 0)))
+
+
+# Strides 1 to 3 on both sides of 32 input channels, output channels that are and are not a multiple of 16 when rounded to 8;
+# layers of few or odd channels, whose padding and shared products must not show either; split and unsplit contractions
+NON_FINITE = [(2, 20, 24, 28, 40, 3, 3, 2, 1), (2, 40, 24, 28, 24, 3, 3, 2, 1), (2, 40, 25, 31, 40, 3, 3, 3, 1), (1, 40, 16, 18, 40, 4, 4, 2, 1),
+              (2, 24, 24, 26, 40, 1, 1, 2, 0), (1, 64, 30, 30, 64, 3, 3, 1, 1), (3, 17, 22, 24, 23, 3, 3, 1, 1), (3, 17, 32, 34, 23, 3, 3, 2, 1),
+              (2, 3, 20, 22, 24, 5, 5, 2, 2), (2, 150, 9, 9, 75, 3, 3, 1, 1), (16, 33, 28, 28, 50, 3, 3, 1, 0)]
+
+
+@pytest.mark.parametrize("shape", NON_FINITE, ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("mode", [0, 1], ids=["3xtf32", "tf32"])
+def test_infinities_and_nans_reach_exactly_their_results(ctx, oracle, mode, shape):
+    """As f32 multiply-adds over a result's own terms have them.  Regular layers (channels from 16 on in multiples of 4) are held
+    to that for an x or g that is no number; in padded rows and columns a weight that is none reaches their results as NaN."""
+    n, c, h, w, k, r, s, stride, pad = shape
+    xs, ws = [n, c, h, w], [k, c, r, s]
+    oh, ow = oracle.conv_out_dims(h, w, r, s, stride, pad)
+    regular = c >= 16 and k >= 16 and c % 4 == 0 and k % 4 == 0
+    rng = np.random.default_rng(sum(shape))
+    whole = {name: np.rint(rng.standard_normal(v) * 4).astype(np.float32) + np.float32(0.5)  # few bits, no zero
+             for name, v in (("x", n * c * h * w), ("w", k * c * r * s), ("g", n * k * oh * ow))}
+    bias = rng.standard_normal(k).astype(np.float32)
+    ctx.set_precision(mode)
+    try:
+        for which in "xwg":
+            for value in (np.inf, np.nan, None):
+                t = {name: v.copy() for name, v in whole.items()}
+                if value is None:
+                    t[which][t[which].size // 3], t[which][-1] = np.inf, -np.inf
+                else:
+                    t[which][t[which].size // 3] = value
+                with np.errstate(all="ignore"):
+                    y = oracle.conv2d_forward_f64(t["x"], t["w"], xs, ws, stride, pad).reshape(-1)
+                    dx, dw = (v.reshape(-1) for v in oracle.conv2d_backward_f64(t["x"], t["w"], t["g"], xs, ws, stride, pad))
+                    by_channel = np.repeat(np.tile(bias, n), oh * ow)
+                    relu = np.fmax(y + by_channel, 0)  # (a NaN is cut off)
+                with DeviceArrays(ctx, x=t["x"], w=t["w"], g=t["g"], b=bias, dx2=np.ones(dx.size, np.float32), dw2=np.ones(dw.size, np.float32)) as d:
+                    for name, size in (("y", y.size), ("relu", y.size), ("dx", dx.size), ("dw", dw.size)):
+                        d.alloc(name, size, fill=7.0)
+                    ctx.conv2d_fwd(d["x"], d["w"], d["y"], *shape)
+                    ctx.conv2d_fwd_staged(d["x"], None, d["w"], d["b"], d["relu"], *shape, 1)
+                    ctx.conv2d_bwd(d["x"], d["w"], d["g"], d["dx"], d["dw"], *shape, 0)
+                    ctx.conv2d_bwd(d["x"], d["w"], d["g"], d["dx2"], d["dw2"], *shape, 1)
+                    results = [("y", y), ("relu", relu), ("dx", dx), ("dx2", dx + 1), ("dw", dw), ("dw2", dw + 1)]
+                    if regular:
+                        results = {"x": results[:2], "w": [], "g": results[2:4]}[which]
+                    for name, want in results:
+                        got = d.get(name)
+                        assert np.array_equal(kinds(got), kinds(want)), (name, which, value)
+                        numbers = np.isfinite(want)
+                        assert rel_l2(got[numbers], want[numbers]) <= BARS[mode][1], (name, which, value)
+    finally:
+        ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("size", [(200, 520, 648), (401, 333, 517), (260, 6000, 260)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("mode", [0, 1], ids=["3xtf32", "tf32"])
+def test_infinities_and_nans_in_matrices(ctx, oracle, mode, size):
+    m, k, n = size
+    rng = np.random.default_rng(m)
+    whole = [np.rint(rng.standard_normal(v) * 4).astype(np.float32) + np.float32(0.5) for v in ((m, k), (k, n), (m, n))]
+    ctx.set_precision(mode)
+    try:
+        for which in range(3):
+            for value in (np.inf, np.nan):
+                operands = [v.copy() for v in whole]
+                operands[which].reshape(-1)[1234] = value
+                a, b, g = operands
+                with np.errstate(all="ignore"):
+                    want = [v.reshape(-1) for v in (oracle.matmul_f64(a, b, m, k, n), *oracle.matmul_backward_f64(a, b, g, m, k, n))]
+                with DeviceArrays(ctx, a=a, b=b, g=g) as d:
+                    d.alloc("c", m * n), d.alloc("da", m * k), d.alloc("db", k * n)
+                    ctx.matmul_fwd(d["a"], d["b"], d["c"], m, k, n)
+                    ctx.matmul_bwd(d["a"], d["b"], d["g"], d["da"], d["db"], m, k, n, 0)
+                    for name, w in zip(("c", "da", "db"), want):
+                        assert np.array_equal(kinds(d.get(name)), kinds(w)), (name, which, value)
+    finally:
+        ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("mode", [0, 1], ids=["3xtf32", "tf32"])
+def test_a_held_copy_beside_an_infinite_weight(ctx, oracle, mode):
+    """x's copy, fp16 or bf16 planes, was made before the call and knows nothing of w: the call makes planes of its own."""
+    shape = (2, 32, 12, 14, 40, 3, 3, 1, 0)
+    n, c, h, w, k, r, s, stride, pad = shape
+    rng = np.random.default_rng(8)
+    x, wt = (np.rint(rng.standard_normal(v) * 4).astype(np.float32) + np.float32(0.5) for v in (n * c * h * w, k * c * 9))
+    wt[700] = np.inf
+    ctx.set_precision(mode)
+    try:
+        for scale in (1.0, 2.0 ** -60):
+            x[:x.size // n] *= np.float32(scale)
+            with np.errstate(all="ignore"):
+                want = oracle.conv2d_forward_f64(x, wt, [n, c, h, w], [k, c, 3, 3], 1, 0).reshape(-1)
+            with DeviceArrays(ctx, x=x, w=wt) as d:
+                d.alloc("y", want.size), d.alloc("copy", ctx.conv2d_staged_floats(*shape))
+                ctx.conv2d_stage(d["x"], d["copy"], n, c, h, w)
+                ctx.conv2d_fwd_staged(d["x"], d["copy"], d["w"], None, d["y"], *shape, 0)
+                assert np.array_equal(kinds(d.get("y")), kinds(want)), scale
+    finally:
+        ctx.set_precision(0)
+
+
 @pytest.mark.parametrize("shape", [(1, 16, 8, 8, 16, 3, 3, 1, 1), (1, 16, 14, 14, 24, 3, 3, 1, 1), (2, 24, 13, 13, 32, 3, 3, 2, 1)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_small_regular_layers_stay_on_the_tensor_cores(ctx, oracle, shape):
