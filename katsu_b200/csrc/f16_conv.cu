@@ -283,7 +283,7 @@ int32_t katsu_f16_conv_fwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
         p.col_stride = (long long)(oh * ow);
         p.row_begin[1] = (int)r;
         for (size_t i = 0; i < r; ++i) p.off_h[i] = p.b_row[i] = (short)i;
-        p.chunks[0] = (short)chunks;
+        p.chunks[0] = (int)chunks;
         p.steps_last[0] = (short)katsu_div_up(width - 64 * (chunks - 1), 16);
         p.in_step = (int)stride;
         p.lower_h = -(int)pad;
@@ -363,7 +363,7 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
     for (size_t i = 0; i < (merged ? 1 : stride); ++i) {
         const int cols = (merged ? q.span_x : q.taps_x[i]) * (int)kp;
         pd.b_col[i] = width;
-        pd.chunks[i] = (short)((cols + 63) / 64);
+        pd.chunks[i] = (cols + 63) / 64;
         pd.steps_last[i] = (short)((cols - 64 * (pd.chunks[i] - 1) + 15) / 16);
         pd.off_w[i] = merged ? 0 : (short)(q.off_x[i] - q.first_x);
         width += pd.chunks[i] * 64;

@@ -39,8 +39,8 @@ struct KatsuF16Problem {
     int classes_y, classes_x;
     int row_begin[KATSU_F16_MAX_CLASSES + 1];
     short off_h[KATSU_F16_MAX_ROWS], b_row[KATSU_F16_MAX_ROWS];
-    short off_w[KATSU_F16_MAX_CLASSES], chunks[KATSU_F16_MAX_CLASSES], steps_last[KATSU_F16_MAX_CLASSES];
-    int b_col[KATSU_F16_MAX_CLASSES];
+    short off_w[KATSU_F16_MAX_CLASSES], steps_last[KATSU_F16_MAX_CLASSES];
+    int chunks[KATSU_F16_MAX_CLASSES], b_col[KATSU_F16_MAX_CLASSES];
     int gemm_chunks;  // GEMM: k-blocks of the contraction (its chunks[0])
     // ---- pixels (conv kinds), in boxes of bw x bh pixels of nb images: box b is (b % blocks_x, b / blocks_x % blocks_y,
     // rest).  CONV: one box is the 128 lanes of a block (bw * bh * nb <= 128); grid pixel (jy, jx) reads operand rows

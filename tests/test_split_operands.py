@@ -396,3 +396,20 @@ def test_accumulation_error_of_layers(ctx, oracle, shape, bars):
     x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (n * c * h * w, k * c * r * s, n * k * oh * ow))
     errors = conv_errors(ctx, oracle, shape, x, wt, g)
     assert all(e <= bar for e, bar in zip(errors, bars)), (errors, bars)
+
+
+@pytest.mark.parametrize("c, s", [(65536, 32), (65536, 64)])
+def test_filter_rows_of_millions_of_products(ctx, c, s):
+    """32 768 and 65 536 k-blocks to a filter row: the largest that the path takes, past what 16 bits count."""
+    k = 2
+    shape = (1, c, 1, s, k, 1, s, 1, 0)
+    rng = np.random.default_rng(c + s)
+    x, wt, g = (rng.standard_normal(v).astype(np.float32) for v in (c * s, k * c * s, k))
+    x64, w64, g64 = x.astype(np.float64), wt.astype(np.float64).reshape(k, -1), g.astype(np.float64)
+    with DeviceArrays(ctx, x=x, w=wt, g=g) as d:
+        d.alloc("y", k, fill=np.nan), d.alloc("dx", x.size, fill=np.nan), d.alloc("dw", wt.size, fill=np.nan)
+        ctx.conv2d_fwd(d["x"], d["w"], d["y"], *shape)
+        ctx.conv2d_bwd(d["x"], d["w"], d["g"], d["dx"], d["dw"], *shape, 0)
+        assert rel_l2(d.get("y"), w64 @ x64) <= REL_L2_TOL
+        assert rel_l2(d.get("dx"), g64 @ w64) <= REL_L2_TOL
+        assert rel_l2(d.get("dw"), np.outer(g64, x64)) <= REL_L2_TOL
