@@ -414,7 +414,9 @@ int32_t katsu_f16_conv_bwd(katsu_cuda_ctx *ctx, const float *x, const float *w, 
                                           plan_dw.bn >= 128 ? 64 : 32, box_dw, b_pairs)))
             return katsu_f16_drop_call(ctx);
         *handled = 1;
-        const KatsuF16Call call = katsu_f16_call(ctx, ig, dx ? iw : nullptr, dw ? info : nullptr);
+        KatsuF16Call call = katsu_f16_call(ctx, ig, dx ? iw : nullptr, dw ? info : nullptr);
+        call.gscale = gscale;
+        call.gfactor = gfactor;
         KatsuAmaxJob amax[3];
         KatsuStageJob jobs[3];
         int na = 0, nj = 0;

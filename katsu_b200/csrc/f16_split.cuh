@@ -42,6 +42,9 @@ struct KatsuF16Info {
 struct KatsuF16Call {
     const KatsuF16Info *info[3];
     int span;
+    // factors of the results, of a call whose first operand meets the others
+    const float *gscale;  // device scalar or null
+    float gfactor;
 };
 
 // 2^-48 .. 2^48 keeps the product of two operands' scales inside f32.
@@ -63,7 +66,12 @@ __device__ __forceinline__ bool katsu_f16_wide(const KatsuF16Call &call) {
     KatsuF16Info v[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) v[i] = call.info[i] ? katsu_f16_load(call.info[i]) : KatsuF16Info{0, 0};
-    return !(katsu_f16_narrow(v[0], call.span) && katsu_f16_narrow(v[1], call.span) && katsu_f16_narrow(v[2], call.span));
+    if (!(katsu_f16_narrow(v[0], call.span) && katsu_f16_narrow(v[1], call.span) && katsu_f16_narrow(v[2], call.span))) return true;
+    if (call.gscale == nullptr && call.gfactor == 1.f) return false;
+    // The sums are multiplied by the factors and the operands' scales as one f32, which has to be a normal number.
+    const float factor = call.gscale ? call.gfactor * __ldg(call.gscale) : call.gfactor;
+    const int e = int((__float_as_uint(factor) >> 23) & 255) - 127, e0 = katsu_f16_exp(v[0]), e1 = katsu_f16_exp(v[1]), e2 = katsu_f16_exp(v[2]);
+    return e - e0 - max(e1, e2) < -100 || e - e0 - min(e1, e2) > 100;
 }
 
 __device__ __forceinline__ bool katsu_f16_finite(KatsuF16Info info) { return info.most < 0x7f800000u; }

@@ -441,7 +441,7 @@ int32_t katsu_f16_drop_call(katsu_cuda_ctx *ctx) {
 KatsuF16Info *katsu_f16_slot(katsu_cuda_ctx *ctx, int slot) { return slots(ctx, ctx->f16_captured ? 2 : ctx->f16_set) + slot; }
 
 KatsuF16Call katsu_f16_call(const katsu_cuda_ctx *ctx, const KatsuF16Info *a, const KatsuF16Info *b, const KatsuF16Info *c) {
-    return KatsuF16Call{{a, b, c}, ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28};
+    return KatsuF16Call{{a, b, c}, ctx->precision == KATSU_MODE_3XTF32 ? 17 : 28, nullptr, 1.f};
 }
 
 int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count) {

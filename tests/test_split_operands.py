@@ -413,3 +413,19 @@ def test_filter_rows_of_millions_of_products(ctx, c, s):
         assert rel_l2(d.get("y"), w64 @ x64) <= REL_L2_TOL
         assert rel_l2(d.get("dx"), g64 @ w64) <= REL_L2_TOL
         assert rel_l2(d.get("dw"), np.outer(g64, x64)) <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("factor", [1e-3, 1.0, 1e6])
+def test_upstream_factor_beside_tiny_operands(ctx, oracle, factor):
+    """Operand scales of 2^61 and a factor below 1: their product is no normal f32 although the results are."""
+    shape = (2, 32, 14, 14, 40, 3, 3, 1, 1)
+    n, c, h, w, k, r, s, stride, pad = shape
+    rng = np.random.default_rng(3)
+    x, wt, g = ((rng.standard_normal(v) * 1.2e-15).astype(np.float32) for v in (n * c * h * w, k * c * 9, n * k * h * w))
+    dx64, dw64 = oracle.conv2d_backward_f64(x, wt, g, [n, c, h, w], [k, c, 3, 3], stride, pad)
+    scale = 0.75 * factor
+    with DeviceArrays(ctx, x=x, w=wt, g=g, scale=np.array([0.75], np.float32)) as d:
+        d.alloc("dx", x.size), d.alloc("dw", wt.size)
+        ctx.conv2d_bwd_staged(d["x"], None, d["w"], d["g"], d["scale"], factor, d["dx"], d["dw"], *shape, 0)
+        assert rel_l2(d.get("dx") / 1e-30, dx64 * scale / 1e-30) <= REL_L2_TOL
+        assert rel_l2(d.get("dw") / 1e-30, dw64 * scale / 1e-30) <= REL_L2_TOL
