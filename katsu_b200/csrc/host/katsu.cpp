@@ -229,6 +229,17 @@ struct TensorNode {
         }
         return grad_dev;
     }
+
+    // The same as a buffer that no other node holds (Adjoint::share), to be written to.
+    float *own_grad() const {
+        dense_grad();
+        if (grad_dev.use_count() > 1) {
+            auto own = uninit_buffer(numel);
+            if (numel) check(katsu_cuda_d2d(device_context(), own->ptr, grad_dev->ptr, numel));
+            grad_dev = std::move(own);
+        }
+        return grad_dev->ptr;
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -344,7 +355,8 @@ const Tensor &Tensor::to_host() const {
 }
 
 const float *Tensor::device_data() const { return node_->device(); }
-const float *Tensor::device_grad() const { return node_->has_grad() ? node_->dense_grad()->ptr : nullptr; }
+// (the caller may write through the address: clipping, an all-reduce)
+const float *Tensor::device_grad() const { return node_->has_grad() ? node_->own_grad() : nullptr; }
 
 Tensor Tensor::make_lazy_square(const Tensor &parent) {
     auto node = std::make_shared<TensorNode>();
@@ -662,13 +674,7 @@ void Tensor::backward_with(const std::vector<float> &seed) const {
         if (n.has_grad()) {
             // tensor.rs:353-356: old += new, element by element
             const float *add = adjoint.to_dense();
-            n.dense_grad();
-            if (n.grad_dev.use_count() > 1) {  // another node's gradient is the same buffer (Adjoint::share)
-                auto own = uninit_buffer(n.numel);
-                if (n.numel) check(katsu_cuda_d2d(ctx, own->ptr, n.grad_dev->ptr, n.numel));
-                n.grad_dev = std::move(own);
-            }
-            check(katsu_cuda_axpy_acc(ctx, n.grad_dev->ptr, add, n.numel));
+            check(katsu_cuda_axpy_acc(ctx, n.own_grad(), add, n.numel));
         } else if (adjoint.kind == Adjoint::Dense) {
             adjoint.to_dense();  // a node nothing contributed to still gets Some(zeros)
             n.grad_dev = std::move(adjoint.dense);  // tensor.rs:357-359: the adjoint buffer becomes the gradient

@@ -35,3 +35,30 @@ def test_gradients_are_independent(oracle, backwards):
         assert np.array_equal(np.asarray(dev[name].grad()).reshape(-1), np.asarray(want).reshape(-1)), name
     dev["v"].zero_grad()
     assert dev["v"].grad() is None and dev["u"].grad() is not None
+
+
+def test_a_gradient_changed_in_place_is_one_tensors_own():
+    """A caller that scales or reduces gradients through their device addresses must not reach another tensor's, nor the seed of
+    later backward passes."""
+    import katsu_b200 as K
+    from katsu_b200 import cabi
+
+    def overwrite(tensor, value):
+        address = tensor.device_grad()
+        K.synchronize()
+        with cabi.Context(0) as context:
+            context.h2d(address, np.full(tensor.numel(), value, np.float32))
+            context.sync()
+
+    values = np.arange(12, dtype=np.float32)
+    a, b = K.Tensor(values, [3, 4]), K.Tensor(values + 1, [3, 4])
+    total = a.add(b)
+    loss = total.sum()
+    loss.backward()
+    overwrite(a, 7.0), overwrite(loss, 5.0)
+    assert (np.asarray(a.grad()) == 7).all() and (np.asarray(loss.grad()) == 5).all()
+    assert (np.asarray(b.grad()) == 1).all() and (np.asarray(total.grad()) == 1).all()
+    for t in (a, b, total, loss):
+        t.zero_grad()
+    loss.backward()
+    assert (np.asarray(a.grad()) == 1).all() and (np.asarray(loss.grad()) == 1).all()
