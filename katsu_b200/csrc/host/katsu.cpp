@@ -375,6 +375,7 @@ void Tensor::sgd_step(float lr) const {
     float *values = const_cast<float *>(node_->device());
     if (numel()) check(katsu_cuda_sgd_step(device_context(), values, gradient, lr, numel()));
     node_->host_valid = false;  // the host mirror is refilled from the device on the next data()
+    node_->staged.reset();      // as is the copy for convolutions, by the next one
 }
 
 // tensor.rs:226-240

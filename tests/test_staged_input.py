@@ -70,6 +70,21 @@ def test_a_pointer_given_with_a_shape_that_has_no_copy_is_not_read(ctx, oracle, 
         assert np.array_equal(d.get("y"), d.get("y2")) and np.array_equal(d.get("dw"), d.get("dw2"))
 
 
+def test_an_input_changed_by_a_step_is_staged_again(oracle):
+    """The graph keeps the copy on the input's node; sgd_step changes the values in place."""
+    import katsu_b200 as K
+
+    rng = np.random.default_rng(4)
+    x, w = rng.standard_normal(2 * 16 * 10 * 10).astype(np.float32), rng.standard_normal(16 * 16 * 9).astype(np.float32)
+    xt, wt = K.Tensor(x, [2, 16, 10, 10]), K.Tensor(w, [16, 16, 3, 3])
+    layer = K.Conv2D.from_weights(wt, 1, 1)
+    layer.forward(xt).sum().backward()
+    xt.sgd_step(0.5)
+    after = np.asarray(layer.forward(xt).data())
+    fresh = K.Conv2D.from_weights(wt, 1, 1).forward(K.Tensor(np.asarray(xt.data()), [2, 16, 10, 10]))
+    assert np.array_equal(after, np.asarray(fresh.data())) and not np.array_equal(np.asarray(xt.data()), x)
+
+
 def test_shapes_that_stage_nothing_report_zero(ctx):
     assert ctx.conv2d_staged_floats(4, 3, 32, 32, 16, 3, 3, 1, 1) == 0     # stem kernels
     assert ctx.conv2d_staged_floats(2, 7, 13, 11, 9, 3, 3, 1, 1) == 0      # direct kernels
