@@ -18,7 +18,9 @@ constexpr int AMAX_ROWS = 16;    // rows of a strip at most
 
 struct AmaxSegment {
     KatsuAmaxJob job;
-    unsigned strips, strip_rows, col_tiles;  // of a matrix
+    // Of a matrix.  The first `longer` strips have strip_rows + 1 rows, the others strip_rows: no strip of a row or two at the
+    // end, whose elements would be groups by themselves.
+    unsigned strips, strip_rows, longer, col_tiles;
     unsigned first_block, blocks;
     int vec;  // 128 columns to a tile, a float4 to a lane; else 32
 };
@@ -75,7 +77,8 @@ __device__ __forceinline__ void amax_tiles(const AmaxSegment &sg, unsigned first
         const unsigned long long rest = (left - 1) / sg.col_tiles;
         const unsigned tile = unsigned(left - 1 - rest * sg.col_tiles);
         const unsigned long long image = rest / sg.strips;
-        const unsigned row = unsigned(rest - image * sg.strips) * sg.strip_rows, rows = min(sg.strip_rows, j.rows - row);
+        const unsigned strip = unsigned(rest - image * sg.strips);
+        const unsigned row = strip * sg.strip_rows + min(strip, sg.longer), rows = sg.strip_rows + (strip < sg.longer ? 1 : 0);
         // the last tile reaches back so that it is a full one; lanes past a narrow row read its last columns again
         unsigned col = tile * (32 * W);
         if (col + 32 * W > j.cols) col = j.cols > 32 * W ? j.cols - 32 * W : 0;
@@ -453,8 +456,8 @@ int32_t katsu_f16_amax(katsu_cuda_ctx *ctx, const KatsuAmaxJob *jobs, int count)
         s.job = jobs[i];
         s.vec = (jobs[i].cols & 3) == 0 && (reinterpret_cast<uintptr_t>(jobs[i].src) & 15u) == 0;
         s.strips = (jobs[i].rows + AMAX_ROWS - 1) / AMAX_ROWS;
-        s.strip_rows = (jobs[i].rows + s.strips - 1) / s.strips;  // even strips: no group of a row or two at the end
-        s.strips = (jobs[i].rows + s.strip_rows - 1) / s.strip_rows;
+        s.strip_rows = jobs[i].rows / s.strips;
+        s.longer = jobs[i].rows % s.strips;
         s.col_tiles = (jobs[i].cols + (s.vec ? 127 : 31)) / (s.vec ? 128 : 32);
         size_t blocks = katsu_div_up(size_t(jobs[i].images) * s.strips * s.col_tiles, (size_t)(THREADS / 32));
         if (blocks > size_t(ctx->num_sms) * AMAX_BLOCKS) blocks = size_t(ctx->num_sms) * AMAX_BLOCKS;
