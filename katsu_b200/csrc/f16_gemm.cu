@@ -240,7 +240,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     // k-blocks between two drains: in TF32 mode up to 12 288 accumulation steps (4e-4 of 2e-3)
     const int drain = NARROW == 2 ? (wide ? (p.drain + 1) / 2 : p.drain) : 1024;
     // accumulators that take turns; hand-over q is the one q & (2^acc_bits - 1), acc_cols columns apart
-    const int acc_bits = p.bn <= 128 ? 2 : 1, acc_mask = (1 << acc_bits) - 1, acc_cols = 512 >> acc_bits;
+    const int acc_bits = NARROW == 2 && p.bn <= 128 ? 2 : 1, acc_mask = (1 << acc_bits) - 1, acc_cols = 512 >> acc_bits;
     const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
     const int stages = min(MAX_STAGES, SMEM_RING / stage_bytes);
 
@@ -361,7 +361,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                         tc_fence_after_sync();
                         const uint32_t acc = tmem_base + uint32_t(b * acc_cols);
                         const int kb_end = min(kb + drain, kb1);
-                        bool add = false;
+                        bool first = true;
                         for (; kb < kb_end; ++kb) {
                             if (!mbar_wait_warp_ready(&full[s], phase, p.status, 173)) { ok = false; break; }
                             tc_fence_after_sync();
@@ -371,23 +371,22 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             const uint64_t b0 = smem_desc(st + b_off, lbo, b_sbo, b_layout);
                             const int steps = (!MN && chunk == chunks - 1) ? last : BK / 16;
                             if (issue) {
-                                // plane pa of A times plane pb of B, all steps of the k-block
-                                auto product = [&](uint32_t pa, uint32_t pb) {
-                                    const uint64_t ap = a0 + pa * (A_BYTES >> 4), bp = b0 + pb * (uint32_t(b_bytes) >> 4);
-#pragma unroll
-                                    for (int j = 0; j < BK / 16; ++j) {
-                                        if (j < steps) {
-                                            mma_f16_pair(acc, ap + j * (a_step >> 4), bp + j * (b_step >> 4), idesc, add);
-                                            add = true;
-                                        }
-                                    }
-                                };
-                                if (NARROW == 2 && wide) {
-                                    product(2, 0);
-                                    product(1, 1);
-                                    product(0, 2);
-                                }
+                                const uint32_t na = A_BYTES >> 4, nb = b_bytes >> 4;  // to the next plane
                                 if (NARROW == 2 && p.fine) {
+                                    // plane pa of A times plane pb of B, all steps of the k-block
+                                    auto product = [&](uint32_t pa, uint32_t pb) {
+#pragma unroll
+                                        for (int j = 0; j < BK / 16; ++j)
+                                            if (j < steps) {
+                                                mma_f16_pair(acc, a0 + pa * na + j * (a_step >> 4), b0 + pb * nb + j * (b_step >> 4), idesc, !first);
+                                                first = false;
+                                            }
+                                    };
+                                    if (wide) {
+                                        product(2, 0);
+                                        product(1, 1);
+                                        product(0, 2);
+                                    }
                                     product(1, 0);
                                     product(0, 1);
                                     product(0, 0);
@@ -396,12 +395,23 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                                     for (int j = 0; j < BK / 16; ++j) {
                                         if (j < steps) {
                                             const uint64_t ad = a0 + j * (a_step >> 4), bd = b0 + j * (b_step >> 4);
-                                            if (NARROW == 2 || wide) {
-                                                mma_f16_pair(acc, ad + (A_BYTES >> 4), bd, idesc, add);
-                                                mma_f16_pair(acc, ad, bd + (uint32_t(b_bytes) >> 4), idesc, true);
+                                            const bool add = !(first && j == 0);
+                                            if (NARROW == 2) {
+                                                if (wide) {
+                                                    mma_f16_pair(acc, ad + 2 * na, bd, idesc, add);
+                                                    mma_f16_pair(acc, ad + na, bd + nb, idesc, true);
+                                                    mma_f16_pair(acc, ad, bd + 2 * nb, idesc, true);
+                                                }
+                                                mma_f16_pair(acc, ad + na, bd, idesc, add || wide);
+                                                mma_f16_pair(acc, ad, bd + nb, idesc, true);
+                                                mma_f16_pair(acc, ad, bd, idesc, true);
+                                            } else {
+                                                if (wide) {
+                                                    mma_f16_pair(acc, ad + na, bd, idesc, add);
+                                                    mma_f16_pair(acc, ad, bd + nb, idesc, true);
+                                                }
+                                                mma_f16_pair(acc, ad, bd, idesc, add || wide);
                                             }
-                                            mma_f16_pair(acc, ad, bd, idesc, add || NARROW == 2 || wide);
-                                            add = true;
                                         }
                                     }
                                 }
@@ -410,6 +420,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                                 mma_commit_both(&empty[s]);
                             }
                             __syncwarp();
+                            first = false;
                             if (!MN && ++chunk == chunks) chunk = 0;
                             if (++s == stages) {
                                 s = 0;
@@ -534,12 +545,12 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                             if (2 * c + group < col_chunks) {
                                 float v[32];
                                 tmem_ld_32x32(acc + (2 * c + group) * 32, v);
-                                if (2 * c + group + 2 >= col_chunks) release_acc(q & acc_mask);
+                                if (NARROW == 2 && 2 * c + group + 2 >= col_chunks) release_acc(q & acc_mask);
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) run[c][i] += v[i];
                             }
                         }
-                        if (group >= col_chunks) release_acc(q & acc_mask);
+                        if (NARROW == 1 || group >= col_chunks) release_acc(q & acc_mask);
                     }
                     if (!alive) break;
                     if (pairs_of_x) {
