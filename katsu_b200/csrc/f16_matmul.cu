@@ -12,9 +12,9 @@ namespace {
 
 // Multiply-adds from which the path, three to six launches, pays against gemm_small_kernel on the CUDA cores.  Forward / both
 // gradients in us, here against there: 3xTF32 mode 17.2 / 23.8 against 12.3 / 25.3 at 256 x 512 x 256 (3.4e7), 18.1 / 27.7
-// against 21.3 / 42.1 at 512 x 512 x 256 (6.7e7); TF32 mode 13.8 / 20.2 against 8.0 / 16.0 at 256^3 (1.7e7), 14.5 / 21.1
-// against 14.5 / 30.1 at 320^3 (3.3e7).
-double least_macs(const katsu_cuda_ctx *ctx) { return ctx->precision == KATSU_MODE_3XTF32 ? 4e7 : 3e7; }
+// against 21.3 / 42.1 at 512 x 512 x 256 (6.7e7).  In TF32 mode the times would meet at 3e7 (13.8 / 20.2 against 8.0 / 16.0 at
+// 256^3, 14.5 / 21.1 against 14.5 / 30.1 at 320^3); the line stays at the smallest products that have had 11-bit parts there.
+double least_macs(const katsu_cuda_ctx *ctx) { return ctx->precision == KATSU_MODE_3XTF32 ? 4e7 : 1.5e7; }
 
 bool takes(const katsu_cuda_ctx *ctx, size_t m, size_t k, size_t n) {
     if (ctx->precision == KATSU_MODE_FP32 || ctx->f16_state == nullptr) return false;
