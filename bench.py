@@ -322,21 +322,13 @@ class Job:
             self.dist.destroy_process_group()
 
 
-def tf32_peaks():
-    """TF32 tensor-pipe denominators, TFLOP/s: half the driver-measured dense bf16 rate, and the rate
-    this library's own MMA-issue probe reached on this part (N = 256 tiles)."""
-    _, bf16_peak, kind = measured_peaks()
-    return bf16_peak / 2, 1105.0, kind
-
-
 def tensor_roofline(useful_tflops, passes):
-    half_bf16, direct, kind = tf32_peaks()
+    """The products run on 16-bit operands (fp16 planes): the driver-measured dense bf16 rate is their pipe's."""
+    _, peak, kind = measured_peaks()
     issued = useful_tflops * passes
-    return {"bound": "tensor", "achieved": issued, "peak": half_bf16, "unit": "TFLOP/s", "frac": issued / half_bf16,
-            "useful_tflops": useful_tflops, "issued_tflops": issued, "useful_frac": useful_tflops / half_bf16,
-            "peak_source": f"dense bf16 of {kind} / 2", "traffic": None,
-            "vs_direct_tf32_peak": {"peak": direct, "frac": issued / direct, "useful_frac": useful_tflops / direct,
-                                    "peak_source": "tcgen05 kind::tf32 issue probe of this library, 128x256x8 MMAs"}}
+    return {"bound": "tensor", "achieved": issued, "peak": peak, "unit": "TFLOP/s", "frac": issued / peak,
+            "useful_tflops": useful_tflops, "issued_tflops": issued, "useful_frac": useful_tflops / peak,
+            "peak_source": f"dense bf16, {kind}", "traffic": None}
 
 
 def conv_leg(job, spec_full, precision_name, steps, warmup):

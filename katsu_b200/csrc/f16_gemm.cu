@@ -238,7 +238,7 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
     const bool repairs = CONV && p.raw.form != KatsuF16Raw::NONE && p.splits == 1 && !(katsu_f16_finite(info_a) && katsu_f16_finite(info_b));
     const bool left_out = repairs && (p.accumulate || p.relu);
     // k-blocks between two drains: in TF32 mode up to 12 288 accumulation steps (4e-4 of 2e-3)
-    const int drain = NARROW == 2 ? (wide ? (p.drain + 1) / 2 : p.drain) : 1024;
+    const int drain = NARROW == 2 ? (wide ? max(p.drain / 2, 1) : p.drain) : 1024;
     // accumulators that take turns; hand-over q is the one q & (2^acc_bits - 1), acc_cols columns apart
     const int acc_bits = NARROW == 2 && p.bn <= 128 ? 2 : 1, acc_mask = (1 << acc_bits) - 1, acc_cols = 512 >> acc_bits;
     const int b_off = planes * A_BYTES, stage_bytes = b_off + planes * b_bytes;
@@ -674,14 +674,16 @@ int32_t katsu_f16_launch(katsu_cuda_ctx *ctx, KatsuF16Kind kind, const KatsuF16M
             }
     }
     // 3xTF32 mode: k-blocks to an accumulator, and with it the error against 64-bit sums of normally distributed values: 1 fine
-    // 1.5e-7, 1 2.6e-7, 2 4.8e-7, 5 1.2e-6, 16 3.6e-6.  The lines lie where that is below the error of other arithmetic of this
+    // 1.5e-7, 1 2.6e-7, 2 4.8e-7, 3 7e-7, 4 fine 6e-7 (plain 7e-7) in the small CNN's dX, 5 1.2e-6, 16 3.6e-6.  The lines lie where that is below the error of other arithmetic of this
     // mode's grade: kernels that cut operands into TF32 parts have 4.6e-7 to 8e-7 up to 8 k-blocks, 1.4e-6 and 1.6e-6 at 9
     // and 13, 4e-6 from 16 on, and 5e-7 to 4e-6 in dW; f32 multiply-adds 1.8e-8 times the root of their number (2.9e-7 for
     // 256 terms, 5.1e-7 for 800).  A drain costs more the shorter a tile's k-loop is (4096^3: 351 us with 16, 359 with 4, 375
     // with 2, 411 with 1; 64 channels, 8 x 56 x 56: 26.3, 27.9, 29.4, 31.4).
-    p.fine = p.f32_terms > 0 && p.f32_terms < 256;
+    // A contraction that one accumulator holds saves the sums in registers as well (that dX: 233 us, 300 in two parts).
+    p.fine = p.f32_terms > 0 ? p.f32_terms < 256 : kind != KATSU_F16_CONV_DW && most == 4;
     if (p.f32_terms > 0) p.drain = p.f32_terms < 800 ? 1 : 2;
-    else p.drain = kind == KATSU_F16_CONV_DW || most < 9 ? 2 : most < 16 ? 5 : 16;
+    else if (kind == KATSU_F16_CONV_DW) p.drain = 2;
+    else p.drain = most == 4 ? 4 : most < 9 ? 3 : most < 16 ? 5 : 16;
     p.kb_per_split = (int)((most + plan.splits - 1) / plan.splits);
     if (p.kb_per_split < 1) p.kb_per_split = 1;
     p.split_stride = 0;

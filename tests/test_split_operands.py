@@ -367,12 +367,12 @@ def test_small_regular_layers_stay_on_the_tensor_cores(ctx, oracle, shape):
 
 # What a 3xTF32 result may lose to the tensor core's accumulation, beside the 22 bits of its operands (6e-8): a step truncates
 # the sum by 2e-8 of it on average, and 12 steps (3 products) of 64 terms go to an accumulator before it is added to f32 sums,
-# or 24.  Taken small products first, 4 of the 12 count.  Twice the measured errors of 1.5e-7, 2.6e-7 and 4.8e-7 at most.
-FINE, ONE, TWO = 6e-8 + 4 * 4e-8, 6e-8 + 12 * 2.5e-8, 6e-8 + 24 * 2.5e-8
+# 24 or 36.  Taken small products first, 4 of the first 12 count.  Measured: 1.5e-7, 2.6e-7, 4.8e-7 and 7e-7.
+FINE, ONE, TWO, THREE = 6e-8 + 4 * 4e-8, 6e-8 + 12 * 2.5e-8, 6e-8 + 24 * 2.5e-8, 6e-8 + 36 * 2.5e-8
 
 
 @pytest.mark.parametrize("size, bars", [((333, 1001, 777), (TWO, ONE, ONE)), ((2050, 67, 1030), (FINE, TWO, TWO)), ((200, 300, 3001), (ONE, TWO, FINE)),
-                                        ((1024, 128, 512), (TWO, TWO, REL_L2_TOL)), ((512, 512, 512), (TWO, TWO, TWO))], ids=str)
+                                        ((1024, 128, 512), (TWO, THREE, REL_L2_TOL)), ((512, 512, 512), (THREE, THREE, THREE))], ids=str)
 def test_accumulation_error_of_products(ctx, oracle, size, bars):
     m, k, n = size
     rng = np.random.default_rng(m)
@@ -387,7 +387,7 @@ def test_accumulation_error_of_products(ctx, oracle, size, bars):
 
 
 @pytest.mark.parametrize("shape, bars", [((4, 35, 31, 25, 70, 5, 3, 2, 1), (ONE, ONE, FINE)), ((4, 3, 40, 40, 32, 5, 5, 1, 2), (FINE, TWO, FINE)),
-                                         ((2, 129, 14, 14, 67, 3, 3, 1, 1), (TWO, ONE, FINE)), ((4, 32, 32, 32, 64, 3, 3, 2, 1), (TWO, TWO, TWO)),
+                                         ((2, 129, 14, 14, 67, 3, 3, 1, 1), (TWO, ONE, FINE)), ((4, 32, 32, 32, 64, 3, 3, 2, 1), (THREE, THREE, TWO)),
                                          ((8, 96, 14, 14, 96, 1, 1, 1, 0), (TWO, TWO, TWO))], ids=str)
 def test_accumulation_error_of_layers(ctx, oracle, shape, bars):
     n, c, h, w, k, r, s, stride, pad = shape
