@@ -52,9 +52,8 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t addr) {
 
 // The same on the barrier at this place in both blocks of the pair.
 __device__ __forceinline__ void mma_commit_both(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"((unsigned short)3)
-                 : "memory");
+    mma_commit_pair(smem_u32(bar));
+    mma_commit_pair(map_to_rank(bar, 1));
 }
 
 __device__ __forceinline__ void tma_load_3d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_addr, int c0, int c1,
