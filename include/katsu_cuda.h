@@ -43,9 +43,18 @@ extern "C" {
 /* Arithmetic modes for the contraction kernels.  FP32 = CUDA-core fma.rn.f32.
  * 3XTF32 = tensor-core split precision (hi*hi + lo*hi + hi*lo into an f32
  * accumulator, 22 significand bits an operand), FP32-grade accuracy.  TF32 =
- * single tensor-core pass (11 bits).  The parts are fp16 with a power-of-two
- * scale per operand, or bf16 where an operand's range asks for it. Kernels
- * that run on CUDA cores (low-channel stencils, streaming ops) ignore it. */
+ * single tensor-core pass (11 bits).  Both take layers of at least 16 channels in
+ * multiples of 4, and any shape of 1e6 (matmul: 4e7, in TF32 mode 1.5e7)
+ * multiply-adds or more whatever its alignment; smaller ones, low-channel
+ * stencils and streaming ops run in f32 on CUDA cores.
+ * The parts are fp16 with a power-of-two scale per operand.  An element keeps
+ * its 22 (11) bits down to 2^-17 (2^-28) of the operand's largest magnitude and
+ * an absolute error of 2^-39 of that magnitude below.  An operand in which 128
+ * neighbours of a row, or 16 of a column (the channels of a pixel, the output
+ * channels of a weight), all lie below that line is cut into bf16 parts of 24
+ * (16) bits instead, with the rest of its call; so is one with infinities or
+ * NaNs.  Elements below the line among larger neighbours on both axes keep the
+ * absolute error; KATSU_MODE_FP32 has none. */
 #define KATSU_MODE_3XTF32 0
 #define KATSU_MODE_TF32 1
 #define KATSU_MODE_FP32 2

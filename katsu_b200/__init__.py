@@ -418,6 +418,7 @@ class Tensor:
         return out.value or 0
 
     def device_grad(self) -> int:
+        """Device address of the gradient (0: none), this tensor's own buffer: changing it in place changes no other gradient."""
         out = _vp()
         _check(_lib.kh_tensor_device_grad(self._h, ctypes.byref(out)))
         return out.value or 0

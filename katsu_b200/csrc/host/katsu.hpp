@@ -153,7 +153,7 @@ class Tensor {
     const Tensor &to_host() const;    // fills the host mirror now
     // Device accessors for callers that stay on the GPU (benchmarks).
     const float *device_data() const;
-    const float *device_grad() const;  // nullptr while grad is None
+    const float *device_grad() const;  // nullptr while grad is None; this tensor's own buffer, which the caller may change
 
     const TensorNode *id() const { return node_.get(); }  // Rc::as_ptr, tensor.rs:282-284
     bool defined() const { return node_ != nullptr; }
