@@ -415,9 +415,10 @@ f16_pair_kernel(const __grid_constant__ KatsuF16Maps maps, const __grid_constant
                                         }
                                     }
                                 }
-                                // every release goes to this block's barrier and to the peer's copy of it
-                                if (kb == kb_end - 1) mma_commit_both(&acc_full[b]);
+                                // Every release goes to this block's barrier and to the peer's copy of it.  The accumulator's
+                                // comes last: the blocks leave when it has been drained, and no arrival may be outstanding then.
                                 mma_commit_both(&empty[s]);
+                                if (kb == kb_end - 1) mma_commit_both(&acc_full[b]);
                             }
                             __syncwarp();
                             first = false;
